@@ -61,35 +61,39 @@ EOS_HD bool mt_intersect(f3 o, f3 d, f3 v1, f3 e1, f3 e2, float& t, float& u, fl
   return true;
 }
 
-// The same test with the rejections evaluated cheapest first; the result (accept and the
-// bits of t, u, v) is identical to mt_intersect because acceptance is the conjunction of
-// the same five conditions on the same values:
+// The same test with the rejections ahead of the division; the result (accept and the bits
+// of t, u, v) is identical to mt_intersect because acceptance is the conjunction of the
+// same five conditions on the same values:
 //   u = (T.P) * (1/det), v = (d.Q) * (1/det), t = (e2.Q) * (1/det)
-// A product of two floats rounds to a value of the product's sign (or to zero), so when
-// a numerator's sign is opposite to det's and its magnitude is far from the underflow
-// range, u (v, t) < 0 is decided without the division; misses mostly end there.
-__device__ __forceinline__ bool opposite_sign_reject(float num, float det) {
-  return (num < 0.0f) != (det < 0.0f) && fabsf(num) > 1e-30f;
-}
-
+// A product of two floats rounds to a value of the product's sign (or to zero), so when a
+// numerator's sign is opposite to det's and its magnitude is far from the underflow range,
+// u (v, t) < 0 is decided without the division.  u > 1 and u + v > 1 are decided where the
+// numerators exceed |det| by far more than the three roundings of u (2^-20) or the four of
+// u + v (2^-18).  What is left goes to the division and the exact tests; misses mostly end
+// at the one branch before it, and the conditions are combined there because a warp's lanes
+// rarely agree on any one of them.
 __device__ __forceinline__ bool mt_intersect_fast(f3 o, f3 d, f3 v1, f3 e1, f3 e2, float& t, float& u, float& v) {
-  f3 P = cross3(d, e2);
-  float det = dot3(e1, P);
-  if (det > -0.00001f && det < 0.00001f) return false;
-  f3 T = sub3(o, v1);
-  float nu = dot3(T, P);
-  if (opposite_sign_reject(nu, det)) return false;  // u < 0
-  f3 Q = cross3(T, e1);
-  float nv = dot3(d, Q);
-  if (opposite_sign_reject(nv, det)) return false;  // v < 0
-  float nt = dot3(e2, Q);
-  if (opposite_sign_reject(nt, det)) return false;  // t < 0
-  float inv_det = 1.0f / det;
-  float uu = nu * inv_det;
+  const f3 P = cross3(d, e2);
+  const float det = dot3(e1, P);
+  const f3 T = sub3(o, v1);
+  const float nu = dot3(T, P);
+  const f3 Q = cross3(T, e1);
+  const float nv = dot3(d, Q);
+  const float nt = dot3(e2, Q);
+  const uint32_t sign = det < 0.0f ? 0x80000000u : 0u;
+  const float su = __uint_as_float(__float_as_uint(nu) ^ sign);
+  const float sv = __uint_as_float(__float_as_uint(nv) ^ sign);
+  const float s_t = __uint_as_float(__float_as_uint(nt) ^ sign);
+  const float ad = fabsf(det);
+  const bool out = (ad < 0.00001f) | (su < -1e-30f) | (sv < -1e-30f) | (s_t < -1e-30f) |
+                   (su > ad * (1.0f + 0x1p-20f)) | (su + sv > ad * (1.0f + 0x1p-18f));
+  if (out) return false;
+  const float inv_det = 1.0f / det;
+  const float uu = nu * inv_det;
   if (uu < 0.0f || uu > 1.0f) return false;
-  float vv = nv * inv_det;
+  const float vv = nv * inv_det;
   if (vv < 0.0f || uu + vv > 1.0f) return false;
-  float tt = nt * inv_det;
+  const float tt = nt * inv_det;
   if (tt < 0.0f) return false;
   t = tt;
   u = uu;

@@ -32,7 +32,7 @@ struct PlainParams {
 // One path: colour with the reference's fold c_k = phong_k + w_k c_{k+1} (fold_colour).
 template <int SH>
 __device__ f3 trace_path(const PlainParams& P, f3 o, f3 d, int32_t* hits, uint32_t* masks, unsigned* cnt,
-                         uint2* shs, int stride) {
+                         uint32_t col, uint32_t stride) {
   const DevScene& s = P.s;
   f3 phong[kMaxBounces];
   float weight[kMaxBounces];
@@ -40,7 +40,7 @@ __device__ f3 trace_path(const PlainParams& P, f3 o, f3 d, int32_t* hits, uint32
   const f3 campos = mk3(P.cam[0], P.cam[1], P.cam[2]);
   for (int k = 0; k <= P.trace_depth; ++k) {
     cnt[k == 0 ? kCntPrimary : kCntSecondary]++;
-    Hit h = closest_hit<SH>(s, o, d, shs, stride, P.err);
+    Hit h = closest_hit<SH>(s, o, d, col, stride, P.err);
     cnt[kCntNodesC] += h.nodes;
     cnt[kCntTestsC] += h.tests;
     if (h.pos < 0) {
@@ -60,7 +60,7 @@ __device__ f3 trace_path(const PlainParams& P, f3 o, f3 d, int32_t* hits, uint32
       f3 sd = norm3(sub3(mk3(l[0], l[1], l[2]), Pp));
       f3 so = add3(Pp, scale3(kRayEps, sd));
       cnt[kCntShadow]++;
-      AnyResult ar = any_hit<SH>(s, so, sd, shs, stride, P.err);
+      AnyResult ar = any_hit<SH>(s, so, sd, col, stride, P.err);
       cnt[kCntNodesA] += ar.nodes;
       cnt[kCntTestsA] += ar.tests;
       if (ar.hit)
@@ -97,7 +97,7 @@ struct TreeFrame {
 // colours by tree_colour.  rec (nullable): the path's tree record, heap order.
 template <int SH>
 __device__ f3 trace_tree(const PlainParams& P, f3 o, f3 d, eos_tree_node* rec, int& root_hit, unsigned* cnt,
-                         uint2* shs, int stride) {
+                         uint32_t col, uint32_t stride) {
   const DevScene& s = P.s;
   const f3 campos = mk3(P.cam[0], P.cam[1], P.cam[2]);
   const f3 zero = mk3(0.0f, 0.0f, 0.0f);
@@ -107,7 +107,7 @@ __device__ f3 trace_tree(const PlainParams& P, f3 o, f3 d, eos_tree_node* rec, i
     // trace the ray of (node, depth <= trace_depth) and shade its hit
     f3 c = zero;
     cnt[depth == 0 ? kCntPrimary : kCntSecondary]++;
-    Hit h = closest_hit<SH>(s, o, d, shs, stride, P.err);
+    Hit h = closest_hit<SH>(s, o, d, col, stride, P.err);
     cnt[kCntNodesC] += h.nodes;
     cnt[kCntTestsC] += h.tests;
     if (node == 0) root_hit = h.pos < 0 ? EOS_HIT_NONE : h.id;
@@ -127,7 +127,7 @@ __device__ f3 trace_tree(const PlainParams& P, f3 o, f3 d, eos_tree_node* rec, i
         f3 sd = norm3(sub3(mk3(l[0], l[1], l[2]), Pp));
         f3 so = add3(Pp, scale3(kRayEps, sd));
         cnt[kCntShadow]++;
-        AnyResult ar = any_hit<SH>(s, so, sd, shs, stride, P.err);
+        AnyResult ar = any_hit<SH>(s, so, sd, col, stride, P.err);
         cnt[kCntNodesA] += ar.nodes;
         cnt[kCntTestsA] += ar.tests;
         if (ar.hit) mask |= 1u << li;
@@ -194,8 +194,7 @@ __device__ f3 trace_tree(const PlainParams& P, f3 o, f3 d, eos_tree_node* rec, i
 template <int SH, bool TREE = false>
 __global__ void __maxnreg__(64) k_render_plain(PlainParams P) {
   extern __shared__ uint2 shstack[];
-  uint2* shs = shstack + threadIdx.x;
-  const int stride = blockDim.x;
+  const uint32_t col = shared_address(shstack + threadIdx.x), stride = 8 * blockDim.x;
   unsigned cnt[kNumCounts] = {0, 0, 0, 0, 0, 0, 0, 0};
   // one warp = one 8x4 pixel tile (coherent primary rays)
   const int g = blockIdx.x * blockDim.x + threadIdx.x;
@@ -220,7 +219,7 @@ __global__ void __maxnreg__(64) k_render_plain(PlainParams P) {
         if (rec)
           for (int k = 0; k < nn; ++k) rec[k] = eos_tree_node{EOS_HIT_UNTRACED, 0u};
         int root_hit = EOS_HIT_NONE;
-        f3 c = trace_tree<SH>(P, o, d, rec, root_hit, cnt, shs, stride);
+        f3 c = trace_tree<SH>(P, o, d, rec, root_hit, cnt, col, stride);
         sum = add3(sum, c);
         if (P.hit) P.hit[path] = root_hit;
       } else {
@@ -231,7 +230,7 @@ __global__ void __maxnreg__(64) k_render_plain(PlainParams P) {
           hits[k] = EOS_HIT_UNTRACED;
           masks[k] = 0;
         }
-        f3 c = trace_path<SH>(P, o, d, hits, masks, cnt, shs, stride);
+        f3 c = trace_path<SH>(P, o, d, hits, masks, cnt, col, stride);
         sum = add3(sum, c);
         if (P.hit) P.hit[path] = hits[0];
         if (P.paths) {
@@ -266,20 +265,20 @@ __global__ void k_trace_closest(DevScene s, const float* __restrict__ rays, int 
   int i = blockIdx.x * blockDim.x + threadIdx.x;
   if (i >= n) return;
   const float* r = rays + 6 * (size_t)i;
-  Hit h = closest_hit<SH>(s, mk3(r[0], r[1], r[2]), mk3(r[3], r[4], r[5]), shstack + threadIdx.x, blockDim.x, err);
+  Hit h = closest_hit<SH>(s, mk3(r[0], r[1], r[2]), mk3(r[3], r[4], r[5]), shared_address(shstack + threadIdx.x),
+                          8 * blockDim.x, err);
   ids[i] = h.pos < 0 ? EOS_HIT_NONE : h.id;
   if (ts) ts[i] = h.t;
 }
 
 template <int SH>
 __global__ void k_trace_any(DevScene s, const float* __restrict__ rays, int n, uint8_t* occ, int* err) {
-  extern __shared__ uint2 shstack[];
+  extern __shared__ int shrefs[];
   int i = blockIdx.x * blockDim.x + threadIdx.x;
   if (i >= n) return;
   const float* r = rays + 6 * (size_t)i;
-  occ[i] = any_hit<SH>(s, mk3(r[0], r[1], r[2]), mk3(r[3], r[4], r[5]), shstack + threadIdx.x, blockDim.x, err).hit
-               ? 1
-               : 0;
+  occ[i] = any_hit<SH>(s, mk3(r[0], r[1], r[2]), mk3(r[3], r[4], r[5]), shared_address(shrefs + threadIdx.x),
+                       4 * blockDim.x, err).hit ? 1 : 0;
 }
 
 inline int clamp_block(int b) { return b <= 0 ? 128 : std::min(512, std::max(32, (b / 32) * 32)); }
@@ -359,7 +358,7 @@ eos_status trace_any(eos_ctx* ctx, const eos_scene* sc, const float* d_rays, uin
   if (n == 0) return EOS_OK;
   const int block = 128;
   const int grid = (int)((n + block - 1) / block);
-  k_trace_any<16><<<grid, block, 16 * block * sizeof(uint2), ctx->stream>>>(sc->dev, d_rays, (int)n, d_occ,
+  k_trace_any<16><<<grid, block, 16 * block * sizeof(int), ctx->stream>>>(sc->dev, d_rays, (int)n, d_occ,
                                                                            ctx->d_err);
   EOS_CUDA(cudaGetLastError());
   return EOS_OK;

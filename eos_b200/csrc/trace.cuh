@@ -80,22 +80,6 @@ __device__ __forceinline__ void slab_range(const SlabRay& r, float nx, float ny,
   tf = min3f(tfx, tfy, tfz) * kSlack;
 }
 
-// Entry distance of a box, or kInf when the box is missed or starts beyond `limit`.
-__device__ __forceinline__ float slab(const SlabRay& r, float nx, float ny, float nz, float fx, float fy, float fz,
-                                      float limit) {
-  float tn, tf;
-  slab_range(r, nx, ny, nz, fx, fy, fz, tn, tf);
-  return tn <= fminf(tf, limit) ? tn : kInf;
-}
-
-// Hit test of a box for shadow rays (no distance limit, no entry distance needed).
-__device__ __forceinline__ bool slab_hit(const SlabRay& r, float nx, float ny, float nz, float fx, float fy,
-                                         float fz) {
-  float tn, tf;
-  slab_range(r, nx, ny, nz, fx, fy, fz, tn, tf);
-  return tn <= tf;
-}
-
 // Box test in the form b = fma(p, i, c) per plane (i = 1/d), one instruction where
 // (p - o) * i takes two; used by both traversals.  c is offset per axis: c_near = fl(c - eps),
 // c_far = fl(c + eps), c = fl(-(o i)), eps = 2^-20 |c| + 2^-126.  With u = 2^-24 and
@@ -135,20 +119,6 @@ __device__ __forceinline__ FmaSlabRay make_fma_slab(const SlabRay& r) {
   return q;
 }
 
-__device__ __forceinline__ bool slab_hit(const FmaSlabRay& r, float nx, float ny, float nz, float fx, float fy,
-                                         float fz) {
-  const float tn = fmaxf(max3f(fmaf(nx, r.ix, r.nx), fmaf(ny, r.iy, r.ny), fmaf(nz, r.iz, r.nz)), 0.0f);
-  const float tf = min3f(fmaf(fx, r.ix, r.fx), fmaf(fy, r.iy, r.fy), fmaf(fz, r.iz, r.fz)) * (1.0f + 0x1p-19f);
-  return tn <= tf;
-}
-
-__device__ __forceinline__ float slab(const FmaSlabRay& r, float nx, float ny, float nz, float fx, float fy, float fz,
-                                      float limit) {
-  const float tn = fmaxf(max3f(fmaf(nx, r.ix, r.nx), fmaf(ny, r.iy, r.ny), fmaf(nz, r.iz, r.nz)), 0.0f);
-  const float tf = min3f(fmaf(fx, r.ix, r.fx), fmaf(fy, r.iy, r.fy), fmaf(fz, r.iz, r.fz)) * (1.0f + 0x1p-19f);
-  return tn <= fminf(tf, limit) ? tn : kInf;
-}
-
 // Culling factor on the best hit distance per ray form: the fma form's entry distance can
 // exceed the exact form's by 3.0002u relative, which 2^-19 more covers.
 template <class Ray>
@@ -181,51 +151,6 @@ __device__ __forceinline__ bool is_leaf_ref(int r) { return ((uint32_t)r & 0xC00
 __device__ __forceinline__ int leaf_first(int r) { return r & 0x01ffffff; }
 __device__ __forceinline__ int leaf_count(int r) { return ((r >> 25) & 31) + 1; }
 
-// Per-thread traversal stack of (child ref, entry distance): the first SH entries live in
-// shared memory (column threadIdx.x of a [SH][blockDim] array), deeper entries spill to
-// local memory, CAP in total (kStackMax; CAP = SH, no spill, is the small stack of the
-// error-path test limit, eos_limits.small_stack).
-template <int SH, int CAP = kStackMax>
-struct TraversalStack {
-  static_assert(CAP >= SH, "the shared part is the bottom of the stack");
-  static constexpr int kShared = SH;
-  uint2* sh;
-  int stride;
-  int sp;
-  uint2 spill[CAP > SH ? CAP - SH : 1];
-  __device__ __forceinline__ TraversalStack(uint2* base, int str) : sh(base), stride(str), sp(0) {}
-  __device__ __forceinline__ bool push(int ref, float t) {
-    uint2 v = make_uint2((uint32_t)ref, __float_as_uint(t));
-    if (sp < SH) sh[sp * stride] = v;
-    else if (sp < CAP) spill[sp - SH] = v;
-    else return false;
-    ++sp;
-    return true;
-  }
-  __device__ __forceinline__ void push_shared(int ref, float t) {
-    sh[sp * stride] = make_uint2((uint32_t)ref, __float_as_uint(t));
-    ++sp;
-  }
-  __device__ __forceinline__ uint2 pop() {
-    --sp;
-    return sp < SH ? sh[sp * stride] : spill[sp - SH];
-  }
-  // Next entry whose box starts no later than `limit`, or kDone.
-  __device__ __forceinline__ int next(float limit) {
-    while (sp > 0) {
-      uint2 e = pop();
-      if (__uint_as_float(e.y) <= limit) return (int)e.x;
-    }
-    return kDone;
-  }
-  // Next entry, any distance (shadow rays), or kDone.
-  __device__ __forceinline__ int next_any() { return sp > 0 ? (int)pop().x : kDone; }
-  // Entries without a distance (any-hit traversal).
-  __device__ __forceinline__ bool push_ref(int ref) { return push(ref, 0.0f); }
-  __device__ __forceinline__ void push_ref_shared(int ref) { push_shared(ref, 0.0f); }
-};
-
-
 __device__ __forceinline__ void load_tri(const float4* __restrict__ tris, int p, f3& v1, f3& e1, f3& e2, int& id) {
   float4 a = __ldg(tris + 3 * (size_t)p);
   float4 b = __ldg(tris + 3 * (size_t)p + 1);
@@ -236,112 +161,284 @@ __device__ __forceinline__ void load_tri(const float4* __restrict__ tris, int p,
   id = __float_as_int(c.y);
 }
 
-// One fetch of a node record (128 B, four child slots; a binary tree leaves two of them
-// unused): the child boxes are tested; with SORT the hit children are ordered by entry
-// distance (five compare-exchanges), the nearest becomes `cur` and the others are pushed
-// farthest first; without SORT (shadow rays: no distance limit) only hit / miss is
-// computed and the first hit in slot order is taken, which measured faster for shadow
-// rays than nearest-first.  An unused slot holds the box
-// lo = +inf, hi = -inf: on every axis the near plane gives an entry of +inf and the far
-// plane an exit of -inf, whatever the direction's sign (parallel axes fail the containment
-// test), so both box tests reject it and no per-slot check is needed.  With three free
-// shared-memory stack entries (the most one node pushes) the pushes skip their bound
-// checks.  Returns false on stack overflow.
+// ------------------------------------------------------------------ flat scenes
+// Shared-memory accesses of the traversal stack by 32-bit address.  Each is one instruction
+// under the predicate it depends on, so a node visit pushes its children without branches.
+// What bounds a visit is instruction issue (and, once that fell, L1 wavefronts): with one
+// branch per pushed child and a bound check per pop a visit's integer and control
+// instructions outnumbered its box arithmetic.  Measured on the shadow rays of a 1080p view of
+// 1.06M triangles (2.8M rays), branching form -> this one: 516 -> 411 M warp instructions,
+// 662 -> 574 us; the same view's primary rays 231 -> 220 us.
+__device__ __forceinline__ uint32_t shared_address(const void* p) { return (uint32_t)__cvta_generic_to_shared(p); }
+__device__ __forceinline__ void sts_ref(uint32_t a, int ref) {
+  asm volatile("st.shared.b32 [%0], %1;" ::"r"(a), "r"(ref));
+}
+__device__ __forceinline__ int lds_ref(uint32_t a) {
+  int v;
+  asm volatile("ld.shared.b32 %0, [%1];" : "=r"(v) : "r"(a));
+  return v;
+}
+__device__ __forceinline__ void sts_entry(uint32_t a, int ref, float t) {
+  asm volatile("st.shared.v2.b32 [%0], {%1, %2};" ::"r"(a), "r"(ref), "f"(t));
+}
+__device__ __forceinline__ void lds_entry(uint32_t a, int& ref, float& t) {
+  asm volatile("ld.shared.v2.b32 {%0, %1}, [%2];" : "=r"(ref), "=f"(t) : "r"(a));
+}
+// A visit's four children of a shadow ray (hit where tn <= tf), in slot order: `cur` takes
+// the first hit one, the other hit ones are pushed, and with no hit the top entry is popped.
+__device__ __forceinline__ void follow_hits(uint32_t& top, uint32_t stride, int& cur, const int4& ref,
+                                            const float* tn, const float* tf) {
+  asm volatile(
+      "{\n.reg .pred p0, p1, p2, q1, q2, q3, a1, a2, a3;\n"
+      "setp.le.f32 p0, %7, %11;\n"
+      "setp.le.f32 p1, %8, %12;\n"
+      "setp.le.f32 p2, %9, %13;\n"
+      "and.pred q1, p1, p0;\n"
+      "or.pred a1, p1, p0;\n"
+      "and.pred q2, p2, a1;\n"
+      "or.pred a2, p2, a1;\n"
+      "setp.le.and.f32 q3, %10, %14, a2;\n"
+      "setp.le.or.f32 a3, %10, %14, a2;\n"
+      "@q1 add.u32 %0, %0, %2;\n@q1 st.shared.b32 [%0], %4;\n"
+      "@q2 add.u32 %0, %0, %2;\n@q2 st.shared.b32 [%0], %5;\n"
+      "@q3 add.u32 %0, %0, %2;\n@q3 st.shared.b32 [%0], %6;\n"
+      "selp.b32 %1, %5, %6, p2;\n"
+      "selp.b32 %1, %4, %1, p1;\n"
+      "selp.b32 %1, %3, %1, p0;\n"
+      "@!a3 ld.shared.b32 %1, [%0];\n@!a3 sub.u32 %0, %0, %2;\n}"
+      : "+r"(top), "=&r"(cur)
+      : "r"(stride), "r"(ref.x), "r"(ref.y), "r"(ref.z), "r"(ref.w), "f"(tn[0]), "f"(tn[1]), "f"(tn[2]), "f"(tn[3]),
+        "f"(tf[0]), "f"(tf[1]), "f"(tf[2]), "f"(tf[3]));
+}
+// top += stride and store, where t < inf (nearest hit: a child box in reach).
+__device__ __forceinline__ void push_if_near(uint32_t& top, uint32_t stride, int ref, float t) {
+  asm volatile(
+      "{\n.reg .pred p;\nsetp.lt.f32 p, %3, 0f7F800000;\n@p add.u32 %0, %0, %1;\n"
+      "@p st.shared.v2.b32 [%0], {%2, %3};\n}"
+      : "+r"(top)
+      : "r"(stride), "r"(ref), "f"(t));
+}
 
-template <bool SORT, class Ray, class Stack>
-__device__ __forceinline__ bool visit_node4(const float4* __restrict__ node_base, const Ray& r, int& cur,
-                                            float limit, Stack& st, unsigned& nodes) {
-  constexpr int SH = Stack::kShared;
-  const float4* nd = node_base + 8 * (size_t)cur;
-  const float4 lx = __ldg(nd + r.sx), ly = __ldg(nd + 1 + r.sy), lz = __ldg(nd + 2 + r.sz);  // near planes
-  const float4 hx = __ldg(nd + 3 - r.sx), hy = __ldg(nd + 4 - r.sy), hz = __ldg(nd + 5 - r.sz);  // far planes
-  const int4 ref = __ldg(reinterpret_cast<const int4*>(nd) + 6);
-  ++nodes;
+// Traversal stack of a flat scene: a column of SH shared-memory entries (a child ref, and
+// its entry distance with T), entry k at col + k * stride bytes.  Entry 0 is a sentinel --
+// kDone, or kRefill when older entries lie in local memory -- so a pop needs no emptiness
+// check.  When fewer than three entries are free, everything above the sentinel moves to
+// local memory (at most CAP entries; CAP = SH is the small stack of the error-path test
+// limit, eos_limits.small_stack: SH entries in all).  Shadow rays keep refs only, in 4-byte
+// columns where their kernel traces nothing else: half the shared memory, and the rest of
+// the SM's 256 KB is L1 (with 32 entries instead of 16 both stages lose about 10 %).  A
+// kernel that traces both kinds keeps every thread inside its own 8-byte column, because
+// lanes of one warp may be in different traversals.
+constexpr int kRefill = (int)0xC0000002;
+// Leaf refs as signed ints lie below kSpecial; kDone and kRefill in [kSpecial, 0).
+constexpr int kSpecial = (int)0xC0000000;
+
+template <int SH, int CAP, bool T>
+struct ColumnStack {
+  static_assert(SH >= 8, "a visit pushes up to three entries above the sentinel");
+  static constexpr bool kSmall = CAP == SH;             // at most SH entries in all (test limit)
+  static constexpr int kLocal = kSmall ? SH + 4 : CAP;  // entries of the local part
+  uint32_t col, stride, top;
+  int spilled;
+  int ref_lo[kLocal];
+  float t_lo[T ? kLocal : 1];
+  __device__ __forceinline__ ColumnStack(uint32_t c, uint32_t s) : col(c), stride(s), top(c), spilled(0) {
+    sentinel(kDone);
+  }
+  __device__ __forceinline__ void sentinel(int ref) {
+    if (T) sts_entry(col, ref, -kInf);  // never beyond a limit
+    else sts_ref(col, ref);
+  }
+  // Makes room for a visit's pushes; false when the local part is full too.
+  __device__ __forceinline__ bool reserve() {
+    if (top <= col + (SH - 4) * stride) return true;
+#pragma unroll 1
+    for (uint32_t a = col + stride; a <= top; a += stride) {
+      if (spilled >= kLocal) return false;
+      if (T) lds_entry(a, ref_lo[spilled], t_lo[spilled]);
+      else ref_lo[spilled] = lds_ref(a);
+      ++spilled;
+    }
+    top = col;
+    sentinel(kRefill);
+    return true;
+  }
+  // After a visit: false when the small stack's limit is passed.
+  __device__ __forceinline__ bool within_limit() const {
+    return !kSmall || (int)(top - col) <= (SH - spilled) * (int)stride;
+  }
+  // After a pop of kRefill: brings back the newest entries, half a column at most.
+  __device__ __forceinline__ void refill() {
+    const int n = min(spilled, (SH - 4) / 2);
+    sentinel(spilled > n ? kRefill : kDone);
+    top = col;
+#pragma unroll 1
+    for (int k = spilled - n; k < spilled; ++k) {
+      top += stride;
+      if (T) sts_entry(top, ref_lo[k], t_lo[k]);
+      else sts_ref(top, ref_lo[k]);
+    }
+    spilled -= n;
+  }
+  __device__ __forceinline__ void push(int ref, float t) {
+    top += stride;
+    if (T) sts_entry(top, ref, t);
+    else sts_ref(top, ref);
+  }
+  __device__ __forceinline__ int pop() {
+    const int r = lds_ref(top);
+    top -= stride;
+    return r;
+  }
+  // The next entry whose box starts no later than `limit` (the sentinel's always does).
+  __device__ __forceinline__ int pop_within(float limit) {
+    int r;
+    float t;
+    do {
+      lds_entry(top, r, t);
+      top -= stride;
+    } while (t > limit);
+    return r;
+  }
+};
+
+// Entry and exit distances of the four child boxes of a node record for a prepared ray.
+// The fma form takes two children per instruction (fma.rn.f32x2: each half rounds as fmaf);
+// 410 instead of 429 M warp instructions in the measurement above, at the same registers.
+struct Box4 {
+  float tn[4], tf[4];
+};
+
+__device__ __forceinline__ const char* node_address(const float4* nodes, int node) {
+  return reinterpret_cast<const char*>(nodes) + (size_t)(uint32_t)node * 128u;
+}
+
+__device__ __forceinline__ float4 ldg4(const char* p) { return __ldg(reinterpret_cast<const float4*>(p)); }
+
+__device__ __forceinline__ Box4 child_boxes(const char* nd, const SlabRay& r) {
+  const float4 lx = ldg4(nd + 16 * r.sx), ly = ldg4(nd + 16 * r.sy + 16), lz = ldg4(nd + 16 * r.sz + 32);
+  const float4 hx = ldg4(nd - 16 * r.sx + 48), hy = ldg4(nd - 16 * r.sy + 64), hz = ldg4(nd - 16 * r.sz + 80);
+  Box4 b;
+  slab_range(r, lx.x, ly.x, lz.x, hx.x, hy.x, hz.x, b.tn[0], b.tf[0]);
+  slab_range(r, lx.y, ly.y, lz.y, hx.y, hy.y, hz.y, b.tn[1], b.tf[1]);
+  slab_range(r, lx.z, ly.z, lz.z, hx.z, hy.z, hz.z, b.tn[2], b.tf[2]);
+  slab_range(r, lx.w, ly.w, lz.w, hx.w, hy.w, hz.w, b.tn[3], b.tf[3]);
+  return b;
+}
+
+typedef unsigned long long f2;  // two floats in a register pair
+__device__ __forceinline__ f2 dup2(float v) {
+  f2 r;
+  asm("mov.b64 %0, {%1, %1};" : "=l"(r) : "f"(v));
+  return r;
+}
+__device__ __forceinline__ f2 pack2(float a, float b) {
+  f2 r;
+  asm("mov.b64 %0, {%1, %2};" : "=l"(r) : "f"(a), "f"(b));
+  return r;
+}
+__device__ __forceinline__ void unpack2(f2 v, float& a, float& b) { asm("mov.b64 {%0, %1}, %2;" : "=f"(a), "=f"(b) : "l"(v)); }
+__device__ __forceinline__ f2 fma2(f2 a, f2 b, f2 c) {
+  f2 r;
+  asm("fma.rn.f32x2 %0, %1, %2, %3;" : "=l"(r) : "l"(a), "l"(b), "l"(c));
+  return r;
+}
+__device__ __forceinline__ void axis4(float4 p, float i, float c, float* o) {
+  unpack2(fma2(pack2(p.x, p.y), dup2(i), dup2(c)), o[0], o[1]);
+  unpack2(fma2(pack2(p.z, p.w), dup2(i), dup2(c)), o[2], o[3]);
+}
+
+__device__ __forceinline__ Box4 child_boxes(const char* nd, const FmaSlabRay& r) {
+  const float4 lx = ldg4(nd + 16 * r.sx), ly = ldg4(nd + 16 * r.sy + 16), lz = ldg4(nd + 16 * r.sz + 32);
+  const float4 hx = ldg4(nd - 16 * r.sx + 48), hy = ldg4(nd - 16 * r.sy + 64), hz = ldg4(nd - 16 * r.sz + 80);
+  float x[4], y[4], z[4];
+  Box4 b;
+  axis4(lx, r.ix, r.nx, x);
+  axis4(ly, r.iy, r.ny, y);
+  axis4(lz, r.iz, r.nz, z);
+#pragma unroll
+  for (int i = 0; i < 4; ++i) b.tn[i] = fmaxf(max3f(x[i], y[i], z[i]), 0.0f);
+  axis4(hx, r.ix, r.fx, x);
+  axis4(hy, r.iy, r.fy, y);
+  axis4(hz, r.iz, r.fz, z);
+#pragma unroll
+  for (int i = 0; i < 4; ++i) b.tf[i] = min3f(x[i], y[i], z[i]) * (1.0f + 0x1p-19f);
+  return b;
+}
+
+// A visit's four children of a nearest-hit ray: those in reach (entry within the exit and
+// the limit) sorted by entry distance (five compare-exchanges), the others but the nearest
+// pushed farthest first; returns the nearest, or the next entry of the stack.
+template <class Stack>
+__device__ __forceinline__ int follow_nearest(Stack& st, const int4& ref, const Box4& b, float limit) {
   int c[4] = {ref.x, ref.y, ref.z, ref.w};
-  if constexpr (SORT) {
-    float t[4];
-    t[0] = slab(r, lx.x, ly.x, lz.x, hx.x, hy.x, hz.x, limit);
-    t[1] = slab(r, lx.y, ly.y, lz.y, hx.y, hy.y, hz.y, limit);
-    t[2] = slab(r, lx.z, ly.z, lz.z, hx.z, hy.z, hz.z, limit);
-    t[3] = slab(r, lx.w, ly.w, lz.w, hx.w, hy.w, hz.w, limit);
+  float t[4];
+#pragma unroll
+  for (int i = 0; i < 4; ++i) t[i] = b.tn[i] <= fminf(b.tf[i], limit) ? b.tn[i] : kInf;
 #define EOS_CX(a, b)                 \
   if (t[b] < t[a]) {                 \
     float tt = t[a]; t[a] = t[b]; t[b] = tt; \
     int cc = c[a]; c[a] = c[b]; c[b] = cc;   \
   }
-    EOS_CX(0, 1) EOS_CX(2, 3) EOS_CX(0, 2) EOS_CX(1, 3) EOS_CX(1, 2)
+  EOS_CX(0, 1) EOS_CX(2, 3) EOS_CX(0, 2) EOS_CX(1, 3) EOS_CX(1, 2)
 #undef EOS_CX
-    if (t[0] == kInf) {
-      cur = st.next(limit);
-      return true;
-    }
-    if (st.sp + 3 <= SH) {
-#pragma unroll
-      for (int i = 3; i >= 1; --i)
-        if (t[i] != kInf) st.push_shared(c[i], t[i]);
-    } else {
-#pragma unroll
-      for (int i = 3; i >= 1; --i)
-        if (t[i] != kInf && !st.push(c[i], t[i])) return false;
-    }
-    cur = c[0];
-    return true;
-  } else {
-    bool h[4];
-    h[0] = slab_hit(r, lx.x, ly.x, lz.x, hx.x, hy.x, hz.x);
-    h[1] = slab_hit(r, lx.y, ly.y, lz.y, hx.y, hy.y, hz.y);
-    h[2] = slab_hit(r, lx.z, ly.z, lz.z, hx.z, hy.z, hz.z);
-    h[3] = slab_hit(r, lx.w, ly.w, lz.w, hx.w, hy.w, hz.w);
-    int first = -1;
-    if (st.sp + 3 <= SH) {
-#pragma unroll
-      for (int i = 0; i < 4; ++i) {
-        if (!h[i]) continue;
-        if (first < 0) first = i;
-        else st.push_ref_shared(c[i]);
-      }
-    } else {
-#pragma unroll
-      for (int i = 0; i < 4; ++i) {
-        if (!h[i]) continue;
-        if (first < 0) first = i;
-        else if (!st.push_ref(c[i])) return false;
-      }
-    }
-    cur = first < 0 ? st.next_any() : c[first];
-    return true;
-  }
+  push_if_near(st.top, st.stride, c[3], t[3]);
+  push_if_near(st.top, st.stride, c[2], t[2]);
+  push_if_near(st.top, st.stride, c[1], t[1]);
+  return t[0] == kInf ? st.pop_within(limit) : c[0];
 }
 
 // Nearest hit.  Traversal in the two-loop form of Aila & Laine ("Understanding the
 // efficiency of ray traversal on GPUs", HPG 2009): a lane that reaches a leaf parks it and
 // keeps descending until every lane of the warp holds a leaf, then the lanes intersect
 // their leaves together, so triangle tests run with full warps.
+//
+// A node visit tests the four child boxes of one 128-B record; an unused slot holds the box
+// lo = +inf, hi = -inf: on every axis the near plane gives an entry of +inf and the far
+// plane an exit of -inf, whatever the direction's sign (parallel axes fail the containment
+// test), so both box tests reject it and no per-slot check is needed.  The hit children are
+// sorted by entry distance (five compare-exchanges), pushed farthest first and the nearest
+// popped again.
 template <int SH, int CAP, class Ray>
-__device__ __forceinline__ Hit closest_traverse(const DevScene& s, f3 o, f3 d, const Ray& r, uint2* shs, int stride,
-                                               int* err) {
+__device__ __forceinline__ Hit closest_traverse(const DevScene& s, f3 o, f3 d, const Ray& r, uint32_t col,
+                                               uint32_t stride, int* err) {
   constexpr float kCullR = RayCull<Ray>::k;
   Hit h;
   h.t = kInf; h.u = h.v = 0.0f; h.pos = -1; h.id = -1; h.nodes = 0; h.tests = 0;
-  TraversalStack<SH, CAP> st(shs, stride);
-  int cur = 0;   // interior node, leaf ref or kDone
+  ColumnStack<SH, CAP, true> st(col, stride);
+  int cur = 0;   // interior node, leaf ref, kRefill or kDone
   int leaf = 0;  // parked leaf (0 = none)
   for (;;) {
     while (cur >= 0) {
-      if (!visit_node4<true>(s.nodes, r, cur, h.t * kCullR, st, h.nodes)) {
+      const char* nd = node_address(s.nodes, cur);
+      const int4 ref = __ldg(reinterpret_cast<const int4*>(nd + 96));
+      const Box4 b = child_boxes(nd, r);
+      ++h.nodes;
+      if (!st.reserve()) {
         atomicOr(err, kErrStack);
         return h;
       }
-      if (cur != kDone && cur < 0 && leaf == 0) {
+      cur = follow_nearest(st, ref, b, h.t * kCullR);
+      if (!st.within_limit()) {
+        atomicOr(err, kErrStack);
+        return h;
+      }
+      if (cur < kSpecial && leaf == 0) {
         leaf = cur;
-        cur = st.next(h.t * kCullR);
+        cur = st.pop_within(h.t * kCullR);
       }
       if (!__any_sync(__activemask(), leaf == 0)) break;
     }
+    if (cur < kSpecial && leaf == 0) {
+      leaf = cur;
+      cur = st.pop_within(h.t * kCullR);
+    }
     while (leaf != 0) {
-      const int first = leaf_first(leaf), cnt = leaf_count(leaf);
+      const int cnt = leaf_count(leaf);
+      int p = leaf_first(leaf);
+      const int end = p + cnt;
       h.tests += cnt;
-      for (int p = first; p < first + cnt; ++p) {
+      do {
         f3 v1, e1, e2;
         int id;
         load_tri(s.tris, p, v1, e1, e2, id);
@@ -349,47 +446,67 @@ __device__ __forceinline__ Hit closest_traverse(const DevScene& s, f3 o, f3 d, c
         if (mt_intersect_fast(o, d, v1, e1, e2, t, u, v) && (t < h.t || (t == h.t && id > h.id))) {
           h.t = t; h.u = u; h.v = v; h.pos = p; h.id = id;
         }
-      }
+      } while (++p < end);
       leaf = 0;
-      if (cur != kDone && cur < 0) {
+      if (cur < kSpecial) {
         leaf = cur;
-        cur = st.next(h.t * kCullR);
+        cur = st.pop_within(h.t * kCullR);
       }
     }
     if (cur == kDone) return h;
+    if (cur == kRefill) {
+      st.refill();
+      cur = st.pop_within(h.t * kCullR);
+    }
   }
 }
 
 template <int SH, int CAP = kStackMax>
-__device__ __forceinline__ Hit closest_hit_body(const DevScene& s, f3 o, f3 d, uint2* shs, int stride, int* err) {
+__device__ __forceinline__ Hit closest_hit_body(const DevScene& s, f3 o, f3 d, uint32_t col, uint32_t stride,
+                                                int* err) {
   const SlabRay r = make_slab(o, d);
-  if (fma_slab_ok(r)) return closest_traverse<SH, CAP>(s, o, d, make_fma_slab(r), shs, stride, err);
-  return closest_traverse<SH, CAP>(s, o, d, r, shs, stride, err);
+  if (fma_slab_ok(r)) return closest_traverse<SH, CAP>(s, o, d, make_fma_slab(r), col, stride, err);
+  return closest_traverse<SH, CAP>(s, o, d, r, col, stride, err);
 }
 
-// Any hit at t >= 0 (shadow rays), same two-loop form; returns at the first hit.
+// Any hit at t >= 0 (shadow rays), same two-loop form; returns at the first hit.  Children
+// in slot order: nearest first measured slower for shadow rays.
 template <int SH, int CAP, class Ray>
-__device__ __forceinline__ AnyResult any_traverse(const DevScene& s, f3 o, f3 d, const Ray& r, uint2* shs,
-                                                  int stride, int* err) {
+__device__ __forceinline__ AnyResult any_traverse(const DevScene& s, f3 o, f3 d, const Ray& r, uint32_t col,
+                                                  uint32_t stride, int* err) {
   AnyResult res{0, 0u, 0u};
-  TraversalStack<SH, CAP> st(shs, stride);
+  ColumnStack<SH, CAP, false> st(col, stride);
   int cur = 0;
   int leaf = 0;
   for (;;) {
     while (cur >= 0) {
-      if (!visit_node4<false>(s.nodes, r, cur, kInf, st, res.nodes)) {
+      const char* nd = node_address(s.nodes, cur);
+      const int4 ref = __ldg(reinterpret_cast<const int4*>(nd + 96));
+      const Box4 b = child_boxes(nd, r);
+      ++res.nodes;
+      if (!st.reserve()) {
         atomicOr(err, kErrStack);
         return res;
       }
-      if (cur != kDone && cur < 0 && leaf == 0) {
+      follow_hits(st.top, stride, cur, ref, b.tn, b.tf);
+      if (!st.within_limit()) {
+        atomicOr(err, kErrStack);
+        return res;
+      }
+      if (cur < kSpecial && leaf == 0) {
         leaf = cur;
-        cur = st.next_any();
+        cur = st.pop();
       }
       if (!__any_sync(__activemask(), leaf == 0)) break;
     }
+    if (cur < kSpecial && leaf == 0) {
+      leaf = cur;
+      cur = st.pop();
+    }
     while (leaf != 0) {
-      const int first = leaf_first(leaf), cnt = leaf_count(leaf);
-      for (int p = first; p < first + cnt; ++p) {
+      int p = leaf_first(leaf);
+      const int end = p + leaf_count(leaf);
+      do {
         f3 v1, e1, e2;
         int id;
         load_tri(s.tris, p, v1, e1, e2, id);
@@ -399,33 +516,38 @@ __device__ __forceinline__ AnyResult any_traverse(const DevScene& s, f3 o, f3 d,
           res.hit = 1;
           return res;
         }
-      }
+      } while (++p < end);
       leaf = 0;
-      if (cur != kDone && cur < 0) {
+      if (cur < kSpecial) {
         leaf = cur;
-        cur = st.next_any();
+        cur = st.pop();
       }
     }
     if (cur == kDone) return res;
+    if (cur == kRefill) {
+      st.refill();
+      cur = st.pop();
+    }
   }
 }
 
 template <int SH, int CAP = kStackMax>
-__device__ __forceinline__ AnyResult any_hit_body(const DevScene& s, f3 o, f3 d, uint2* shs, int stride, int* err) {
+__device__ __forceinline__ AnyResult any_hit_body(const DevScene& s, f3 o, f3 d, uint32_t col, uint32_t stride,
+                                                  int* err) {
   const SlabRay r = make_slab(o, d);
-  if (fma_slab_ok(r)) return any_traverse<SH, CAP>(s, o, d, make_fma_slab(r), shs, stride, err);
-  return any_traverse<SH, CAP>(s, o, d, r, shs, stride, err);
+  if (fma_slab_ok(r)) return any_traverse<SH, CAP>(s, o, d, make_fma_slab(r), col, stride, err);
+  return any_traverse<SH, CAP>(s, o, d, r, col, stride, err);
 }
 
 // Out-of-line copies for the plain megakernel, which calls both traversals: keeping them
 // out of line bounds its register allocation.  The specialised wavefront kernels inline.
 template <int SH>
-__device__ __noinline__ Hit closest_hit_call(const DevScene& s, f3 o, f3 d, uint2* shs, int stride, int* err) {
-  return closest_hit_body<SH>(s, o, d, shs, stride, err);
+__device__ __noinline__ Hit closest_hit_call(const DevScene& s, f3 o, f3 d, uint32_t col, uint32_t stride, int* err) {
+  return closest_hit_body<SH>(s, o, d, col, stride, err);
 }
 template <int SH>
-__device__ __noinline__ AnyResult any_hit_call(const DevScene& s, f3 o, f3 d, uint2* shs, int stride, int* err) {
-  return any_hit_body<SH>(s, o, d, shs, stride, err);
+__device__ __noinline__ AnyResult any_hit_call(const DevScene& s, f3 o, f3 d, uint32_t col, uint32_t stride, int* err) {
+  return any_hit_body<SH>(s, o, d, col, stride, err);
 }
 
 // ------------------------------------------------------------------ two-level scenes
@@ -449,7 +571,8 @@ __device__ __forceinline__ void to_object(const DevInstance* I, f3 o, f3 d, f3& 
 
 // ANY: returns at the first hit (h.pos >= 0 then); otherwise the nearest hit.
 template <int SH, bool ANY>
-__device__ __noinline__ Hit traverse_instanced(const DevScene& s, f3 o, f3 d, uint2* shs, int stride, int* err) {
+__device__ __noinline__ Hit traverse_instanced(const DevScene& s, f3 o, f3 d, uint32_t col, uint32_t stride,
+                                               int* err) {
   Hit h;
   h.t = kInf; h.u = h.v = 0.0f; h.pos = -1; h.id = -1; h.nodes = 0; h.tests = 0;
   const SlabRay rw = make_slab(o, d);
@@ -459,15 +582,20 @@ __device__ __noinline__ Hit traverse_instanced(const DevScene& s, f3 o, f3 d, ui
   const float4* tris = nullptr;
   int id_off = 0;
   bool in_mesh = false;
-  TraversalStack<SH> st(shs, stride);
+  ColumnStack<SH, kStackMax, !ANY> st(col, stride);
   int cur = 0;
   for (;;) {
-    const float limit = ANY ? kInf : h.t * kCull;
     if (cur >= 0) {
-      if (!visit_node4<!ANY>(nodes, r, cur, limit, st, h.nodes)) {
+      const char* nd = node_address(nodes, cur);
+      const int4 ref = __ldg(reinterpret_cast<const int4*>(nd + 96));
+      const Box4 b = child_boxes(nd, r);
+      ++h.nodes;
+      if (!st.reserve()) {
         atomicOr(err, kErrStack);
         return h;
       }
+      if (ANY) follow_hits(st.top, stride, cur, ref, b.tn, b.tf);
+      else cur = follow_nearest(st, ref, b, h.t * kCull);
       continue;
     }
     if (cur == kDone) return h;
@@ -475,6 +603,8 @@ __device__ __noinline__ Hit traverse_instanced(const DevScene& s, f3 o, f3 d, ui
       r = rw;
       nodes = s.nodes;
       in_mesh = false;
+    } else if (cur == kRefill) {
+      st.refill();
     } else if (!in_mesh) {  // an instance: continue in its mesh, in object space
       const DevInstance* I = s.inst + leaf_first(cur);
       to_object(I, o, d, oo, od);
@@ -482,10 +612,11 @@ __device__ __noinline__ Hit traverse_instanced(const DevScene& s, f3 o, f3 d, ui
       nodes = I->nodes;
       tris = I->tris;
       id_off = I->id_offset;
-      if (!st.push(kExitMesh, -kInf)) {
+      if (!st.reserve()) {
         atomicOr(err, kErrStack);
         return h;
       }
+      st.push(kExitMesh, -kInf);
       in_mesh = true;
       cur = 0;
       continue;
@@ -508,7 +639,7 @@ __device__ __noinline__ Hit traverse_instanced(const DevScene& s, f3 o, f3 d, ui
         }
       }
     }
-    cur = ANY ? st.next_any() : st.next(h.t * kCull);
+    cur = ANY ? st.pop() : st.pop_within(h.t * kCull);
   }
 }
 
@@ -525,20 +656,22 @@ __device__ __forceinline__ const DevInstance* instance_of(const DevScene& s, int
 
 // CAP (inline traversals of flat scenes only): total stack entries, see TraversalStack.
 template <int SH, bool INLINE = false, int CAP = kStackMax>
-__device__ __forceinline__ Hit closest_hit(const DevScene& s, f3 o, f3 d, uint2* shs, int stride, int* err) {
-  if (s.inst) return traverse_instanced<SH, false>(s, o, d, shs, stride, err);
-  if (INLINE) return closest_hit_body<SH, CAP>(s, o, d, shs, stride, err);
-  return closest_hit_call<SH>(s, o, d, shs, stride, err);
+__device__ __forceinline__ Hit closest_hit(const DevScene& s, f3 o, f3 d, uint32_t col, uint32_t stride,
+                                            int* err) {
+  if (s.inst) return traverse_instanced<SH, false>(s, o, d, col, stride, err);
+  if (INLINE) return closest_hit_body<SH, CAP>(s, o, d, col, stride, err);
+  return closest_hit_call<SH>(s, o, d, col, stride, err);
 }
 
 template <int SH, bool INLINE = false, int CAP = kStackMax>
-__device__ __forceinline__ AnyResult any_hit(const DevScene& s, f3 o, f3 d, uint2* shs, int stride, int* err) {
+__device__ __forceinline__ AnyResult any_hit(const DevScene& s, f3 o, f3 d, uint32_t col, uint32_t stride,
+                                            int* err) {
   if (s.inst) {
-    const Hit h = traverse_instanced<SH, true>(s, o, d, shs, stride, err);
+    const Hit h = traverse_instanced<SH, true>(s, o, d, col, stride, err);
     return AnyResult{h.pos >= 0 ? 1 : 0, h.nodes, h.tests};
   }
-  if (INLINE) return any_hit_body<SH, CAP>(s, o, d, shs, stride, err);
-  return any_hit_call<SH>(s, o, d, shs, stride, err);
+  if (INLINE) return any_hit_body<SH, CAP>(s, o, d, col, stride, err);
+  return any_hit_call<SH>(s, o, d, col, stride, err);
 }
 
 // Traversal work counters, reduced per warp into the context's counter block:

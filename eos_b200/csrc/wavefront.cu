@@ -191,8 +191,7 @@ __device__ __forceinline__ void emit_secondary(const WfArgs& A, int* ctr, bool w
 template <bool PRIMARY, int SH, int CAP = kStackMax, bool TREE = false>
 __global__ void __launch_bounds__(256, 4) k_wf_closest(WfArgs A) {
   extern __shared__ uint2 shstack[];
-  uint2* shs = shstack + threadIdx.x;
-  const int stride = blockDim.x;
+  const uint32_t col = shared_address(shstack + threadIdx.x), stride = 8 * blockDim.x;
   int* ctr = A.ctr + A.k * kCtr;
   // primary rays of the chunk, or the secondary rays of bounce k-1
   const int n_in = budget(PRIMARY ? A.n_chunk : min(ctr[1 - kCtr], A.cap_r), A.work_limit, A.err);
@@ -242,7 +241,7 @@ __global__ void __launch_bounds__(256, 4) k_wf_closest(WfArgs A) {
       const DevJob& J = A.jobs[jb];
       if (valid) {
         ++nrays;
-        Hit h = closest_hit<SH, true, CAP>(J.s, o, d, shs, stride, A.err);
+        Hit h = closest_hit<SH, true, CAP>(J.s, o, d, col, stride, A.err);
         nodes += h.nodes;
         tests += h.tests;
         hit = h.pos >= 0;
@@ -357,9 +356,8 @@ __global__ void __launch_bounds__(256, 4) k_wf_closest(WfArgs A) {
 
 template <int SH, int CAP = kStackMax>
 __global__ void __launch_bounds__(256, 4) k_wf_any(WfArgs A) {
-  extern __shared__ uint2 shstack[];
-  uint2* shs = shstack + threadIdx.x;
-  const int stride = blockDim.x;
+  extern __shared__ int shrefs[];
+  const uint32_t col = shared_address(shrefs + threadIdx.x), stride = 4 * blockDim.x;
   int* ctr = A.ctr + A.k * kCtr;
   const int n = budget(min(ctr[2], A.cap_s), A.work_limit, A.err);
   unsigned long long nodes = 0, tests = 0;
@@ -373,7 +371,7 @@ __global__ void __launch_bounds__(256, 4) k_wf_any(WfArgs A) {
       int key = __float_as_int(s.b.w);
       const DevJob& J = A.jobs[key >> 5];
       AnyResult ar =
-          any_hit<SH, true, CAP>(J.s, mk3(s.a.x, s.a.y, s.a.z), mk3(s.b.x, s.b.y, s.b.z), shs, stride, A.err);
+          any_hit<SH, true, CAP>(J.s, mk3(s.a.x, s.a.y, s.a.z), mk3(s.b.x, s.b.y, s.b.z), col, stride, A.err);
       nodes += ar.nodes;
       tests += ar.tests;
       if (ar.hit) atomicOr(&A.masks[hi], 1u << (key & 31));
@@ -615,7 +613,7 @@ struct Overlap {
 
 template <int SH>
 eos_status launch_sequence(cudaStream_t st, int num_sms, const WfArgs& base, const Chunk* chunks, int n_chunks,
-                           int depth, int block, int grid_closest, int grid_any, int* ctr, size_t smem,
+                           int depth, int block, int grid_closest, int grid_any, int* ctr, size_t smem, size_t smem_a,
                            bool small_stack, bool tree, StageTimer tm, const Overlap& ov, uint32_t& launches) {
   const int grid_lin = num_sms * 8;
   const StageKernels<SH> K = StageKernels<SH>::get(small_stack, tree);
@@ -652,7 +650,7 @@ eos_status launch_sequence(cudaStream_t st, int num_sms, const WfArgs& base, con
         EOS_CUDA(cudaStreamWaitEvent(st2, ov.ev_closest[k], 0));
       }
       EOS_TRY(tm.begin());
-      K.any<<<grid_any, block, smem, st2>>>(A);
+      K.any<<<grid_any, block, smem_a, st2>>>(A);
       EOS_TRY(tm.end(1));
       if (split) {
         EOS_CUDA(cudaEventRecord(ov.ev_any[k], st2));
@@ -717,7 +715,7 @@ struct LaunchConfig {
   int block, sh, qchunk, grid_c, grid_a;
   bool small_stack;  // test limit: 8-entry traversal stacks (chain mode)
   bool tree;         // ray-tree mode
-  size_t smem;
+  size_t smem, smem_a;  // stack columns of the nearest-hit (ref, distance) and shadow (ref) kernels
 };
 
 template <int SH>
@@ -726,11 +724,11 @@ void configure(LaunchConfig& c, int num_sms) {
   if (c.smem > 48 * 1024) {  // opt in to more than the default 48 KB of dynamic shared memory
     cudaFuncSetAttribute(K.closest_primary, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)c.smem);
     cudaFuncSetAttribute(K.closest, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)c.smem);
-    cudaFuncSetAttribute(K.any, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)c.smem);
+    cudaFuncSetAttribute(K.any, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)c.smem_a);
   }
   int occ_c = 0, occ_a = 0;
   cudaOccupancyMaxActiveBlocksPerMultiprocessor(&occ_c, K.closest, c.block, c.smem);
-  cudaOccupancyMaxActiveBlocksPerMultiprocessor(&occ_a, K.any, c.block, c.smem);
+  cudaOccupancyMaxActiveBlocksPerMultiprocessor(&occ_a, K.any, c.block, c.smem_a);
   c.grid_c = num_sms * std::max(1, occ_c);
   c.grid_a = num_sms * std::max(1, occ_a);
 }
@@ -744,6 +742,7 @@ LaunchConfig launch_config(const eos_render_params& p, int num_sms, bool small_s
   c.small_stack = small_stack && !tree;
   if (c.small_stack) c.sh = 8;
   c.smem = (size_t)c.sh * c.block * sizeof(uint2);
+  c.smem_a = (size_t)c.sh * c.block * sizeof(int);
   if (c.sh == 8) configure<8>(c, num_sms);
   else if (c.sh == 16) configure<16>(c, num_sms);
   else configure<32>(c, num_sms);
@@ -754,12 +753,12 @@ eos_status run_sequence(cudaStream_t st, int num_sms, const LaunchConfig& lc, co
                         int n_chunks, int depth, StageTimer tm, const Overlap& ov, uint32_t& launches) {
   if (lc.sh == 8)
     return launch_sequence<8>(st, num_sms, A, chunks, n_chunks, depth, lc.block, lc.grid_c, lc.grid_a, A.ctr, lc.smem,
-                              lc.small_stack, lc.tree, tm, ov, launches);
+                              lc.smem_a, lc.small_stack, lc.tree, tm, ov, launches);
   if (lc.sh == 16)
     return launch_sequence<16>(st, num_sms, A, chunks, n_chunks, depth, lc.block, lc.grid_c, lc.grid_a, A.ctr,
-                               lc.smem, false, lc.tree, tm, ov, launches);
+                               lc.smem, lc.smem_a, false, lc.tree, tm, ov, launches);
   return launch_sequence<32>(st, num_sms, A, chunks, n_chunks, depth, lc.block, lc.grid_c, lc.grid_a, A.ctr, lc.smem,
-                             false, lc.tree, tm, ov, launches);
+                             lc.smem_a, false, lc.tree, tm, ov, launches);
 }
 
 }  // namespace
