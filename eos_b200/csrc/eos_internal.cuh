@@ -2,6 +2,7 @@
 #pragma once
 #include <cuda_runtime.h>
 #include <stdint.h>
+#include <string.h>
 
 #include <map>
 #include <memory>
@@ -50,7 +51,12 @@ inline eos_status err_to_status(int e) {
 //  ref: interior record index; leaf 0x80000000 | (count-1) << 25 | first (sorted positions
 //  [first, first + count), count <= 32, first < 2^25); 0xC0000000 for an unused slot,
 //  whose box is lo = +inf, hi = -inf.  count: triangles of a leaf, 0 interior, -1 unused.
-//  A binary tree (width 2) fills two slots per record.
+//  A binary tree (width 2) fills two slots per record.  Chunk j of record n is stored at
+//  float4 j ^ (n & 7) of the record (node_chunk): the lanes of a warp read the same chunk of
+//  different records at once, and without the swizzle those 16 bytes lie in the same four
+//  L1 banks of every record, one wavefront per record.  Measured (shadow rays of a 1080p
+//  view of 1.06M triangles): bank conflicts 26.1M -> 6.7M, 574 -> 553 us; 4K view of 4.5M
+//  triangles 66.5 -> 61.7 ms.  Scene files hold the chunks in order.
 //
 //  Triangle record (intersection), 48 B = 3 x float4, sorted (Morton) order:
 //    [0] v1.x v1.y v1.z e1.x   [1] e1.y e1.z e2.x e2.y   [2] e2.z id(int) - -
@@ -69,6 +75,9 @@ struct __align__(16) DevInstance {
   const int32_t* pos_of_id;  // the mesh's triangle id -> sorted position (the adjoint's replay)
 };
 static_assert(sizeof(DevInstance) % 16 == 0 && alignof(DevInstance) == 16, "minv is read as float4");
+
+// Position of chunk j in node record n; also the chunk at position j (an involution).
+__host__ __device__ __forceinline__ int node_chunk(int n, int j) { return j ^ (n & 7); }
 
 struct DevScene {
   const float4* nodes;
@@ -203,6 +212,13 @@ eos_status build_scene(eos_ctx* ctx, eos_scene* sc, const float* d_verts, const 
 // Morton position p, *depth = tree depth (above 4 * kStackMax nothing is written).
 eos_status build_ploc(eos_ctx* ctx, int n, const float4* blo, const float4* bhi, int2* child, int2* range,
                       int* parent, uint32_t* perm, int* depth);
+
+// Host copy of node record n between its chunk order and the device's (either way).
+inline void swizzle_record(void* rec, long long n) {
+  float4 in[8], *out = static_cast<float4*>(rec);
+  memcpy(in, rec, sizeof in);
+  for (int j = 0; j < 8; ++j) out[node_chunk((int)(n & 7), j)] = in[j];
+}
 
 // True when some material is both reflective and transparent (the scene renders ray trees).
 inline bool has_branching(const eos_material* m, uint32_t n) {

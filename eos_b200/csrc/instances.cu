@@ -63,7 +63,8 @@ struct Box {
   }
 };
 
-// Box of a mesh scene: the union of the used slots of its root record.
+// Box of a mesh scene: the union of the used slots of its root record (record 0: its chunks
+// are in order).
 eos_status mesh_root_box(const eos_scene* m, Box& b) {
   float rec[32];
   EOS_CUDA(cudaMemcpy(rec, m->d_nodes, sizeof rec, cudaMemcpyDeviceToHost));
@@ -202,6 +203,7 @@ int write_records_host(const std::vector<BNode>& bn, int root, std::vector<float
     }
     std::swap(frontier, next);
   }
+  for (int n = 0; n < n_rec; ++n) swizzle_record(out.data() + 32 * (size_t)n, n);
   return levels;
 }
 

@@ -344,11 +344,13 @@ __global__ void k_refit(int n, const int2* __restrict__ child, const int2* __res
 //   [7] count[4]: triangles of a leaf, 0 for an interior child, -1 for an unused slot
 constexpr int kEmptyRef = (int)0xC0000000;
 
-__device__ __forceinline__ void write_record(float4* o, const float (&v)[6][4], const int (&ref)[4],
+__device__ __forceinline__ void write_record(float4* nodes, int n, const float (&v)[6][4], const int (&ref)[4],
                                              const int (&cnt)[4]) {
-  for (int a = 0; a < 6; ++a) o[a] = make_float4(v[a][0], v[a][1], v[a][2], v[a][3]);
-  o[6] = make_float4(__int_as_float(ref[0]), __int_as_float(ref[1]), __int_as_float(ref[2]), __int_as_float(ref[3]));
-  o[7] = make_float4(__int_as_float(cnt[0]), __int_as_float(cnt[1]), __int_as_float(cnt[2]), __int_as_float(cnt[3]));
+  float4* o = nodes + 8 * (size_t)n;
+#pragma unroll
+  for (int a = 0; a < 6; ++a) o[node_chunk(n, a)] = make_float4(v[a][0], v[a][1], v[a][2], v[a][3]);
+  o[node_chunk(n, 6)] = make_float4(__int_as_float(ref[0]), __int_as_float(ref[1]), __int_as_float(ref[2]), __int_as_float(ref[3]));
+  o[node_chunk(n, 7)] = make_float4(__int_as_float(cnt[0]), __int_as_float(cnt[1]), __int_as_float(cnt[2]), __int_as_float(cnt[3]));
 }
 
 // One level of the wide records, in two passes over the frontier (binary node, record):
@@ -455,7 +457,7 @@ __global__ void __launch_bounds__(kScanBlock) k_wide_write(int n, const int2* __
       cnt[i] = 0;
     }
   }
-  write_record(wnodes + 8 * (size_t)frontier_in[t].y, v, ref, cnt);
+  write_record(wnodes, frontier_in[t].y, v, ref, cnt);
 }
 
 // Root record of a scene with 0 or 1 triangle (no binary interior node exists).
@@ -473,7 +475,7 @@ __global__ void k_small_root(int n, const float4* __restrict__ blo, const float4
     ref[0] = pack_leaf(0, 1);
     cnt[0] = 1;
   }
-  write_record(nodes, v, ref, cnt);
+  write_record(nodes, 0, v, ref, cnt);
 }
 
 inline int grid_for(size_t n, int block) { return (int)std::max<size_t>(1, (n + block - 1) / block); }

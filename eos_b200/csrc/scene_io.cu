@@ -94,6 +94,15 @@ cudaError_t copy_range(const std::vector<Part>& ps, size_t at, size_t len, unsig
   return cudaSuccess;
 }
 
+// The node records of payload bytes [at, at + len), between the file's chunk order (lo.x ..
+// count) and the device's.  The records come first in the payload and a chunk holds whole
+// ones.
+void swizzle_nodes(unsigned char* host, size_t at, size_t len, size_t n_nodes) {
+  static_assert(kChunk % 128 == 0, "whole node records per chunk");
+  for (size_t n = at / 128; n < std::min(n_nodes, (at + len) / 128); ++n)
+    eos::swizzle_record(host + (128 * n - at), (long long)n);
+}
+
 // Two pinned chunks of the context (grown once) and one event per chunk.
 struct Staging {
   unsigned char* buf[2] = {nullptr, nullptr};
@@ -172,6 +181,7 @@ extern "C" eos_status eos_scene_save(const eos_scene* scene, const char* path) {
     cuda_ok = cuda_ok && cudaEventSynchronize(sg.done[i & 1]) == cudaSuccess;
     if (!cuda_ok) break;
     const size_t len = std::min(kChunk, total - i * kChunk);
+    swizzle_nodes(sg.buf[i & 1], i * kChunk, len, sc->n_nodes);
     cs.update(sg.buf[i & 1], len);
     ok = std::fwrite(sg.buf[i & 1], 1, len, f) == len;
   }
@@ -239,6 +249,7 @@ extern "C" eos_status eos_scene_load(eos_ctx* ctx, const char* path, eos_scene**
     if (used[k] && cudaEventSynchronize(sg.done[k]) != cudaSuccess) return fail(EOS_ERR_CUDA);
     if (std::fread(sg.buf[k], 1, len, f) != len) return fail(EOS_ERR_PARSE);
     cs.update(sg.buf[k], len);
+    swizzle_nodes(sg.buf[k], at, len, h.n_nodes);
     if (copy_range(ps, at, len, sg.buf[k], true, ctx->stream) != cudaSuccess ||
         cudaEventRecord(sg.done[k], ctx->stream) != cudaSuccess)
       return fail(EOS_ERR_CUDA);

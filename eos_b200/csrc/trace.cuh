@@ -26,14 +26,14 @@ constexpr float kCull = 1.000244140625f;       // 1 + 2^-12
 constexpr float kParallelEps = 1e-30f;
 constexpr float kRayEps = 1e-3f;               // shadow / mirror ray offset, src/RayTracer.cpp:305
 
-// Ray prepared for box tests.  sx / sy / sz select the near plane of each axis in a node
-// record ([0..2] = lo.xyz, [3..5] = hi.xyz): 0 (lo) for a direction component >= 0 or a
-// parallel axis, 3 (hi) otherwise; the far plane is the other one.  The near and far
+// Ray prepared for box tests.  sx / sy / sz are 16 x the near plane's chunk of each axis in a
+// node record (chunks 0..2 = lo.xyz, 3..5 = hi.xyz): lo for a direction component >= 0 or a
+// parallel axis, hi otherwise; the far plane is the other one.  The near and far
 // distances are then (near - o) / d and (far - o) / d directly, the same values the
 // min / max of the two plane distances would give.
 struct SlabRay {
   float ox, oy, oz, ix, iy, iz;
-  int sx, sy, sz;
+  uint32_t sx, sy, sz;
   bool par;
 };
 
@@ -44,9 +44,9 @@ __device__ __forceinline__ SlabRay make_slab(f3 o, f3 d) {
   r.ix = px ? 0.0f : 1.0f / d.x;
   r.iy = py ? 0.0f : 1.0f / d.y;
   r.iz = pz ? 0.0f : 1.0f / d.z;
-  r.sx = (px || d.x >= 0.0f) ? 0 : 3;
-  r.sy = (py || d.y >= 0.0f) ? 0 : 3;
-  r.sz = (pz || d.z >= 0.0f) ? 0 : 3;
+  r.sx = (px || d.x >= 0.0f) ? 0u : 48u;
+  r.sy = (py || d.y >= 0.0f) ? 16u : 64u;
+  r.sz = (pz || d.z >= 0.0f) ? 32u : 80u;
   r.par = px || py || pz;
   return r;
 }
@@ -95,7 +95,7 @@ __device__ __forceinline__ void slab_range(const SlabRay& r, float nx, float ny,
 // the exact form (fma_slab_ok).
 struct FmaSlabRay {
   float ix, iy, iz, nx, ny, nz, fx, fy, fz;
-  int sx, sy, sz;
+  uint32_t sx, sy, sz;
 };
 
 __device__ __forceinline__ bool fma_slab_ok(const SlabRay& r) {
@@ -309,15 +309,18 @@ struct Box4 {
   float tn[4], tf[4];
 };
 
-__device__ __forceinline__ const char* node_address(const float4* nodes, int node) {
-  return reinterpret_cast<const char*>(nodes) + (size_t)(uint32_t)node * 128u;
+// Address of node record `node`, whose chunk j lies at (address ^ 16 j): the record is
+// 128-byte aligned and its chunks are stored swizzled by the low bits of its index (kNode
+// record layout, eos_internal.cuh).
+__device__ __forceinline__ size_t node_address(const float4* nodes, int node) {
+  return (reinterpret_cast<size_t>(nodes) + (size_t)(uint32_t)node * 128u) ^ (((uint32_t)node & 7u) << 4);
 }
 
-__device__ __forceinline__ float4 ldg4(const char* p) { return __ldg(reinterpret_cast<const float4*>(p)); }
+__device__ __forceinline__ float4 ldg4(size_t a) { return __ldg(reinterpret_cast<const float4*>(a)); }
 
-__device__ __forceinline__ Box4 child_boxes(const char* nd, const SlabRay& r) {
-  const float4 lx = ldg4(nd + 16 * r.sx), ly = ldg4(nd + 16 * r.sy + 16), lz = ldg4(nd + 16 * r.sz + 32);
-  const float4 hx = ldg4(nd - 16 * r.sx + 48), hy = ldg4(nd - 16 * r.sy + 64), hz = ldg4(nd - 16 * r.sz + 80);
+__device__ __forceinline__ Box4 child_boxes(size_t nd, const SlabRay& r) {
+  const float4 lx = ldg4(nd ^ r.sx), ly = ldg4(nd ^ r.sy), lz = ldg4(nd ^ r.sz);  // near planes
+  const float4 hx = ldg4(nd ^ r.sx ^ 48u), hy = ldg4(nd ^ r.sy ^ 80u), hz = ldg4(nd ^ r.sz ^ 112u);  // far planes
   Box4 b;
   slab_range(r, lx.x, ly.x, lz.x, hx.x, hy.x, hz.x, b.tn[0], b.tf[0]);
   slab_range(r, lx.y, ly.y, lz.y, hx.y, hy.y, hz.y, b.tn[1], b.tf[1]);
@@ -348,9 +351,9 @@ __device__ __forceinline__ void axis4(float4 p, float i, float c, float* o) {
   unpack2(fma2(pack2(p.z, p.w), dup2(i), dup2(c)), o[2], o[3]);
 }
 
-__device__ __forceinline__ Box4 child_boxes(const char* nd, const FmaSlabRay& r) {
-  const float4 lx = ldg4(nd + 16 * r.sx), ly = ldg4(nd + 16 * r.sy + 16), lz = ldg4(nd + 16 * r.sz + 32);
-  const float4 hx = ldg4(nd - 16 * r.sx + 48), hy = ldg4(nd - 16 * r.sy + 64), hz = ldg4(nd - 16 * r.sz + 80);
+__device__ __forceinline__ Box4 child_boxes(size_t nd, const FmaSlabRay& r) {
+  const float4 lx = ldg4(nd ^ r.sx), ly = ldg4(nd ^ r.sy), lz = ldg4(nd ^ r.sz);  // near planes
+  const float4 hx = ldg4(nd ^ r.sx ^ 48u), hy = ldg4(nd ^ r.sy ^ 80u), hz = ldg4(nd ^ r.sz ^ 112u);  // far planes
   float x[4], y[4], z[4];
   Box4 b;
   axis4(lx, r.ix, r.nx, x);
@@ -410,8 +413,8 @@ __device__ __forceinline__ Hit closest_traverse(const DevScene& s, f3 o, f3 d, c
   int leaf = 0;  // parked leaf (0 = none)
   for (;;) {
     while (cur >= 0) {
-      const char* nd = node_address(s.nodes, cur);
-      const int4 ref = __ldg(reinterpret_cast<const int4*>(nd + 96));
+      size_t nd = node_address(s.nodes, cur);
+      const int4 ref = __ldg(reinterpret_cast<const int4*>(nd ^ 96u));
       const Box4 b = child_boxes(nd, r);
       ++h.nodes;
       if (!st.reserve()) {
@@ -480,8 +483,8 @@ __device__ __forceinline__ AnyResult any_traverse(const DevScene& s, f3 o, f3 d,
   int leaf = 0;
   for (;;) {
     while (cur >= 0) {
-      const char* nd = node_address(s.nodes, cur);
-      const int4 ref = __ldg(reinterpret_cast<const int4*>(nd + 96));
+      size_t nd = node_address(s.nodes, cur);
+      const int4 ref = __ldg(reinterpret_cast<const int4*>(nd ^ 96u));
       const Box4 b = child_boxes(nd, r);
       ++res.nodes;
       if (!st.reserve()) {
@@ -586,8 +589,8 @@ __device__ __noinline__ Hit traverse_instanced(const DevScene& s, f3 o, f3 d, ui
   int cur = 0;
   for (;;) {
     if (cur >= 0) {
-      const char* nd = node_address(nodes, cur);
-      const int4 ref = __ldg(reinterpret_cast<const int4*>(nd + 96));
+      size_t nd = node_address(nodes, cur);
+      const int4 ref = __ldg(reinterpret_cast<const int4*>(nd ^ 96u));
       const Box4 b = child_boxes(nd, r);
       ++h.nodes;
       if (!st.reserve()) {
