@@ -160,10 +160,12 @@ __device__ __forceinline__ int budget(int n, int work_limit, int* err) {
   return work_limit;
 }
 
-// The wavefront traversal kernels are capped at 64 registers (blocks up to 256, 4 per SM):
-// measured faster than no cap (77 registers) and than caps of 56 or 48 (spills).  CAP is
-// the traversal stack's size (TraversalStack): kStackMax, or SH for the small-stack test
-// limit.
+// The nearest-hit kernels are capped at 64 registers (blocks up to 256, 4 per SM): 56 and 72
+// cost 2 and 0.5 % of a four-view 1080p batch of 1.06M triangles (5,107 us), 5 and 4 % of a
+// 30-job batch.  The shadow kernels are capped at 56, one more block of 128 threads per SM
+// than at 64 for 12 B less of spill stores: 5,107 -> 5,049 us; 48 (196 B of spills) 5,521, 72
+// 5,131.  CAP is the traversal stack's size (ColumnStack): kStackMax, or SH for the
+// small-stack test limit.
 // Appends the secondary rays of the lanes with `want` to R_k+1 (ballot / popc compaction,
 // one atomic per warp); node = the ray-tree node of the ray (0 outside tree mode).
 // Warp-uniform: every lane calls it.
@@ -355,7 +357,7 @@ __global__ void __launch_bounds__(256, 4) k_wf_closest(WfArgs A) {
 }
 
 template <int SH, int CAP = kStackMax>
-__global__ void __launch_bounds__(256, 4) k_wf_any(WfArgs A) {
+__global__ void __maxnreg__(56) k_wf_any(WfArgs A) {
   extern __shared__ int shrefs[];
   const uint32_t col = shared_address(shrefs + threadIdx.x), stride = 4 * blockDim.x;
   int* ctr = A.ctr + A.k * kCtr;
