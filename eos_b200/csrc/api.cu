@@ -43,6 +43,7 @@ eos_ctx::~eos_ctx() {
   if (d_counts) cudaFree(d_counts);
   if (ev0) cudaEventDestroy(ev0);
   if (ev1) cudaEventDestroy(ev1);
+  if (pool) cudaMemPoolDestroy(pool);
   if (own_stream) cudaStreamDestroy(own_stream);
 }
 
@@ -58,7 +59,13 @@ void* scratch(eos_ctx* ctx, const char* name, size_t bytes, eos_status* st) {
     b.bytes = 0;
   }
   size_t want = std::max<size_t>(bytes, 256);
-  if (cudaMalloc(&b.ptr, want) != cudaSuccess) {
+  cudaError_t e = cudaMalloc(&b.ptr, want);
+  if (e != cudaSuccess) {  // again with what the pool keeps given back
+    cudaGetLastError();
+    cudaMemPoolTrimTo(ctx->pool, 0);
+    e = cudaMalloc(&b.ptr, want);
+  }
+  if (e != cudaSuccess) {
     cudaGetLastError();
     b.ptr = nullptr;
     if (st) *st = EOS_ERR_OOM;
@@ -66,6 +73,25 @@ void* scratch(eos_ctx* ctx, const char* name, size_t bytes, eos_status* st) {
   }
   b.bytes = want;
   return b.ptr;
+}
+
+cudaError_t scene_alloc(eos_ctx* ctx, void** p, size_t bytes) {
+  *p = nullptr;
+  cudaError_t e = cudaMallocFromPoolAsync(p, bytes, ctx->pool, ctx->own_stream);
+  if (e == cudaErrorMemoryAllocation) {  // again with what the pool keeps given back
+    cudaGetLastError();
+    cudaMemPoolTrimTo(ctx->pool, 0);
+    e = cudaMallocFromPoolAsync(p, bytes, ctx->pool, ctx->own_stream);
+  }
+  if (e == cudaSuccess) e = cudaStreamSynchronize(ctx->own_stream);
+  return e;
+}
+
+void scene_free(eos_ctx* ctx, void* const* p, int n) {
+  cudaDeviceSynchronize();
+  for (int k = 0; k < n; ++k)
+    if (p[k]) cudaFreeAsync(p[k], ctx->own_stream);
+  cudaStreamSynchronize(ctx->own_stream);
 }
 
 namespace {
@@ -314,6 +340,16 @@ eos_status eos_ctx_create(int32_t device, eos_ctx** out) {
     cudaDeviceGetAttribute(&ctx->num_sms, cudaDevAttrMultiProcessorCount, device);
     if (cudaStreamCreateWithFlags(&ctx->own_stream, cudaStreamNonBlocking) != cudaSuccess) { st = EOS_ERR_CUDA; break; }
     ctx->stream = ctx->own_stream;
+    cudaMemPoolProps props = {};
+    props.allocType = cudaMemAllocationTypePinned;
+    props.location.type = cudaMemLocationTypeDevice;
+    props.location.id = device;
+    unsigned long long keep = kPoolKeep;
+    if (cudaMemPoolCreate(&ctx->pool, &props) != cudaSuccess ||
+        cudaMemPoolSetAttribute(ctx->pool, cudaMemPoolAttrReleaseThreshold, &keep) != cudaSuccess) {
+      st = EOS_ERR_CUDA;
+      break;
+    }
     if (cudaEventCreate(&ctx->ev0) != cudaSuccess || cudaEventCreate(&ctx->ev1) != cudaSuccess) { st = EOS_ERR_CUDA; break; }
     if (cudaMalloc(&ctx->d_err, sizeof(int)) != cudaSuccess) { st = EOS_ERR_OOM; break; }
     if (cudaMalloc(&ctx->d_counts, kCounters * sizeof(unsigned long long)) != cudaSuccess) { st = EOS_ERR_OOM; break; }
@@ -420,8 +456,8 @@ eos_status eos_scene_create(eos_ctx* ctx, const float* verts, const float* norma
   const uint32_t* dt = (const uint32_t*)stage_in(ctx, "in.tris", tris, 12ull * n_tris, &st);
   const uint32_t* dob = (const uint32_t*)stage_in(ctx, "in.obj", tri_obj, 4ull * n_tris, &st);
   if (st != EOS_OK) return fail(st);
-  if (cudaMalloc(&sc->d_mats, sizeof(eos_material) * n_materials) != cudaSuccess) return fail(EOS_ERR_OOM);
-  if (cudaMalloc(&sc->d_lights, sizeof(eos_light) * std::max<uint32_t>(1, n_lights)) != cudaSuccess)
+  if (scene_alloc(ctx, &sc->d_mats, sizeof(eos_material) * n_materials) != cudaSuccess) return fail(EOS_ERR_OOM);
+  if (scene_alloc(ctx, &sc->d_lights, sizeof(eos_light) * std::max<uint32_t>(1, n_lights)) != cudaSuccess)
     return fail(EOS_ERR_OOM);
   sc->device_bytes += sizeof(eos_material) * n_materials + sizeof(eos_light) * std::max<uint32_t>(1, n_lights);
   sc->dev.n_obj = (int)n_materials;
@@ -455,8 +491,7 @@ eos_status eos_scene_destroy(eos_scene* sc) {
   }
   void* bufs[] = {sc->d_nodes, sc->d_tris, sc->d_shade, sc->d_pos_of_id, sc->d_mats, sc->d_lights, sc->d_codes,
                   sc->d_order, sc->d_inst};
-  for (void* b : bufs)
-    if (b) cudaFree(b);
+  if (sc->ctx) scene_free(sc->ctx, bufs, (int)(sizeof bufs / sizeof bufs[0]));
   delete sc;
   return EOS_OK;
 }
