@@ -114,8 +114,8 @@ struct eos_ctx {
   cudaMemPool_t pool = nullptr;  // scene arrays (scene_alloc)
   void* pinned = nullptr;
   size_t pinned_bytes = 0;
-  // PLOC round read-back ring (made on first use): mapped pinned slots the merge kernel
-  // writes, and one event per slot
+  // read-back ring of the builders' launches that run ahead of the host (made on first use,
+  // ring.cuh): mapped pinned slots, and one event per slot
   int* ring_host = nullptr;
   int* ring_dev = nullptr;
   cudaEvent_t ring_ev[4] = {};
@@ -218,11 +218,12 @@ bool is_device_ptr(const void* p);
 eos_status build_scene(eos_ctx* ctx, eos_scene* sc, const float* d_verts, const float* d_normals,
                        uint32_t n_verts, const uint32_t* d_tris, const uint32_t* d_obj, uint32_t n_tris);
 
-// PLOC hierarchy over n >= 2 leaves with boxes at blo / bhi[n-1+p] in Morton order
-// (ploc.cu): child / range / parent in the refit's layout, perm[p] = record position of
-// Morton position p, *depth = tree depth (above 4 * kStackMax nothing is written).
-eos_status build_ploc(eos_ctx* ctx, int n, const float4* blo, const float4* bhi, int2* child, int2* range,
-                      int* parent, uint32_t* perm, int* depth);
+// PLOC hierarchy over n >= 2 leaves with boxes at blo / bhi[n-1+p] in Morton order (ploc.cu):
+// child / count / box / cost / leaf decision of the interior nodes in creation order (root
+// n-2), perm[p] = record position of Morton position p, first[v] = that of a collapsed
+// subtree, *depth = tree depth (above 4 * kStackMax first and perm are incomplete).
+eos_status build_ploc(eos_ctx* ctx, int n, int max_leaf, int sah, float4* blo, float4* bhi, int2* child, int* count,
+                      int* first, uint32_t* perm, int* depth);
 
 // Host copy of node record n between its chunk order and the device's (either way).
 inline void swizzle_record(void* rec, long long n) {

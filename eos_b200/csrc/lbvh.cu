@@ -1,6 +1,6 @@
 // GPU BVH build: Morton codes -> stable radix sort -> hierarchy (Karras radix tree, or
-// PLOC clustering in ploc.cu) -> atomic refit -> 128-byte node records (4-wide, or 2
-// children per record) / 48-byte triangle records.
+// PLOC clustering in ploc.cu) -> refit (LBVH; PLOC makes its boxes as it merges) -> 128-byte
+// node records (4-wide, or 2 children per record) / 48-byte triangle records.
 //
 // Replaces the reference's CPU top-down median/SAH build (src/BVH.cpp:97-111,549-606) and
 // its SoA upload (src/cudaStructures.cu:36-174,274-405).  The Morton encoder is the
@@ -10,9 +10,10 @@
 // Primitive order = stable sort by (code, triangle id).
 #include <algorithm>
 
-
 #include "eos_internal.cuh"
+#include "ring.cuh"
 #include "scan.cuh"
+#include "tree.cuh"
 
 namespace eos {
 namespace {
@@ -214,7 +215,7 @@ __device__ __forceinline__ int common_prefix(const uint32_t* __restrict__ k, int
 // Internal node i of n-1 (Karras 2012, "Maximizing parallelism in the construction of
 // BVHs, octrees and k-d trees").  Node numbering: interior 0..n-2, leaf p -> n-1+p.
 __global__ void k_karras(const uint32_t* __restrict__ k, int n, int2* __restrict__ child,
-                         int2* __restrict__ range, int* __restrict__ parent) {
+                         int* __restrict__ first_of, int* __restrict__ count, int* __restrict__ parent) {
   int i = blockIdx.x * blockDim.x + threadIdx.x;
   if (i >= n - 1) return;
   int d = (common_prefix(k, n, i, i + 1) - common_prefix(k, n, i, i - 1)) >= 0 ? 1 : -1;
@@ -237,13 +238,35 @@ __global__ void k_karras(const uint32_t* __restrict__ k, int n, int2* __restrict
   int left = (first == gamma) ? (n - 1 + gamma) : gamma;
   int right = (last == gamma + 1) ? (n - 1 + gamma + 1) : gamma + 1;
   child[i] = make_int2(left, right);
-  range[i] = make_int2(first, last);
+  first_of[i] = first;
+  count[i] = last - first + 1;
   parent[left] = i;
   parent[right] = i;
 }
 
-// Triangle records, leaf boxes, id -> position map.  The triangle at Morton position m
-// goes to record position p = perm[m] (perm NULL: p = m).
+// Box of a triangle; .w: SAH cost of one triangle, leaf flag.
+__device__ __forceinline__ void triangle_box(f3 v1, f3 v2, f3 v3, float4& lo, float4& hi) {
+  lo = make_float4(fminf(fminf(v1.x, v2.x), v3.x), fminf(fminf(v1.y, v2.y), v3.y), fminf(fminf(v1.z, v2.z), v3.z),
+                   1.0f);
+  hi = make_float4(fmaxf(fmaxf(v1.x, v2.x), v3.x), fmaxf(fmaxf(v1.y, v2.y), v3.y), fmaxf(fmaxf(v1.z, v2.z), v3.z),
+                   1.0f);
+}
+
+// Leaf boxes in Morton order (the PLOC builder's input; its records come after the tree,
+// in the tree's leaf order).
+__global__ void k_leaf_boxes(const float* __restrict__ verts, uint32_t n_verts, const uint32_t* __restrict__ tris,
+                             const uint32_t* __restrict__ order, int n, float4* __restrict__ blo,
+                             float4* __restrict__ bhi) {
+  const int m = blockIdx.x * blockDim.x + threadIdx.x;
+  if (m >= n) return;
+  const uint32_t id = order[m];
+  uint32_t a = tris[3 * (size_t)id], b = tris[3 * (size_t)id + 1], c = tris[3 * (size_t)id + 2];
+  if (a >= n_verts || b >= n_verts || c >= n_verts) a = b = c = 0;  // flagged in k_centroids
+  triangle_box(load_vert(verts, a), load_vert(verts, b), load_vert(verts, c), blo[n - 1 + m], bhi[n - 1 + m]);
+}
+
+// Triangle records, id -> position map and (blo not NULL) leaf boxes.  The triangle at Morton
+// position m goes to record position p = perm[m] (perm NULL: p = m).
 __global__ void k_records(const float* __restrict__ verts, const float* __restrict__ normals, uint32_t n_verts,
                           const uint32_t* __restrict__ tris, const uint32_t* __restrict__ obj,
                           const uint32_t* __restrict__ order, const uint32_t* __restrict__ perm, int n, uint32_t n_obj,
@@ -270,11 +293,7 @@ __global__ void k_records(const float* __restrict__ verts, const float* __restri
   }
   srec[3 * (size_t)p + 2] = make_float4(n3.z, __int_as_float((int)ob), 0.0f, 0.0f);
   pos_of_id[id] = p;
-  size_t leaf = (size_t)(n - 1) + p;  // .w: SAH cost of one triangle, leaf flag
-  blo[leaf] = make_float4(fminf(fminf(v1.x, v2.x), v3.x), fminf(fminf(v1.y, v2.y), v3.y),
-                          fminf(fminf(v1.z, v2.z), v3.z), 1.0f);
-  bhi[leaf] = make_float4(fmaxf(fmaxf(v1.x, v2.x), v3.x), fmaxf(fmaxf(v1.y, v2.y), v3.y),
-                          fmaxf(fmaxf(v1.z, v2.z), v3.z), 1.0f);
+  if (blo) triangle_box(v1, v2, v3, blo[n - 1 + p], bhi[n - 1 + p]);
 }
 
 // Leaf reference: 0x80000000 | (count - 1) << 25 | first  (count <= 32, first < 2^25).
@@ -282,21 +301,11 @@ __host__ __device__ __forceinline__ int pack_leaf(int first, int count) {
   return (int)(0x80000000u | ((uint32_t)(count - 1) << 25) | (uint32_t)first);
 }
 
-constexpr float kCostNode = 1.0f;  // SAH cost of visiting one node (two box tests)
-constexpr float kCostTri = 1.0f;   // SAH cost of one triangle test
-
-__device__ __forceinline__ float half_area(float4 l, float4 h) {
-  float dx = h.x - l.x, dy = h.y - l.y, dz = h.z - l.z;
-  return dx * dy + dy * dz + dz * dx;
-}
-
 // Bottom-up refit: one thread per leaf walks to the root; the second thread to reach an
 // interior node merges the two child boxes and decides whether the subtree becomes one
-// leaf (node records are written afterwards by the wide conversion).  Leaf decision: fixed layout -> the range has at most
-// max_leaf triangles; SAH layout -> additionally the leaf's cost kCostTri * n is not above
-// kCostNode + (A_l cost_l + A_r cost_r) / A.  Box .w carries the subtree cost (lo) and the
-// leaf decision (hi).  Bounded walk: the tree depth is at most kStackMax.
-__global__ void k_refit(int n, const int2* __restrict__ child, const int2* __restrict__ range,
+// leaf (join_boxes; node records are written afterwards by the wide conversion).  Bounded
+// walk: the tree depth is at most kStackMax.
+__global__ void k_refit(int n, const int2* __restrict__ child, const int* __restrict__ count,
                         const int* __restrict__ parent, float4* blo, float4* bhi, int* __restrict__ arrive,
                         int max_leaf, int sah, int* err) {
   int p = blockIdx.x * blockDim.x + threadIdx.x;
@@ -311,18 +320,9 @@ __global__ void k_refit(int n, const int2* __restrict__ child, const int2* __res
     if (atomicAdd(&arrive[node], 1) == 0) return;
     __threadfence();
     int2 c = child[node];
-    float4 l0 = __ldcg(&blo[c.x]), h0 = __ldcg(&bhi[c.x]);
-    float4 l1 = __ldcg(&blo[c.y]), h1 = __ldcg(&bhi[c.y]);
-    float4 lo = make_float4(fminf(l0.x, l1.x), fminf(l0.y, l1.y), fminf(l0.z, l1.z), 0.0f);
-    float4 hi = make_float4(fmaxf(h0.x, h1.x), fmaxf(h0.y, h1.y), fmaxf(h0.z, h1.z), 0.0f);
-    int2 rg = range[node];
-    int size = rg.y - rg.x + 1;
-    float a = half_area(lo, hi);
-    float inner = kCostNode + (a > 0.0f ? (half_area(l0, h0) * l0.w + half_area(l1, h1) * l1.w) / a : l0.w + l1.w);
-    float as_leaf = size <= max_leaf ? kCostTri * (float)size : kInf;
-    bool collapse = sah ? (as_leaf <= inner) : (size <= max_leaf);
-    lo.w = collapse ? as_leaf : inner;
-    hi.w = collapse ? 1.0f : 0.0f;
+    float4 lo, hi;
+    join_boxes(__ldcg(&blo[c.x]), __ldcg(&bhi[c.x]), __ldcg(&blo[c.y]), __ldcg(&bhi[c.y]), count[node], max_leaf, sah,
+               lo, hi);
     blo[node] = lo;
     bhi[node] = hi;
     node = parent[node];
@@ -334,9 +334,9 @@ __global__ void k_refit(int n, const int2* __restrict__ child, const int2* __res
 // replacing its interior child of largest surface area by that child's two children until
 // it has `max_children` children (4 for the 4-wide layout, 2 for the binary one) or only
 // leaves (one-triangle leaves and collapsed subtrees stay leaves).  Top-down, one launch
-// per level; frontier entries are (binary node, record) pairs.
+// per level (k_wide_level).
 //
-// Record, 128 B = 8 x float4 (structure of arrays over the four slots):
+// Record, 128 B = 8 x float4 (structure of arrays over the four slots; node_chunk order):
 //   [0] lo.x[4] [1] lo.y[4] [2] lo.z[4] [3] hi.x[4] [4] hi.y[4] [5] hi.z[4]
 //   [6] ref[4]: interior record index, packed leaf, or kEmptyRef for an unused slot
 //       (whose box is lo = +inf, hi = -inf: every slab test misses it, so the traversal
@@ -353,111 +353,166 @@ __device__ __forceinline__ void write_record(float4* nodes, int n, const float (
   o[node_chunk(n, 7)] = make_float4(__int_as_float(cnt[0]), __int_as_float(cnt[1]), __int_as_float(cnt[2]), __int_as_float(cnt[3]));
 }
 
-// One level of the wide records, in two passes over the frontier (binary node, record):
-// k_wide_select opens each frontier node's children greedily (the largest-area interior
-// child is replaced by its two children until max_children) and counts those that get a
-// record of their own; after an exclusive scan of the counts, k_wide_write numbers them
-// base + scan[t] + j and writes the record.  Records come out level by level, each node's
-// children in consecutive records, the same on every run.
-// Greedy opening of one frontier node (k_wide_select): its children, then the children of
-// the largest-area interior child until max_children are reached; returns how many of
-// them get records of their own.
+// Greedy opening of one binary node: its children, then the children of the largest-area
+// interior child until max_children are reached; returns how many of them get records of
+// their own.
 __device__ __forceinline__ int wide_select_one(int n, const int2* __restrict__ child, const float4* __restrict__ blo,
-                                               const float4* __restrict__ bhi, int node, int max_children,
-                                               int4& sel) {
-  int c[4] = {-1, -1, -1, -1};
-  const int2 ch = child[node];
+                                               const float4* __restrict__ bhi, int node, int max_children, int* c,
+                                               float4* lo, float4* hi) {
+  int2 ch = child[node];
   c[0] = ch.x;
   c[1] = ch.y;
-  int k = 2;
-  while (k < max_children) {
+  c[2] = c[3] = -1;
+  for (int i = 0; i < 2; ++i) {
+    lo[i] = blo[c[i]];
+    hi[i] = bhi[c[i]];
+  }
+#pragma unroll
+  for (int k = 2; k < 4; ++k) {
+    if (k >= max_children) break;
     int best = -1;
     float best_area = -1.0f;
+#pragma unroll
     for (int i = 0; i < k; ++i) {
-      const int ci = c[i];
-      if (ci >= n - 1 || bhi[ci].w != 0.0f) continue;  // triangle or collapsed subtree: a leaf
-      const float a = half_area(blo[ci], bhi[ci]);
+      if (c[i] >= n - 1 || hi[i].w != 0.0f) continue;  // triangle or collapsed subtree: a leaf
+      const float a = half_area(lo[i], hi[i]);
       if (a > best_area) {
         best_area = a;
         best = i;
       }
     }
     if (best < 0) break;
-    const int2 g = child[c[best]];
-    c[best] = g.x;
-    c[k++] = g.y;
+#pragma unroll
+    for (int i = 0; i < k; ++i)
+      if (i == best) {
+        ch = child[c[i]];
+        c[i] = ch.x;
+        lo[i] = blo[ch.x];
+        hi[i] = bhi[ch.x];
+      }
+    c[k] = ch.y;
+    lo[k] = blo[ch.y];
+    hi[k] = bhi[ch.y];
   }
   int m = 0;
-  for (int i = 0; i < k; ++i) m += c[i] < n - 1 && bhi[c[i]].w == 0.0f;
-  sel = make_int4(c[0], c[1], c[2], c[3]);
+#pragma unroll
+  for (int i = 0; i < 4; ++i) m += c[i] >= 0 && c[i] < n - 1 && hi[i].w == 0.0f;
   return m;
 }
 
-__global__ void __launch_bounds__(kScanBlock) k_wide_select(int n, const int2* __restrict__ child,
-                                                            const float4* __restrict__ blo,
-                                                            const float4* __restrict__ bhi,
-                                                            const int2* __restrict__ frontier_in, int n_in,
-                                                            int max_children, int4* __restrict__ sel,
-                                                            int* __restrict__ n_interior, int* __restrict__ bsum) {
-  const int t = blockIdx.x * blockDim.x + threadIdx.x;
-  const int m = t < n_in ? wide_select_one(n, child, blo, bhi, frontier_in[t].x, max_children, sel[t]) : 0;
-  if (t < n_in) n_interior[t] = m;
-  block_total(m, bsum);  // the scan's first step (scan.cuh)
+// The binary tree as the wide conversion reads it: interior 0..n-2, leaf n-1+p; blo / bhi
+// (hi.w: leaf decision); record position of a leaf (perm, NULL: p) and of a collapsed
+// subtree's first triangle, and its triangle count.
+struct BinaryTree {
+  int n;
+  const int2* child;
+  const float4* blo;
+  const float4* bhi;
+  const int* first;
+  const int* count;
+  const uint32_t* perm;
+};
+
+// Level state: [0] nodes of the level, [1] their first record, [3] tickets taken.
+__global__ void k_wide_init(int* __restrict__ state, int root, int* __restrict__ frontier) {
+  state[0] = 1;
+  state[1] = 0;
+  state[3] = 0;
+  frontier[0] = root;
 }
 
-// The first record number of frontier node t's children: its block's exclusive scan of n_interior
-// plus the block's scanned sum (bsum after k_scan_totals); same grid as k_wide_select.
-__global__ void __launch_bounds__(kScanBlock) k_wide_write(int n, const int2* __restrict__ range,
-                                                           const float4* __restrict__ blo,
-                                                           const float4* __restrict__ bhi,
-                                                           const int2* __restrict__ frontier_in, int n_in,
-                                                           const int4* __restrict__ sel,
-                                                           const int* __restrict__ n_interior,
-                                                           const int* __restrict__ bsum, int base,
-                                                           int2* __restrict__ frontier_out,
+// One level of the wide records: each frontier node's children are opened greedily, those
+// that get a record of their own are numbered by a scan over the level (tiles by ticket, the
+// offsets by look-back), and the record is written.  Records come out level by level, each
+// node's children in consecutive records, the same on every run.  Bound by the latency of
+// the child -> box chain and by launches (a tree has 10 to 20 levels): one launch per level,
+// with the level's size read from the state the previous one wrote, where a select / scan /
+// write sequence took three and a read-back of the size.
+__global__ void __launch_bounds__(kScanBlock) k_wide_level(BinaryTree T, int* __restrict__ state,
+                                                           int* __restrict__ state_out, int* __restrict__ slot,
+                                                           int level, unsigned long long* __restrict__ words,
+                                                           const int* __restrict__ frontier,
+                                                           int* __restrict__ frontier_out, int max_children,
                                                            float4* __restrict__ wnodes, int max_nodes, int* err) {
-  const int t = blockIdx.x * blockDim.x + threadIdx.x;
-  int block_sum;
-  int next = bsum[blockIdx.x] + block_exclusive_scan(t < n_in ? n_interior[t] : 0, block_sum);
-  if (t >= n_in) return;
-  const int4 s4 = sel[t];
-  const int c[4] = {s4.x, s4.y, s4.z, s4.w};
-  float v[6][4];
-  int ref[4], cnt[4];
-  for (int i = 0; i < 4; ++i) {
-    const int ci = c[i];
-    if (ci < 0) {
-      for (int a = 0; a < 6; ++a) v[a][i] = a < 3 ? kInf : -kInf;  // a box no ray enters
-      ref[i] = kEmptyRef;
-      cnt[i] = -1;
-      continue;
-    }
-    const float4 l = blo[ci], h = bhi[ci];
-    v[0][i] = l.x; v[1][i] = l.y; v[2][i] = l.z;
-    v[3][i] = h.x; v[4][i] = h.y; v[5][i] = h.z;
-    if (ci >= n - 1) {
-      cnt[i] = 1;
-      ref[i] = pack_leaf(ci - (n - 1), 1);
-    } else if (h.w != 0.0f) {
-      const int2 r = range[ci];
-      cnt[i] = r.y - r.x + 1;
-      ref[i] = pack_leaf(r.x, cnt[i]);
-    } else {
-      const int w = base + next;
-      if (w >= max_nodes) {  // cannot happen: the tree has at most n - 1 records (the host stops)
-        atomicOr(err, kErrQueue);
-        for (int a = 0; a < 6; ++a) v[a][i] = a < 3 ? kInf : -kInf;
-        ref[i] = kEmptyRef;
-        cnt[i] = -1;
-        ++next;
-        continue;
-      }
-      frontier_out[next++] = make_int2(ci, w);
-      ref[i] = w;
-      cnt[i] = 0;
+  __shared__ int s_tile;
+  __shared__ unsigned long long s_before;
+  const int n_in = state[0], base = state[1], n = T.n;
+  const int n_tiles = (n_in + kScanBlock - 1) / kScanBlock;
+  const int next_base = base + n_in;
+  if (blockIdx.x == 0 && threadIdx.x == 0) {
+    state_out[3] = 0;
+    if (n_in == 0) {  // past the last level
+      state_out[0] = slot[0] = 0;
+      state_out[1] = slot[1] = next_base;
+      slot[3] = level;
     }
   }
-  write_record(wnodes, frontier_in[t].y, v, ref, cnt);
+  for (;;) {
+    if (threadIdx.x == 0) s_tile = atomicAdd(&state[3], 1);
+    __syncthreads();
+    const int tile = s_tile;
+    if (tile >= n_tiles) return;
+    const int t = tile * kScanBlock + threadIdx.x;
+    int c[4];
+    float4 lo[4], hi[4];
+    int m = 0;
+    if (t < n_in) m = wide_select_one(n, T.child, T.blo, T.bhi, frontier[t], max_children, c, lo, hi);
+    int total;
+    const int ex = block_exclusive_scan(m, total);
+    if (threadIdx.x < 32) {
+      const unsigned long long before = tiles_before(words, tile, (unsigned long long)total, (unsigned)(level % 4095 + 1));
+      if (threadIdx.x == 0) {
+        s_before = before;
+        if (tile == n_tiles - 1 && before <= kTileValue) {
+          state_out[0] = slot[0] = (int)before + total;
+          state_out[1] = slot[1] = next_base;
+          slot[3] = level;
+        }
+      }
+    }
+    __syncthreads();
+    if (s_before > kTileValue) {  // an earlier tile did not publish its sum
+      if (threadIdx.x == 0) atomicOr(err, kErrTimeout);
+      return;
+    }
+    if (t < n_in) {
+      int next = (int)s_before + ex;
+      float v[6][4];
+      int ref[4], cnt[4];
+#pragma unroll
+      for (int i = 0; i < 4; ++i) {
+        const int ci = c[i];
+        ref[i] = kEmptyRef;
+        cnt[i] = -1;
+        bool used = ci >= 0;
+        if (used) {
+          if (ci >= n - 1) {
+            cnt[i] = 1;
+            ref[i] = pack_leaf(T.perm ? (int)T.perm[ci - (n - 1)] : ci - (n - 1), 1);
+          } else if (hi[i].w != 0.0f) {
+            cnt[i] = T.count[ci];
+            ref[i] = pack_leaf(T.first[ci], cnt[i]);
+          } else if (next_base + next < max_nodes) {
+            frontier_out[next] = ci;
+            ref[i] = next_base + next++;
+            cnt[i] = 0;
+          } else {  // cannot happen: the tree has at most n - 1 records (the host stops)
+            atomicOr(err, kErrQueue);
+            used = false;
+            ++next;
+          }
+        }
+        v[0][i] = used ? lo[i].x : kInf;  // unused: a box no ray enters
+        v[1][i] = used ? lo[i].y : kInf;
+        v[2][i] = used ? lo[i].z : kInf;
+        v[3][i] = used ? hi[i].x : -kInf;
+        v[4][i] = used ? hi[i].y : -kInf;
+        v[5][i] = used ? hi[i].z : -kInf;
+      }
+      write_record(wnodes, base + t, v, ref, cnt);
+    }
+    __syncthreads();  // s_tile and s_before are reused
+  }
 }
 
 // Root record of a scene with 0 or 1 triangle (no binary interior node exists).
@@ -480,59 +535,59 @@ __global__ void k_small_root(int n, const float4* __restrict__ blo, const float4
 
 inline int grid_for(size_t n, int block) { return (int)std::max<size_t>(1, (n + block - 1) / block); }
 
-// Writes the node records of the binary tree in the given width (top-down, one select /
-// scan / write per level).  Returns the number of levels through *levels (kStackMax * 4 + 1 when the walk
-// did not end, which cannot happen for a tree of depth <= kStackMax).
-eos_status write_records(eos_ctx* ctx, int n, const int2* child, const int2* range, const float4* blo,
-                         const float4* bhi, int width, float4* out, int max_nodes, int* levels, int* n_records) {
+// Writes the node records of the binary tree in the given width (top-down, one launch per
+// level; the launches run ahead of the host as the PLOC rounds do, and a launch past the last
+// level writes nothing).  Returns the number of levels through *levels (kStackMax * 4 + 1
+// when the walk did not end, which cannot happen for a tree of depth <= kStackMax).
+eos_status write_records(eos_ctx* ctx, const BinaryTree& T, int root, int width, float4* out, int max_nodes,
+                         int* levels, int* n_records) {
   cudaStream_t st = ctx->stream;
   eos_status es = EOS_OK;
-  const size_t nn = (size_t)n;
-  int2* fa = (int2*)scratch(ctx, "lbvh.wide.fa", 8 * nn, &es);
-  int2* fb = (int2*)scratch(ctx, "lbvh.wide.fb", 8 * nn, &es);
-  int4* sel = (int4*)scratch(ctx, "lbvh.wide.sel", 16 * nn, &es);
-  int* m = (int*)scratch(ctx, "lbvh.wide.m", 4 * (nn + 1), &es);
-  int* bsum = (int*)scratch(ctx, "lbvh.wide.bsum", 4 * ((size_t)scan_blocks(n + 1) + 1), &es);
+  const size_t nn = (size_t)T.n;
+  int* frontier[2] = {(int*)scratch(ctx, "lbvh.wide.fa", 4 * nn, &es), (int*)scratch(ctx, "lbvh.wide.fb", 4 * nn, &es)};
+  const size_t words_bytes = 8 * (size_t)scan_blocks(T.n);
+  unsigned long long* words = (unsigned long long*)scratch(ctx, "lbvh.wide.words", words_bytes, &es);
+  int* state = (int*)scratch(ctx, "lbvh.wide.state", 32, &es);
   if (es != EOS_OK) return es;
-  const int2 root = make_int2(0, 0);  // the binary root becomes record 0
-  EOS_CUDA(cudaMemcpyAsync(fa, &root, sizeof root, cudaMemcpyHostToDevice, st));
-  int n_in = 1, base = 1, lv = 0;
-  while (n_in > 0 && lv <= 4 * kStackMax) {  // bounded: the depth is at most the binary depth
-    const int nb = scan_blocks(n_in);
-    k_wide_select<<<nb, kScanBlock, 0, st>>>(n, child, blo, bhi, fa, n_in, width, sel, m, bsum);
-    k_scan_totals<<<1, 1024, 0, st>>>(bsum, nb);
-    k_wide_write<<<nb, kScanBlock, 0, st>>>(n, range, blo, bhi, fa, n_in, sel, m, bsum, base, fb, out, max_nodes,
-                                            ctx->d_err);
-    EOS_CUDA(cudaGetLastError());
-    ++lv;
-    int n_out = 0;
-    EOS_CUDA(cudaMemcpyAsync(&n_out, bsum + nb, sizeof(int), cudaMemcpyDeviceToHost, st));
-    EOS_CUDA(cudaStreamSynchronize(st));
-    if ((long long)base + n_out > max_nodes) return EOS_ERR_QUEUE_OVERFLOW;  // cannot happen, as above
-    base += n_out;
-    n_in = n_out;
-    std::swap(fa, fb);
+  RoundRing ring(ctx);
+  if ((es = ring.init()) != EOS_OK) return es;
+  EOS_CUDA(cudaMemsetAsync(words, 0, words_bytes, st));
+  k_wide_init<<<1, 1, 0, st>>>(state, root, frontier[0]);
+  long long most = 1;  // nodes of the level at most
+  int s[3] = {1, 0, 0}, lv = 0;
+  for (;;) {
+    if (ring.full()) {
+      if ((es = ring.read(s)) != EOS_OK) return es;
+      ++lv;
+      if ((long long)s[1] + s[0] > max_nodes) return EOS_ERR_QUEUE_OVERFLOW;  // cannot happen, as above
+      if (s[0] == 0 || lv > 4 * kStackMax) break;
+    }
+    const int k = (int)(ring.issued & 1);
+    const int grid = (int)std::min<long long>(scan_blocks(most), ctx->num_sms * 4);
+    k_wide_level<<<grid, kScanBlock, 0, st>>>(T, state + 4 * k, state + 4 * (k ^ 1), ring.next_slot(),
+                                              (int)ring.issued, words, frontier[k], frontier[k ^ 1], width, out,
+                                              max_nodes, ctx->d_err);
+    if ((es = ring.launched()) != EOS_OK) return es;
+    most = std::min<long long>(most * width, T.n);
   }
-  *n_records = std::min(base, max_nodes);
-  *levels = n_in > 0 ? 4 * kStackMax + 1 : lv;
+  *n_records = std::min(s[1] + s[0], max_nodes);
+  *levels = s[0] > 0 ? 4 * kStackMax + 1 : lv;
   return EOS_OK;
 }
 
 // Node records of the scene.  The traversal stack holds at most width - 1 entries per
 // level, so a 4-wide tree deeper than kStackMax / 3 levels (degenerate geometry) is written
 // with two children per record instead; a binary tree's depth is at most 62 <= kStackMax.
-eos_status build_records(eos_ctx* ctx, eos_scene* sc, int n, const int2* child, const int2* range,
-                         const float4* blo, const float4* bhi) {
-  const int max_nodes = n - 1;
+eos_status build_records(eos_ctx* ctx, eos_scene* sc, const BinaryTree& T, int root) {
+  const int max_nodes = T.n - 1;
   EOS_CUDA(scene_alloc(ctx, &sc->d_nodes, 128 * (size_t)max_nodes));
   sc->device_bytes += 128 * (size_t)max_nodes;
   int levels = 0, records = 0;
-  eos_status es = write_records(ctx, n, child, range, blo, bhi, sc->width, (float4*)sc->d_nodes, max_nodes, &levels,
-                                &records);
+  eos_status es = write_records(ctx, T, root, sc->width, (float4*)sc->d_nodes, max_nodes, &levels, &records);
   if (es != EOS_OK) return es;
   if (sc->width == 4 && 3 * levels > kStackMax) {
     sc->width = 2;
-    es = write_records(ctx, n, child, range, blo, bhi, 2, (float4*)sc->d_nodes, max_nodes, &levels, &records);
+    es = write_records(ctx, T, root, 2, (float4*)sc->d_nodes, max_nodes, &levels, &records);
     if (es != EOS_OK) return es;
   }
   if ((sc->width - 1) * levels > kStackMax) return EOS_ERR_STACK_OVERFLOW;
@@ -566,9 +621,8 @@ eos_status build_scene(eos_ctx* ctx, eos_scene* sc, const float* d_verts, const 
   uint32_t* counts = (uint32_t*)scratch(ctx, "lbvh.counts", 4 * (size_t)kRadix * n_tiles, &es);
   uint32_t* totals = (uint32_t*)scratch(ctx, "lbvh.totals", 4 * kRadix, &es);
   int2* child = (int2*)scratch(ctx, "lbvh.child", 8 * n_nodes, &es);
-  int2* range = (int2*)scratch(ctx, "lbvh.range", 8 * n_nodes, &es);
-  int* parent = (int*)scratch(ctx, "lbvh.parent", 4 * (2 * nn), &es);
-  int* arrive = (int*)scratch(ctx, "lbvh.arrive", 4 * n_nodes, &es);
+  int* count = (int*)scratch(ctx, "lbvh.count", 4 * n_nodes, &es);
+  int* first = (int*)scratch(ctx, "lbvh.first", 4 * n_nodes, &es);
   float4* blo = (float4*)scratch(ctx, "lbvh.blo", 16 * (2 * nn), &es);
   float4* bhi = (float4*)scratch(ctx, "lbvh.bhi", 16 * (2 * nn), &es);
   if (es != EOS_OK) return es;
@@ -592,40 +646,50 @@ eos_status build_scene(eos_ctx* ctx, eos_scene* sc, const float* d_verts, const 
       std::swap(vi, vo);
     }
     // 4 passes: the sorted result is back in (keys, vals)
-    k_records<<<grid_for(nn, 256), 256, 0, st>>>(d_verts, d_normals, n_verts, d_tris, d_obj, vals, nullptr, n,
-                                                 (uint32_t)sc->dev.n_obj, (float4*)sc->d_tris, (float4*)sc->d_shade,
-                                                 (int32_t*)sc->d_pos_of_id, blo, bhi, ctx->d_err);
   }
+  auto records = [&](const uint32_t* perm, float4* lo, float4* hi) {
+    k_records<<<grid_for(nn, 256), 256, 0, st>>>(d_verts, d_normals, n_verts, d_tris, d_obj, vals, perm, n,
+                                                 (uint32_t)sc->dev.n_obj, (float4*)sc->d_tris, (float4*)sc->d_shade,
+                                                 (int32_t*)sc->d_pos_of_id, lo, hi, ctx->d_err);
+  };
   if (n >= 2) {
-    bool ploc = sc->builder == EOS_BUILDER_PLOC;
-    if (ploc) {
-      // PLOC over the leaf boxes in Morton order, then the records again in the tree's
-      // depth-first leaf order (every subtree a contiguous range)
-      uint32_t* perm = (uint32_t*)scratch(ctx, "lbvh.perm", 4 * nn, &es);
+    uint32_t* perm = nullptr;
+    int root = 0;
+    if (sc->builder == EOS_BUILDER_PLOC) {
+      // PLOC over the leaf boxes in Morton order; the records in the tree's depth-first leaf
+      // order (every subtree a contiguous range)
+      perm = (uint32_t*)scratch(ctx, "lbvh.perm", 4 * nn, &es);
       if (es != EOS_OK) return es;
+      k_leaf_boxes<<<grid_for(nn, 256), 256, 0, st>>>(d_verts, n_verts, d_tris, vals, n, blo, bhi);
       int depth = 0;
-      if ((es = build_ploc(ctx, n, blo, bhi, child, range, parent, perm, &depth)) != EOS_OK) return es;
-      ploc = depth + 2 <= kStackMax;  // the refit walks at most kStackMax levels
-      if (ploc)
-        k_records<<<grid_for(nn, 256), 256, 0, st>>>(d_verts, d_normals, n_verts, d_tris, d_obj, vals, perm, n,
-                                                     (uint32_t)sc->dev.n_obj, (float4*)sc->d_tris,
-                                                     (float4*)sc->d_shade, (int32_t*)sc->d_pos_of_id, blo, bhi,
-                                                     ctx->d_err);
-      else
+      es = build_ploc(ctx, n, sc->leaf_size, sc->layout == EOS_LAYOUT_SAH, blo, bhi, child, count, first, perm, &depth);
+      if (es != EOS_OK) return es;
+      if (depth + 2 <= kStackMax) {
+        root = n - 2;
+        records(perm, nullptr, nullptr);
+      } else {  // deeper than the refit walks: the LBVH instead
         sc->builder = EOS_BUILDER_LBVH;
+      }
     }
-    EOS_CUDA(cudaMemsetAsync(arrive, 0, 4 * n_nodes, st));
-    if (!ploc) {
+    if (sc->builder == EOS_BUILDER_LBVH) {
+      perm = nullptr;
+      int* parent = (int*)scratch(ctx, "lbvh.parent", 4 * (2 * nn), &es);
+      int* arrive = (int*)scratch(ctx, "lbvh.arrive", 4 * n_nodes, &es);
+      if (es != EOS_OK) return es;
+      records(nullptr, blo, bhi);
+      EOS_CUDA(cudaMemsetAsync(arrive, 0, 4 * n_nodes, st));
       EOS_CUDA(cudaMemsetAsync(parent, 0xff, 4 * (2 * nn), st));
-      k_karras<<<grid_for(n - 1, 256), 256, 0, st>>>(keys, n, child, range, parent);
+      k_karras<<<grid_for(n - 1, 256), 256, 0, st>>>(keys, n, child, first, count, parent);
+      k_refit<<<grid_for(nn, 256), 256, 0, st>>>(n, child, count, parent, blo, bhi, arrive, sc->leaf_size,
+                                                sc->layout == EOS_LAYOUT_SAH, ctx->d_err);
     }
-    k_refit<<<grid_for(nn, 256), 256, 0, st>>>(n, child, range, parent, blo, bhi, arrive, sc->leaf_size,
-                                              sc->layout == EOS_LAYOUT_SAH, ctx->d_err);
     // SAH cost of the tree (subtree cost of the root, in triangle-test units)
-    EOS_CUDA(cudaMemcpyAsync(&sc->sah_cost, &blo[0].w, sizeof(float), cudaMemcpyDeviceToHost, st));
-    eos_status ws = build_records(ctx, sc, n, child, range, blo, bhi);
+    EOS_CUDA(cudaMemcpyAsync(&sc->sah_cost, &blo[root].w, sizeof(float), cudaMemcpyDeviceToHost, st));
+    const BinaryTree T{n, child, blo, bhi, first, count, perm};
+    eos_status ws = build_records(ctx, sc, T, root);
     if (ws != EOS_OK) return ws;
   } else {
+    if (n == 1) records(nullptr, blo, bhi);
     EOS_CUDA(scene_alloc(ctx, &sc->d_nodes, 128));
     sc->device_bytes += 128;
     k_small_root<<<1, 1, 0, st>>>(n, blo, bhi, (float4*)sc->d_nodes);

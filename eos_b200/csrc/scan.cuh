@@ -1,21 +1,18 @@
-// Device-wide exclusive scan in three steps fused into the kernels around it (used by the
-// hierarchy builders for the per-round and per-level compactions):
-//
-//   producer kernel   writes its values and, per block of kScanBlock threads, their sum
-//                     (block_total)
-//   k_scan_totals     one block scans the block sums in place (exclusive) and appends
-//                     the grand total
-//   consumer kernel   recomputes its block's exclusive scan of the same values in shared
-//                     memory and adds the block's scanned sum (block_exclusive_scan)
-//
-// Producer and consumer use the same block size and grid (block b covers values
-// [b * kScanBlock, (b + 1) * kScanBlock)); both call the block helpers from every thread.
+// Device-wide exclusive scans inside one launch, for the per-round and per-level compactions
+// of the hierarchy builders.  A block takes its tile by a ticket, scans its own values in
+// shared memory and gets the sum of all earlier tiles by looking back over their published
+// sums (Merrill & Garland, "Single-pass Parallel Prefix Scan with Decoupled Look-back",
+// 2016).  Tickets are taken in order by running blocks, so the tiles waited for always run.
 #pragma once
 #include <cuda_runtime.h>
+#include <stdint.h>
 
 namespace eos {
 
 constexpr int kScanBlock = 256;
+// Polls of a look-back before it gives up (a fraction of a second); its caller then raises
+// the timeout bit of the error word and leaves the launch without writing.
+constexpr int kMaxPolls = 1 << 18;
 
 template <class T>
 __device__ __forceinline__ T warp_inclusive_scan(T v) {
@@ -48,28 +45,43 @@ __device__ __forceinline__ T block_exclusive_scan(T v, T& total) {
   return ex;
 }
 
-// Sum of one value per thread over the block, written to totals[blockIdx.x].
-template <class T>
-__device__ __forceinline__ void block_total(T v, T* totals) {
-  T total;
-  block_exclusive_scan(v, total);
-  if (threadIdx.x == 0) totals[blockIdx.x] = total;
+// Published sum of a tile: flag in the top two bits (1 = the tile's own sum, 2 = the sum of
+// all tiles up to it), the launch's epoch in the next twelve, the value in the low 50.  A
+// word of an earlier launch carries another epoch, so the array is cleared once per build,
+// not per launch.  Epochs repeat after 4,095 launches: a build of more (PLOC rounds of a
+// degenerate scene) must write every word it reads in each of them, which it does because
+// its tiles only get fewer.
+constexpr unsigned long long kTileValue = (1ull << 50) - 1;
+__device__ __forceinline__ unsigned long long tile_word(unsigned flag, unsigned epoch, unsigned long long value) {
+  return ((unsigned long long)flag << 62) | ((unsigned long long)(epoch & 0xfffu) << 50) | value;
 }
 
-// In-place exclusive scan of totals[0, n_blocks) by one block of 1024 threads;
-// totals[n_blocks] = the grand total.
-template <class T>
-__global__ void __launch_bounds__(1024) k_scan_totals(T* __restrict__ totals, int n_blocks) {
-  T carry = T(0);
-  for (int base = 0; base < n_blocks; base += blockDim.x) {
-    const int i = base + threadIdx.x;
-    const T v = i < n_blocks ? totals[i] : T(0);
-    T chunk;
-    const T ex = block_exclusive_scan(v, chunk);
-    if (i < n_blocks) totals[i] = carry + ex;
-    carry += chunk;
+// Sum of the tiles before `tile`, whose own sum is `sum`; called by all lanes of one warp
+// with the same arguments.  kTileValue + 1 when a tile did not publish in time.
+__device__ __forceinline__ unsigned long long tiles_before(volatile unsigned long long* words, int tile,
+                                                           unsigned long long sum, unsigned epoch) {
+  const int lane = threadIdx.x & 31;
+  if (lane == 0) words[tile] = tile_word(tile == 0 ? 2u : 1u, epoch, sum);
+  unsigned long long before = 0;
+  for (int at = tile - 1; at >= 0; at -= 32) {
+    const int i = at - lane;
+    unsigned long long w = tile_word(2u, epoch, 0);  // before the first tile
+    unsigned missing = 1;
+    for (int poll = 0; missing && poll < kMaxPolls; ++poll) {
+      if (i >= 0) w = words[i];
+      const bool there = (w >> 62) != 0 && ((w >> 50) & 0xfffu) == (epoch & 0xfffu);
+      missing = __ballot_sync(0xffffffffu, !there);
+    }
+    if (missing) return kTileValue + 1;
+    const unsigned whole = __ballot_sync(0xffffffffu, (w >> 62) == 2u);
+    const int last = whole ? __ffs(whole) - 1 : 31;  // nearest tile that holds a full prefix
+    unsigned long long v = lane <= last ? (w & kTileValue) : 0;
+    for (int off = 16; off > 0; off >>= 1) v += __shfl_xor_sync(0xffffffffu, v, off);
+    before += v;
+    if (whole) break;
   }
-  if (threadIdx.x == 0) totals[n_blocks] = carry;
+  if (lane == 0 && tile > 0) words[tile] = tile_word(2u, epoch, before + sum);
+  return before;
 }
 
 inline int scan_blocks(long long n) { return (int)((n + kScanBlock - 1) / kScanBlock); }
