@@ -83,7 +83,8 @@ cudaError_t scene_alloc(eos_ctx* ctx, void** p, size_t bytes) {
     cudaMemPoolTrimTo(ctx->pool, 0);
     e = cudaMallocFromPoolAsync(p, bytes, ctx->pool, ctx->own_stream);
   }
-  if (e == cudaSuccess) e = cudaStreamSynchronize(ctx->own_stream);
+  // used on the context's stream from here on: when that is not the allocating one, wait
+  if (e == cudaSuccess && ctx->stream != ctx->own_stream) e = cudaStreamSynchronize(ctx->own_stream);
   return e;
 }
 

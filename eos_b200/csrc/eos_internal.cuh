@@ -206,8 +206,10 @@ void* scratch(eos_ctx* ctx, const char* name, size_t bytes, eos_status* st);
 // which 3.8 ms build, and up to 0.7 s on a busy host).  A destroyed scene's memory stays in the
 // pool for the next one up to kPoolKeep bytes; the rest goes back to the device at once
 // and all of it with the context, or when an allocation of the context fails.  Allocations
-// and frees are ordered on the context's own stream and waited for, so the arrays may be
-// used on any stream; a free waits for the whole device first, as cudaFree does.
+// and frees are ordered on the context's own stream; the calls that make a scene fill its
+// arrays on the context's stream, after the allocation, and wait for it before they return,
+// so a finished scene may be used on any stream.  A free waits for the whole device first,
+// as cudaFree does.
 constexpr unsigned long long kPoolKeep = 1ull << 30;
 cudaError_t scene_alloc(eos_ctx* ctx, void** p, size_t bytes);
 void scene_free(eos_ctx* ctx, void* const* p, int n);

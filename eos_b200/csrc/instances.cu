@@ -274,7 +274,9 @@ extern "C" eos_status eos_scene_create_instanced(eos_ctx* ctx, const eos_instanc
     cudaGetLastError();
     return fail(EOS_ERR_OOM);
   }
-  if (cudaMemcpy(sc->d_nodes, rec.data(), rec_bytes, cudaMemcpyHostToDevice) != cudaSuccess ||
+  // the copies below are on the default stream, the allocations on the context's own
+  if (cudaStreamSynchronize(ctx->own_stream) != cudaSuccess ||
+      cudaMemcpy(sc->d_nodes, rec.data(), rec_bytes, cudaMemcpyHostToDevice) != cudaSuccess ||
       cudaMemcpy(sc->d_inst, dev.data(), inst_bytes, cudaMemcpyHostToDevice) != cudaSuccess)
     return fail(EOS_ERR_CUDA);
   sc->device_bytes = rec_bytes + inst_bytes + sizeof(eos_material) * n_materials +

@@ -21,7 +21,7 @@ namespace {
 constexpr int kSortThreads = 256;
 constexpr int kSortItems = 8;
 constexpr int kSortTile = kSortThreads * kSortItems;  // keys per block
-constexpr int kRadixBits = 8;
+constexpr int kRadixBits = 10;  // the 30-bit codes in three passes
 constexpr int kRadix = 1 << kRadixBits;
 
 __device__ __forceinline__ uint32_t float_to_ordered(float f) {
@@ -59,134 +59,161 @@ __global__ void k_centroids(const float* __restrict__ verts, uint32_t n_verts,
       hi[k] = fmaxf(hi[k], __shfl_xor_sync(0xffffffffu, hi[k], off));
     }
   }
+  // one atomic per block and bound: a warp's six atomics on the same six words were most of
+  // the kernel's time (1.06M triangles: 43 us)
+  __shared__ uint32_t s[6];
+  if (threadIdx.x < 6) s[threadIdx.x] = threadIdx.x < 3 ? 0xffffffffu : 0u;
+  __syncthreads();
   if ((threadIdx.x & 31) == 0) {
     for (int k = 0; k < 3; ++k) {
       if (lo[k] <= hi[k]) {
-        atomicMin(&bounds[k], float_to_ordered(lo[k]));
-        atomicMax(&bounds[3 + k], float_to_ordered(hi[k]));
+        atomicMin(&s[k], float_to_ordered(lo[k]));
+        atomicMax(&s[3 + k], float_to_ordered(hi[k]));
       }
     }
   }
+  __syncthreads();
+  if (threadIdx.x < 3) atomicMin(&bounds[threadIdx.x], s[threadIdx.x]);
+  else if (threadIdx.x < 6) atomicMax(&bounds[threadIdx.x], s[threadIdx.x]);
 }
 
-__global__ void k_morton(const float4* __restrict__ cent, int n, const uint32_t* __restrict__ bounds,
-                         uint32_t* __restrict__ keys, uint32_t* __restrict__ vals) {
-  int i = blockIdx.x * blockDim.x + threadIdx.x;
-  if (i >= n) return;
-  float4 c = cent[i];
-  float cc[3] = {c.x, c.y, c.z};
-  uint32_t q[3];
-  for (int k = 0; k < 3; ++k) {
-    float lo = ordered_to_float(bounds[k]);
-    float hi = ordered_to_float(bounds[3 + k]);
-    float ext = hi - lo;
-    if (ext > 0.0f) {
-      float f = (1024.0f * (cc[k] - lo)) / ext;
-      uint32_t u = (uint32_t)f;
-      q[k] = u > 1023u ? 1023u : u;
-    } else {
-      q[k] = 0u;
+// Morton codes of one tile and, as k_sort_hist, the tile's counts of the first pass's digit.
+__global__ void __launch_bounds__(kSortThreads) k_morton(const float4* __restrict__ cent, int n,
+                                                         const uint32_t* __restrict__ bounds,
+                                                         uint32_t* __restrict__ keys, uint32_t* __restrict__ vals,
+                                                         uint32_t* __restrict__ counts, int n_tiles) {
+  __shared__ uint32_t h[kRadix];
+  for (int i = threadIdx.x; i < kRadix; i += kSortThreads) h[i] = 0;
+  __syncthreads();
+#pragma unroll
+  for (int r = 0; r < kSortItems; ++r) {
+    const int i = blockIdx.x * kSortTile + r * kSortThreads + threadIdx.x;
+    if (i >= n) break;
+    float4 c = cent[i];
+    float cc[3] = {c.x, c.y, c.z};
+    uint32_t q[3];
+    for (int k = 0; k < 3; ++k) {
+      float lo = ordered_to_float(bounds[k]);
+      float hi = ordered_to_float(bounds[3 + k]);
+      float ext = hi - lo;
+      if (ext > 0.0f) {
+        float f = (1024.0f * (cc[k] - lo)) / ext;
+        uint32_t u = (uint32_t)f;
+        q[k] = u > 1023u ? 1023u : u;
+      } else {
+        q[k] = 0u;
+      }
     }
+    const uint32_t key = morton3(q[0], q[1], q[2]);
+    keys[i] = key;
+    vals[i] = (uint32_t)i;
+    atomicAdd(&h[key & (kRadix - 1)], 1u);
   }
-  keys[i] = morton3(q[0], q[1], q[2]);
-  vals[i] = (uint32_t)i;
+  __syncthreads();
+  for (int d = threadIdx.x; d < kRadix; d += kSortThreads) counts[(size_t)d * n_tiles + blockIdx.x] = h[d];
 }
 
 // ------------------------------------------------------------------ stable LSD radix sort
-// Per pass: per-tile digit histogram -> per-digit exclusive scan over tiles -> scan of the
-// digit totals -> stable scatter.  Inside a tile, warp w owns keys [w*256, w*256+256) in
-// 8 rounds of 32; peers with the same digit are found with __match_any_sync and ranked
-// with popc, so the scatter keeps the input order (stability gives the (code, id) order).
-__global__ void k_sort_hist(const uint32_t* __restrict__ keys, int n, int shift, uint32_t* __restrict__ counts,
-                            int n_tiles) {
+// Three passes of ten bits: per-tile digit counts (of the first pass: k_morton) -> per-digit
+// exclusive scan over the tiles -> stable scatter, which scans the digit totals itself.
+// Inside a tile, warp w owns keys [w*256, w*256+256) in 8 rounds of 32; peers with the same
+// digit are found with __match_any_sync and ranked with popc, so the scatter keeps the input
+// order (stability gives the (code, id) order).  Small sorts are bound by launches: nine
+// with the codes, where four passes of eight bits with a scan of their own took seventeen.
+__global__ void __launch_bounds__(kSortThreads) k_sort_hist(const uint32_t* __restrict__ keys, int n, int shift,
+                                                            uint32_t* __restrict__ counts, int n_tiles) {
   __shared__ uint32_t h[kRadix];
-  for (int i = threadIdx.x; i < kRadix; i += blockDim.x) h[i] = 0;
-  __syncthreads();
-  int base = blockIdx.x * kSortTile;
-  for (int j = threadIdx.x; j < kSortTile; j += blockDim.x) {
-    int idx = base + j;
-    if (idx < n) atomicAdd(&h[(keys[idx] >> shift) & (kRadix - 1)], 1u);
+  uint32_t key[kSortItems];
+#pragma unroll
+  for (int r = 0; r < kSortItems; ++r) {
+    const int i = blockIdx.x * kSortTile + r * kSortThreads + threadIdx.x;
+    key[r] = i < n ? keys[i] : 0u;
   }
+  for (int i = threadIdx.x; i < kRadix; i += kSortThreads) h[i] = 0;
   __syncthreads();
-  for (int d = threadIdx.x; d < kRadix; d += blockDim.x) counts[(size_t)d * n_tiles + blockIdx.x] = h[d];
+#pragma unroll
+  for (int r = 0; r < kSortItems; ++r)
+    if (blockIdx.x * kSortTile + r * kSortThreads + threadIdx.x < n) atomicAdd(&h[(key[r] >> shift) & (kRadix - 1)], 1u);
+  __syncthreads();
+  for (int d = threadIdx.x; d < kRadix; d += kSortThreads) counts[(size_t)d * n_tiles + blockIdx.x] = h[d];
 }
 
-// One block per digit: exclusive scan of that digit's per-tile counts (in place).
-__global__ void k_sort_scan_rows(uint32_t* __restrict__ counts, int n_tiles, uint32_t* __restrict__ totals) {
-  __shared__ uint32_t s[kSortThreads];
-  __shared__ uint32_t carry;
-  uint32_t* row = counts + (size_t)blockIdx.x * n_tiles;
-  if (threadIdx.x == 0) carry = 0;
-  __syncthreads();
-  for (int b = 0; b < n_tiles; b += blockDim.x) {
-    int i = b + threadIdx.x;
-    uint32_t v = i < n_tiles ? row[i] : 0u;
-    s[threadIdx.x] = v;
-    __syncthreads();
-    for (int off = 1; off < blockDim.x; off <<= 1) {
-      uint32_t t = threadIdx.x >= off ? s[threadIdx.x - off] : 0u;
-      __syncthreads();
-      s[threadIdx.x] += t;
-      __syncthreads();
+// One warp per digit: exclusive scan of that digit's per-tile counts (in place), and its total.
+__global__ void __launch_bounds__(kSortThreads) k_sort_scan_rows(uint32_t* __restrict__ counts, int n_tiles,
+                                                                 uint32_t* __restrict__ totals) {
+  const int lane = threadIdx.x & 31, digit = (blockIdx.x * kSortThreads + threadIdx.x) >> 5;
+  uint32_t* row = counts + (size_t)digit * n_tiles;
+  uint32_t carry = 0;
+  for (int b = 0; b < n_tiles; b += 128) {  // four loads in flight
+    uint32_t v[4];
+#pragma unroll
+    for (int k = 0; k < 4; ++k) {
+      const int i = b + 32 * k + lane;
+      v[k] = i < n_tiles ? row[i] : 0u;
     }
-    uint32_t incl = s[threadIdx.x];
-    if (i < n_tiles) row[i] = carry + incl - v;
-    __syncthreads();
-    if (threadIdx.x == blockDim.x - 1) carry += incl;
-    __syncthreads();
+#pragma unroll
+    for (int k = 0; k < 4; ++k) {
+      const int i = b + 32 * k + lane;
+      const uint32_t incl = warp_inclusive_scan(v[k]);
+      if (i < n_tiles) row[i] = carry + incl - v[k];
+      carry += __shfl_sync(0xffffffffu, incl, 31);
+    }
   }
-  if (threadIdx.x == 0) totals[blockIdx.x] = carry;
-}
-
-__global__ void k_sort_scan_digits(uint32_t* __restrict__ totals) {
-  __shared__ uint32_t s[kRadix];
-  uint32_t v = totals[threadIdx.x];
-  s[threadIdx.x] = v;
-  __syncthreads();
-  for (int off = 1; off < kRadix; off <<= 1) {
-    uint32_t t = threadIdx.x >= off ? s[threadIdx.x - off] : 0u;
-    __syncthreads();
-    s[threadIdx.x] += t;
-    __syncthreads();
-  }
-  totals[threadIdx.x] = s[threadIdx.x] - v;
+  if (lane == 0) totals[digit] = carry;
 }
 
 __global__ void __launch_bounds__(kSortThreads) k_sort_scatter(
     const uint32_t* __restrict__ kin, const uint32_t* __restrict__ vin, uint32_t* __restrict__ kout,
     uint32_t* __restrict__ vout, int n, int shift, const uint32_t* __restrict__ counts, int n_tiles,
-    const uint32_t* __restrict__ digit_base) {
-  constexpr int kWarps = kSortThreads / 32;
+    const uint32_t* __restrict__ totals) {
+  constexpr int kWarps = kSortThreads / 32, kPer = kRadix / kSortThreads;
   __shared__ uint32_t wh[kWarps][kRadix];
   __shared__ uint32_t tile_base[kRadix];
   const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
-  for (int i = threadIdx.x; i < kWarps * kRadix; i += blockDim.x) (&wh[0][0])[i] = 0;
-  for (int d = threadIdx.x; d < kRadix; d += blockDim.x)
-    tile_base[d] = digit_base[d] + counts[(size_t)d * n_tiles + blockIdx.x];
-  __syncthreads();
   const uint32_t lt_mask = (1u << lane) - 1u;
   uint32_t key[kSortItems], val[kSortItems], local[kSortItems];
-  int base = blockIdx.x * kSortTile + w * 32 * kSortItems;
+  const int base = blockIdx.x * kSortTile + w * 32 * kSortItems;
 #pragma unroll
   for (int r = 0; r < kSortItems; ++r) {
-    int idx = base + r * 32 + lane;
-    bool valid = idx < n;
-    key[r] = valid ? kin[idx] : 0u;
-    val[r] = valid ? vin[idx] : 0u;
-    uint32_t digit = valid ? ((key[r] >> shift) & (kRadix - 1)) : (uint32_t)kRadix + lane;
-    uint32_t peers = __match_any_sync(0xffffffffu, digit);
-    uint32_t rank = __popc(peers & lt_mask);
-    uint32_t pre = valid ? wh[w][digit] : 0u;
+    const int idx = base + r * 32 + lane;
+    key[r] = idx < n ? kin[idx] : 0u;
+    val[r] = idx < n ? vin[idx] : 0u;
+  }
+  // each thread's kPer consecutive digits: scan of the totals + this tile's place in each
+  uint32_t sum = 0, mine[kPer];
+#pragma unroll
+  for (int k = 0; k < kPer; ++k) {
+    mine[k] = totals[kPer * threadIdx.x + k];
+    sum += mine[k];
+  }
+  for (int i = threadIdx.x; i < kWarps * kRadix; i += kSortThreads) (&wh[0][0])[i] = 0;
+  uint32_t all;
+  uint32_t before = block_exclusive_scan(sum, all);
+#pragma unroll
+  for (int k = 0; k < kPer; ++k) {
+    const int d = kPer * threadIdx.x + k;
+    tile_base[d] = before + counts[(size_t)d * n_tiles + blockIdx.x];
+    before += mine[k];
+  }
+  __syncthreads();
+#pragma unroll
+  for (int r = 0; r < kSortItems; ++r) {
+    const bool valid = base + r * 32 + lane < n;
+    const uint32_t digit = valid ? ((key[r] >> shift) & (kRadix - 1)) : (uint32_t)kRadix + lane;
+    const uint32_t peers = __match_any_sync(0xffffffffu, digit);
+    const uint32_t rank = __popc(peers & lt_mask);
+    const uint32_t pre = valid ? wh[w][digit] : 0u;
     __syncwarp();
     if (valid && rank == 0) wh[w][digit] = pre + __popc(peers);
     __syncwarp();
     local[r] = pre + rank;
   }
   __syncthreads();
-  for (int d = threadIdx.x; d < kRadix; d += blockDim.x) {
-    uint32_t s = 0;
+  for (int d = threadIdx.x; d < kRadix; d += kSortThreads) {
+    uint32_t s = tile_base[d];
+#pragma unroll
     for (int ww = 0; ww < kWarps; ++ww) {
-      uint32_t t = wh[ww][d];
+      const uint32_t t = wh[ww][d];
       wh[ww][d] = s;
       s += t;
     }
@@ -194,10 +221,8 @@ __global__ void __launch_bounds__(kSortThreads) k_sort_scatter(
   __syncthreads();
 #pragma unroll
   for (int r = 0; r < kSortItems; ++r) {
-    int idx = base + r * 32 + lane;
-    if (idx < n) {
-      uint32_t digit = (key[r] >> shift) & (kRadix - 1);
-      uint32_t pos = tile_base[digit] + wh[w][digit] + local[r];
+    if (base + r * 32 + lane < n) {
+      const uint32_t pos = wh[w][(key[r] >> shift) & (kRadix - 1)] + local[r];
       kout[pos] = key[r];
       vout[pos] = val[r];
     }
@@ -549,7 +574,7 @@ eos_status write_records(eos_ctx* ctx, const BinaryTree& T, int root, int width,
   unsigned long long* words = (unsigned long long*)scratch(ctx, "lbvh.wide.words", words_bytes, &es);
   int* state = (int*)scratch(ctx, "lbvh.wide.state", 32, &es);
   if (es != EOS_OK) return es;
-  RoundRing ring(ctx);
+  RoundRing ring(ctx, 2);  // as many launches run past the last level
   if ((es = ring.init()) != EOS_OK) return es;
   EOS_CUDA(cudaMemsetAsync(words, 0, words_bytes, st));
   k_wide_init<<<1, 1, 0, st>>>(state, root, frontier[0]);
@@ -635,17 +660,15 @@ eos_status build_scene(eos_ctx* ctx, eos_scene* sc, const float* d_verts, const 
     EOS_CUDA(cudaMemcpyAsync(bounds, init, sizeof init, cudaMemcpyHostToDevice, st));
     int g = std::min(grid_for(nn, 256), ctx->num_sms * 8);
     k_centroids<<<g, 256, 0, st>>>(d_verts, n_verts, d_tris, n, cent, bounds, ctx->d_err);
-    k_morton<<<grid_for(nn, 256), 256, 0, st>>>(cent, n, bounds, keys, vals);
-    uint32_t *ki = keys, *vi = vals, *ko = k2, *vo = v2;
+    uint32_t *ki = k2, *vi = v2, *ko = keys, *vo = vals;  // three passes end in (keys, vals)
+    k_morton<<<n_tiles, kSortThreads, 0, st>>>(cent, n, bounds, ki, vi, counts, n_tiles);
     for (int shift = 0; shift < 30; shift += kRadixBits) {
-      k_sort_hist<<<n_tiles, kSortThreads, 0, st>>>(ki, n, shift, counts, n_tiles);
-      k_sort_scan_rows<<<kRadix, kSortThreads, 0, st>>>(counts, n_tiles, totals);
-      k_sort_scan_digits<<<1, kRadix, 0, st>>>(totals);
+      if (shift > 0) k_sort_hist<<<n_tiles, kSortThreads, 0, st>>>(ki, n, shift, counts, n_tiles);
+      k_sort_scan_rows<<<kRadix * 32 / kSortThreads, kSortThreads, 0, st>>>(counts, n_tiles, totals);
       k_sort_scatter<<<n_tiles, kSortThreads, 0, st>>>(ki, vi, ko, vo, n, shift, counts, n_tiles, totals);
       std::swap(ki, ko);
       std::swap(vi, vo);
     }
-    // 4 passes: the sorted result is back in (keys, vals)
   }
   auto records = [&](const uint32_t* perm, float4* lo, float4* hi) {
     k_records<<<grid_for(nn, 256), 256, 0, st>>>(d_verts, d_normals, n_verts, d_tris, d_obj, vals, perm, n,

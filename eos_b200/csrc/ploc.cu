@@ -64,7 +64,8 @@ struct PlocTree {
   float4* bhi;
 };
 
-__device__ __forceinline__ int node_count(const PlocTree& T, int v) { return v >= T.n - 1 ? 1 : T.count[v]; }
+// Triangles below a cluster: in its hi.w; the first round's clusters (cid NULL) are the leaves.
+__device__ __forceinline__ int cluster_count(const int* cid, float4 hi) { return cid ? __float_as_int(hi.w) : 1; }
 
 // Writes node k = (a, b) and returns its box (lo.w its cost).
 __device__ __forceinline__ void make_node(const PlocTree& T, int k, int a, int b, int ca, int cb, float4 al, float4 ah,
@@ -98,7 +99,7 @@ __global__ void __launch_bounds__(kRoundThreads) k_ploc_round(
     int* __restrict__ err) {
   constexpr int kBoxes = 2 * kRoundThreads + 2 * kRadius;
   __shared__ float4 slo[2][kBoxes / 2], shi[2][kBoxes / 2];
-  __shared__ int snn[2 * kRoundThreads];
+  __shared__ int sid[kBoxes], snn[2 * kRoundThreads];
   __shared__ int s_tile;
   __shared__ unsigned long long s_before;
   const int t = threadIdx.x;
@@ -114,6 +115,7 @@ __global__ void __launch_bounds__(kRoundThreads) k_ploc_round(
     const bool in = g >= 0 && g < nc;
     slo[e & 1][e >> 1] = in ? lo[g] : make_float4(-kInf, -kInf, -kInf, 0.0f);
     shi[e & 1][e >> 1] = in ? hi[g] : make_float4(kInf, kInf, kInf, 0.0f);
+    sid[e] = !in ? 0 : cid ? cid[g] : T.n - 1 + g;
   }
   __syncthreads();
   const int i0 = base - kRadius + 2 * t;  // this thread's clusters: i0 and i0 + 1
@@ -181,19 +183,20 @@ __global__ void __launch_bounds__(kRoundThreads) k_ploc_round(
     if (!(c ? keep1 : keep0)) continue;
     const int e = i - base + 2 * kRadius;
     const float4 al = slo[e & 1][e >> 1], ah = shi[e & 1][e >> 1];
-    int id = cid ? cid[i] : T.n - 1 + i;
+    int id = sid[e], cnt = cluster_count(cid, ah);
     float4 ol = al, oh = ah;
     if (p >= 0) {
       const int f = p - base + 2 * kRadius;
-      const int b = cid ? cid[p] : T.n - 1 + p;
+      const float4 bl = slo[f & 1][f >> 1], bh = shi[f & 1][f >> 1];
+      const int cb = cluster_count(cid, bh);
       if (k < T.n - 1)  // always: n leaves make n - 1 nodes
-        make_node(T, k, id, b, node_count(T, id), node_count(T, b), al, ah, slo[f & 1][f >> 1], shi[f & 1][f >> 1], ol,
-                  oh);
+        make_node(T, k, id, sid[f], cnt, cb, al, ah, bl, bh, ol, oh);
       id = k++;
+      cnt += cb;
     }
     cid_out[pos] = id;
     lo_out[pos] = ol;
-    hi_out[pos] = oh;
+    hi_out[pos] = make_float4(oh.x, oh.y, oh.z, __int_as_float(cnt));
     ++pos;
   }
 }
@@ -206,9 +209,13 @@ __global__ void __launch_bounds__(kRoundThreads) k_ploc_round(
 __global__ void __launch_bounds__(kTail) k_ploc_tail(PlocTree T, int* __restrict__ state, const int* __restrict__ cid_in,
                                                      const float4* __restrict__ lo_in, const float4* __restrict__ hi_in,
                                                      int* __restrict__ err) {
-  __shared__ float4 slo[kTail], shi[kTail];
+  // boxes with kRadius places on each side, which hold an infinite box (as those past the
+  // last cluster): its merged area is never below the best, so the search checks no range
+  __shared__ float4 slo_[kTail + 2 * kRadius], shi_[kTail + 2 * kRadius];
   __shared__ int scid[kTail], scount[kTail], snn[kTail];
   __shared__ int wsum[kTail / 32];
+  float4 *const slo = slo_ + kRadius, *const shi = shi_ + kRadius;
+  const float4 out_lo = make_float4(-kInf, -kInf, -kInf, 0.0f), out_hi = make_float4(kInf, kInf, kInf, 0.0f);
   const int i = threadIdx.x, lane = i & 31, warp = i >> 5;
   int nc = state[0], node_base = state[1];
   int force = state[2] == 0 && nc > 1;  // the last round merged nothing: the forced round is next
@@ -220,7 +227,14 @@ __global__ void __launch_bounds__(kTail) k_ploc_tail(PlocTree T, int* __restrict
     slo[i] = lo_in[i];
     shi[i] = hi_in[i];
     scid[i] = cid_in ? cid_in[i] : T.n - 1 + i;
-    scount[i] = node_count(T, scid[i]);
+    scount[i] = cluster_count(cid_in, shi[i]);
+  } else {
+    slo[i] = out_lo;
+    shi[i] = out_hi;
+  }
+  if (i < kRadius) {
+    slo_[i] = slo[kTail + i] = out_lo;
+    shi_[i] = shi[kTail + i] = out_hi;
   }
   __syncthreads();
   int iters = 0;
@@ -233,22 +247,30 @@ __global__ void __launch_bounds__(kTail) k_ploc_tail(PlocTree T, int* __restrict
       // 2^lg threads per cluster, each 32 / 2^lg of the neighbours; the least (area, index)
       const int lg = nc > 512 ? 0 : nc > 256 ? 1 : nc > 128 ? 2 : nc > 64 ? 3 : nc > 32 ? 4 : 5;
       const int c = i >> lg, g = i & ((1 << lg) - 1), per = (2 * kRadius) >> lg;
-      unsigned long long best = ~0ull;
+      float best = kInf;
+      int bj = kTail;
       if (c < nc) {
         const float4 al = slo[c], ah = shi[c];
-        for (int w = g * per; w < (g + 1) * per; ++w) {
-          const int j = c + (w < kRadius ? w - kRadius : w - kRadius + 1);
-          if (j < 0 || j >= nc) continue;
+        const int j0 = c - kRadius + g * per;
+#pragma unroll 4
+        for (int w = 0; w < per; ++w) {
+          const int j = j0 + w + (g * per + w >= kRadius);  // all places but c
           const float a = merged_area(al, ah, slo[j], shi[j]);
-          const unsigned long long key = ((unsigned long long)__float_as_uint(a) << 32) | (unsigned)j;
-          if (a < kInf && key < best) best = key;
+          if (a < best) {
+            best = a;
+            bj = j;
+          }
         }
       }
       for (int off = 1; off < (1 << lg); off <<= 1) {
-        const unsigned long long o = __shfl_xor_sync(0xffffffffu, best, off);
-        best = o < best ? o : best;
+        const float o = __shfl_xor_sync(0xffffffffu, best, off);
+        const int oj = __shfl_xor_sync(0xffffffffu, bj, off);
+        if (o < best || (o == best && oj < bj)) {
+          best = o;
+          bj = oj;
+        }
       }
-      if (c < nc && g == 0) snn[c] = best != ~0ull ? (int)(unsigned)best : (c == 0 ? 1 : c - 1);
+      if (c < nc && g == 0) snn[c] = best < kInf ? bj : (c == 0 ? 1 : c - 1);
     }
     __syncthreads();
     int partner = -1;
@@ -294,9 +316,13 @@ __global__ void __launch_bounds__(kTail) k_ploc_tail(PlocTree T, int* __restrict
       slo[pos] = ol;
       shi[pos] = oh;
     }
-    const int made = (int)(total >> 16);
+    const int made = (int)(total >> 16), kept = (int)(total & 0xffff);
+    if (i >= kept && i < nc) {
+      slo[i] = out_lo;
+      shi[i] = out_hi;
+    }
     node_base += made;
-    nc = (int)(total & 0xffff);
+    nc = kept;
     force = made == 0 && !force;
     __syncthreads();
   }

@@ -10,8 +10,9 @@ namespace eos {
 struct RoundRing {
   static constexpr int kAhead = 4;
   eos_ctx* ctx;
+  int ahead;
   long long issued = 0, done = 0;
-  explicit RoundRing(eos_ctx* c) : ctx(c) {}
+  explicit RoundRing(eos_ctx* c, int n = kAhead) : ctx(c), ahead(n) {}
   eos_status init() {
     static_assert(kAhead <= (int)(sizeof(ctx->ring_ev) / sizeof(ctx->ring_ev[0])), "one event per slot");
     if (!ctx->ring_host) {
@@ -29,7 +30,7 @@ struct RoundRing {
     return EOS_OK;
   }
   int* next_slot() const { return ctx->ring_dev + 4 * (int)(issued % kAhead); }
-  bool full() const { return issued - done == kAhead; }
+  bool full() const { return issued - done == ahead; }
   bool empty() const { return issued == done; }
   // After a launch that writes next_slot().
   eos_status launched() {
