@@ -34,7 +34,11 @@ eos_ctx::~eos_ctx() {
   for (cudaEvent_t e : ev_join)
     if (e) cudaEventDestroy(e);
   for (auto& kv : scratch)
-    if (kv.second.ptr) cudaFree(kv.second.ptr);
+    if (kv.second.ptr) {
+      if (kv.second.pooled) cudaFreeAsync(kv.second.ptr, own_stream);
+      else cudaFree(kv.second.ptr);
+    }
+  if (own_stream) cudaStreamSynchronize(own_stream);
   if (pinned) cudaFreeHost(pinned);
   if (ring_host) cudaFreeHost(ring_host);
   for (cudaEvent_t e : ring_ev)
@@ -53,14 +57,19 @@ void* scratch(eos_ctx* ctx, const char* name, size_t bytes, eos_status* st) {
   DevBuffer& b = ctx->scratch[name];
   if (b.bytes >= bytes && b.ptr) return b.ptr;
   if (b.ptr) {
-    cudaStreamSynchronize(ctx->stream);
-    cudaFree(b.ptr);
+    if (b.pooled) {
+      pool_free(ctx, &b.ptr, 1);
+    } else {
+      cudaStreamSynchronize(ctx->stream);
+      cudaFree(b.ptr);
+    }
     b.ptr = nullptr;
     b.bytes = 0;
   }
-  size_t want = std::max<size_t>(bytes, 256);
-  cudaError_t e = cudaMalloc(&b.ptr, want);
-  if (e != cudaSuccess) {  // again with what the pool keeps given back
+  const size_t want = std::max<size_t>(bytes, 256);
+  b.pooled = want < kPoolScratch;
+  cudaError_t e = b.pooled ? pool_alloc(ctx, &b.ptr, want) : cudaMalloc(&b.ptr, want);
+  if (e != cudaSuccess && !b.pooled) {  // again with what the pool keeps given back
     cudaGetLastError();
     cudaMemPoolTrimTo(ctx->pool, 0);
     e = cudaMalloc(&b.ptr, want);
@@ -75,7 +84,7 @@ void* scratch(eos_ctx* ctx, const char* name, size_t bytes, eos_status* st) {
   return b.ptr;
 }
 
-cudaError_t scene_alloc(eos_ctx* ctx, void** p, size_t bytes) {
+cudaError_t pool_alloc(eos_ctx* ctx, void** p, size_t bytes) {
   *p = nullptr;
   cudaError_t e = cudaMallocFromPoolAsync(p, bytes, ctx->pool, ctx->own_stream);
   if (e == cudaErrorMemoryAllocation) {  // again with what the pool keeps given back
@@ -88,7 +97,7 @@ cudaError_t scene_alloc(eos_ctx* ctx, void** p, size_t bytes) {
   return e;
 }
 
-void scene_free(eos_ctx* ctx, void* const* p, int n) {
+void pool_free(eos_ctx* ctx, void* const* p, int n) {
   cudaDeviceSynchronize();
   for (int k = 0; k < n; ++k)
     if (p[k]) cudaFreeAsync(p[k], ctx->own_stream);
@@ -457,8 +466,8 @@ eos_status eos_scene_create(eos_ctx* ctx, const float* verts, const float* norma
   const uint32_t* dt = (const uint32_t*)stage_in(ctx, "in.tris", tris, 12ull * n_tris, &st);
   const uint32_t* dob = (const uint32_t*)stage_in(ctx, "in.obj", tri_obj, 4ull * n_tris, &st);
   if (st != EOS_OK) return fail(st);
-  if (scene_alloc(ctx, &sc->d_mats, sizeof(eos_material) * n_materials) != cudaSuccess) return fail(EOS_ERR_OOM);
-  if (scene_alloc(ctx, &sc->d_lights, sizeof(eos_light) * std::max<uint32_t>(1, n_lights)) != cudaSuccess)
+  if (pool_alloc(ctx, &sc->d_mats, sizeof(eos_material) * n_materials) != cudaSuccess) return fail(EOS_ERR_OOM);
+  if (pool_alloc(ctx, &sc->d_lights, sizeof(eos_light) * std::max<uint32_t>(1, n_lights)) != cudaSuccess)
     return fail(EOS_ERR_OOM);
   sc->device_bytes += sizeof(eos_material) * n_materials + sizeof(eos_light) * std::max<uint32_t>(1, n_lights);
   sc->dev.n_obj = (int)n_materials;
@@ -492,7 +501,7 @@ eos_status eos_scene_destroy(eos_scene* sc) {
   }
   void* bufs[] = {sc->d_nodes, sc->d_tris, sc->d_shade, sc->d_pos_of_id, sc->d_mats, sc->d_lights, sc->d_codes,
                   sc->d_order, sc->d_inst};
-  if (sc->ctx) scene_free(sc->ctx, bufs, (int)(sizeof bufs / sizeof bufs[0]));
+  if (sc->ctx) pool_free(sc->ctx, bufs, (int)(sizeof bufs / sizeof bufs[0]));
   delete sc;
   return EOS_OK;
 }

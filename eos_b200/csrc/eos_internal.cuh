@@ -98,6 +98,7 @@ struct DevScene {
 struct DevBuffer {
   void* ptr = nullptr;
   size_t bytes = 0;
+  bool pooled = false;  // from the context's pool (pool_alloc), else cudaMalloc
 };
 
 }  // namespace eos
@@ -111,7 +112,7 @@ struct eos_ctx {
   int* d_err = nullptr;                   // device error word
   unsigned long long* d_counts = nullptr; // ray / traversal counters [kCounters]
   std::map<std::string, eos::DevBuffer> scratch;
-  cudaMemPool_t pool = nullptr;  // scene arrays (scene_alloc)
+  cudaMemPool_t pool = nullptr;  // scene arrays and small scratch (pool_alloc)
   void* pinned = nullptr;
   size_t pinned_bytes = 0;
   // read-back ring of the builders' launches that run ahead of the host (made on first use,
@@ -201,18 +202,22 @@ namespace eos {
 
 // Scratch buffers owned by the context, grown on demand and reused across calls.
 void* scratch(eos_ctx* ctx, const char* name, size_t bytes, eos_status* st);
-// Scene arrays come from a memory pool of the context, because cudaMalloc and cudaFree of
-// the 250 MB of a 1M-triangle scene cost more than its build (create + destroy 26 ms of
-// which 3.8 ms build, and up to 0.7 s on a busy host).  A destroyed scene's memory stays in the
-// pool for the next one up to kPoolKeep bytes; the rest goes back to the device at once
-// and all of it with the context, or when an allocation of the context fails.  Allocations
-// and frees are ordered on the context's own stream; the calls that make a scene fill its
-// arrays on the context's stream, after the allocation, and wait for it before they return,
-// so a finished scene may be used on any stream.  A free waits for the whole device first,
-// as cudaFree does.
+// Scene arrays and scratch buffers below kPoolScratch come from a memory pool of the context,
+// because cudaMalloc and cudaFree of the 250 MB of a 1M-triangle scene cost more than its
+// build (create + destroy 26 ms of which 3.8 ms build, and up to 0.7 s on a busy host).  What
+// is freed stays in the pool for the next scene up to kPoolKeep bytes; the rest goes back to
+// the device at once and all of it with the context, or when an allocation of the context
+// fails.  Allocations and frees are ordered on the context's own stream; the calls that
+// allocate fill the arrays on the context's stream, after the allocation, and wait for it
+// before they return, so a finished scene may be used on any stream.  A free waits for the
+// whole device first, as cudaFree does.  Scratch from kPoolScratch bytes on stays with
+// cudaMalloc: a new context's first call that needs 3.6 GB of queues (four 1080p views) takes
+// 12 ms with it and 28 ms from the pool, while one that needs buffers below the line takes
+// 2.1 ms from the pool and 3.6 without (a 512 x 512 view with four samples).
 constexpr unsigned long long kPoolKeep = 1ull << 30;
-cudaError_t scene_alloc(eos_ctx* ctx, void** p, size_t bytes);
-void scene_free(eos_ctx* ctx, void* const* p, int n);
+constexpr size_t kPoolScratch = 64u << 20;
+cudaError_t pool_alloc(eos_ctx* ctx, void** p, size_t bytes);
+void pool_free(eos_ctx* ctx, void* const* p, int n);
 // Pointer classification (cudaPointerGetAttributes): true for device/managed memory.
 bool is_device_ptr(const void* p);
 

@@ -268,9 +268,9 @@ extern "C" eos_status eos_scene_create_instanced(eos_ctx* ctx, const eos_instanc
     return s;
   };
   const size_t rec_bytes = rec.size() * sizeof(float), inst_bytes = sizeof(DevInstance) * n_instances;
-  if (scene_alloc(ctx, &sc->d_nodes, rec_bytes) != cudaSuccess || scene_alloc(ctx, &sc->d_inst, inst_bytes) != cudaSuccess ||
-      scene_alloc(ctx, &sc->d_mats, sizeof(eos_material) * n_materials) != cudaSuccess ||
-      scene_alloc(ctx, &sc->d_lights, sizeof(eos_light) * std::max<uint32_t>(1, n_lights)) != cudaSuccess) {
+  if (pool_alloc(ctx, &sc->d_nodes, rec_bytes) != cudaSuccess || pool_alloc(ctx, &sc->d_inst, inst_bytes) != cudaSuccess ||
+      pool_alloc(ctx, &sc->d_mats, sizeof(eos_material) * n_materials) != cudaSuccess ||
+      pool_alloc(ctx, &sc->d_lights, sizeof(eos_light) * std::max<uint32_t>(1, n_lights)) != cudaSuccess) {
     cudaGetLastError();
     return fail(EOS_ERR_OOM);
   }

@@ -605,7 +605,7 @@ eos_status write_records(eos_ctx* ctx, const BinaryTree& T, int root, int width,
 // with two children per record instead; a binary tree's depth is at most 62 <= kStackMax.
 eos_status build_records(eos_ctx* ctx, eos_scene* sc, const BinaryTree& T, int root) {
   const int max_nodes = T.n - 1;
-  EOS_CUDA(scene_alloc(ctx, &sc->d_nodes, 128 * (size_t)max_nodes));
+  EOS_CUDA(pool_alloc(ctx, &sc->d_nodes, 128 * (size_t)max_nodes));
   sc->device_bytes += 128 * (size_t)max_nodes;
   int levels = 0, records = 0;
   eos_status es = write_records(ctx, T, root, sc->width, (float4*)sc->d_nodes, max_nodes, &levels, &records);
@@ -631,11 +631,11 @@ eos_status build_scene(eos_ctx* ctx, eos_scene* sc, const float* d_verts, const 
   eos_status es = EOS_OK;
   const size_t n_nodes = std::max<size_t>(1, nn - 1);
   // persistent scene buffers (node records: build_records, or one root record below)
-  EOS_CUDA(scene_alloc(ctx, &sc->d_tris, 48 * nn));
-  EOS_CUDA(scene_alloc(ctx, &sc->d_shade, 48 * nn));
-  EOS_CUDA(scene_alloc(ctx, &sc->d_pos_of_id, 4 * nn));
-  EOS_CUDA(scene_alloc(ctx, &sc->d_codes, 4 * nn));
-  EOS_CUDA(scene_alloc(ctx, &sc->d_order, 4 * nn));
+  EOS_CUDA(pool_alloc(ctx, &sc->d_tris, 48 * nn));
+  EOS_CUDA(pool_alloc(ctx, &sc->d_shade, 48 * nn));
+  EOS_CUDA(pool_alloc(ctx, &sc->d_pos_of_id, 4 * nn));
+  EOS_CUDA(pool_alloc(ctx, &sc->d_codes, 4 * nn));
+  EOS_CUDA(pool_alloc(ctx, &sc->d_order, 4 * nn));
   sc->device_bytes += 48 * nn * 2 + 4 * nn * 3;
   // temporaries
   float4* cent = (float4*)scratch(ctx, "lbvh.cent", 16 * nn, &es);
@@ -713,7 +713,7 @@ eos_status build_scene(eos_ctx* ctx, eos_scene* sc, const float* d_verts, const 
     if (ws != EOS_OK) return ws;
   } else {
     if (n == 1) records(nullptr, blo, bhi);
-    EOS_CUDA(scene_alloc(ctx, &sc->d_nodes, 128));
+    EOS_CUDA(pool_alloc(ctx, &sc->d_nodes, 128));
     sc->device_bytes += 128;
     k_small_root<<<1, 1, 0, st>>>(n, blo, bhi, (float4*)sc->d_nodes);
     sc->n_nodes = 1;

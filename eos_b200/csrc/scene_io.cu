@@ -232,7 +232,7 @@ extern "C" eos_status eos_scene_load(eos_ctx* ctx, const char* path, eos_scene**
   const std::vector<Part> ps = parts(sc, n, h.n_nodes, h.n_obj, h.n_lights);
   for (const Part& p : ps) {
     const size_t bytes = std::max<size_t>(p.bytes, 16);
-    if (eos::scene_alloc(ctx, p.dev, bytes) != cudaSuccess) {
+    if (eos::pool_alloc(ctx, p.dev, bytes) != cudaSuccess) {
       cudaGetLastError();
       return fail(EOS_ERR_OOM);
     }
