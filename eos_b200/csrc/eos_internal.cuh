@@ -113,6 +113,7 @@ struct eos_ctx {
   unsigned long long* d_counts = nullptr; // ray / traversal counters [kCounters]
   std::map<std::string, eos::DevBuffer> scratch;
   cudaMemPool_t pool = nullptr;  // scene arrays and small scratch (pool_alloc)
+  std::vector<float> bw_cams;  // cameras of the adjoint call in progress
   void* pinned = nullptr;
   size_t pinned_bytes = 0;
   // read-back ring of the builders' launches that run ahead of the host (made on first use,
