@@ -43,7 +43,6 @@ eos_ctx::~eos_ctx() {
   if (ring_host) cudaFreeHost(ring_host);
   for (cudaEvent_t e : ring_ev)
     if (e) cudaEventDestroy(e);
-  if (d_err) cudaFree(d_err);
   if (d_counts) cudaFree(d_counts);
   if (ev0) cudaEventDestroy(ev0);
   if (ev1) cudaEventDestroy(ev1);
@@ -128,6 +127,12 @@ bool is_device_ptr(const void* p) {
 
 namespace {
 
+// The context's device words (eos_ctx::d_counts).
+struct CallWords {
+  unsigned long long c[kCounters];
+  int err, work;
+};
+
 // Device view of a caller buffer: device pointers pass through, host buffers are copied
 // into a named scratch buffer on the context stream.
 const void* stage_in(eos_ctx* ctx, const char* name, const void* p, size_t bytes, eos_status* st) {
@@ -172,19 +177,14 @@ eos_status copy_out(eos_ctx* ctx, const OutBuf& o) {
 eos_status begin_call(eos_ctx* ctx) {
   ctx->launches = 0;
   ctx->stage_ms[0] = ctx->stage_ms[1] = ctx->stage_ms[2] = 0.0f;
-  EOS_CUDA(cudaMemsetAsync(ctx->d_err, 0, sizeof(int), ctx->stream));
-  EOS_CUDA(cudaMemsetAsync(ctx->d_counts, 0, kCounters * sizeof(unsigned long long), ctx->stream));
+  EOS_CUDA(cudaMemsetAsync(ctx->d_counts, 0, sizeof(CallWords), ctx->stream));
   return EOS_OK;
 }
 
 // Waits for the call, reads the error word (and counters into stats).
 eos_status end_call(eos_ctx* ctx, eos_stats* stats) {
-  struct {
-    unsigned long long c[kCounters];
-    int err;
-  } h;
-  EOS_CUDA(cudaMemcpyAsync(h.c, ctx->d_counts, sizeof h.c, cudaMemcpyDeviceToHost, ctx->stream));
-  EOS_CUDA(cudaMemcpyAsync(&h.err, ctx->d_err, sizeof(int), cudaMemcpyDeviceToHost, ctx->stream));
+  CallWords h;
+  EOS_CUDA(cudaMemcpyAsync(&h, ctx->d_counts, sizeof h, cudaMemcpyDeviceToHost, ctx->stream));
   EOS_CUDA(cudaStreamSynchronize(ctx->stream));
   if (stats) {
     stats->primary_rays = h.c[0];
@@ -361,10 +361,10 @@ eos_status eos_ctx_create(int32_t device, eos_ctx** out) {
       break;
     }
     if (cudaEventCreate(&ctx->ev0) != cudaSuccess || cudaEventCreate(&ctx->ev1) != cudaSuccess) { st = EOS_ERR_CUDA; break; }
-    if (cudaMalloc(&ctx->d_err, sizeof(int)) != cudaSuccess) { st = EOS_ERR_OOM; break; }
-    if (cudaMalloc(&ctx->d_counts, kCounters * sizeof(unsigned long long)) != cudaSuccess) { st = EOS_ERR_OOM; break; }
-    cudaMemset(ctx->d_err, 0, sizeof(int));
-    cudaMemset(ctx->d_counts, 0, kCounters * sizeof(unsigned long long));
+    if (cudaMalloc(&ctx->d_counts, sizeof(CallWords)) != cudaSuccess) { st = EOS_ERR_OOM; break; }
+    cudaMemset(ctx->d_counts, 0, sizeof(CallWords));
+    ctx->d_err = &reinterpret_cast<CallWords*>(ctx->d_counts)->err;
+    ctx->d_work = &reinterpret_cast<CallWords*>(ctx->d_counts)->work;
   } while (0);
   if (st != EOS_OK) {
     cudaGetLastError();

@@ -109,8 +109,11 @@ struct eos_ctx {
   cudaStream_t own_stream = nullptr;
   cudaStream_t stream = nullptr;
   cudaEvent_t ev0 = nullptr, ev1 = nullptr;
-  int* d_err = nullptr;                   // device error word
-  unsigned long long* d_counts = nullptr; // ray / traversal counters [kCounters]
+  // one block of device words, cleared at the start of a call and read back whole at its end:
+  // ray / traversal counters [kCounters], the error word and the plain renderer's work counter
+  unsigned long long* d_counts = nullptr;
+  int* d_err = nullptr;
+  int* d_work = nullptr;
   std::map<std::string, eos::DevBuffer> scratch;
   cudaMemPool_t pool = nullptr;  // scene arrays and small scratch (pool_alloc)
   std::vector<float> bw_cams;  // cameras of the adjoint call in progress

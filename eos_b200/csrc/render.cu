@@ -1,11 +1,12 @@
-// Plain renderer: one launch per frame, one thread per pixel (all its samples), the whole
-// Whitted path of that pixel in the thread: nearest hit, one shadow ray per light, Phong,
+// Plain renderer: one launch per frame, a lane per pixel (all its samples), the whole
+// Whitted path of that pixel in the lane: nearest hit, one shadow ray per light, Phong,
 // mirror bounce up to trace_depth (src/RayTracer.cpp:99-174,268-458).  This is the
 // B200 replacement of the reference's primary-only __rayTrace_MegaKernel
 // (src/kernelInvocations.cu:172-310) with the CPU renderer's full semantics.
 //
 // Also the ray-query kernels behind eos_trace_closest / eos_trace_any.
 #include <algorithm>
+#include <type_traits>
 
 #include "trace.cuh"
 
@@ -27,127 +28,177 @@ struct PlainParams {
   eos_tree_node* tree;         // tree-form records (TREE kernel): EOS_TREE_NODES(trace_depth) per path
   int* err;
   unsigned long long* counts;  // kNumCounts traversal counters
+  uint32_t* work;     // pixels taken (zero at the call's start)
+  uint32_t n_work;    // pixels of the band's 8x4 tiles
+  int lanes;          // lanes of a warp that trace (lanes_of)
 };
 
-// One path: colour with the reference's fold c_k = phong_k + w_k c_{k+1} (fold_colour).
+// A shaded hit: its point, normal and material, the Phong sum over its unblocked lights and
+// the mask of the blocked ones.
+struct ShadedHit {
+  f3 P, N, phong;
+  const float* m;
+  uint32_t mask;
+};
+
 template <int SH>
-__device__ f3 trace_path(const PlainParams& P, f3 o, f3 d, int32_t* hits, uint32_t* masks, unsigned* cnt,
-                         uint32_t col, uint32_t stride) {
+__device__ __forceinline__ ShadedHit shade_hit(const PlainParams& P, f3 o, f3 d, const Hit& h, unsigned* cnt,
+                                               uint32_t col, uint32_t stride) {
   const DevScene& s = P.s;
+  const f3 campos = mk3(P.cam[0], P.cam[1], P.cam[2]);
+  ShadedHit r;
+  int obj;
+  hit_geometry(s, o, d, h, r.P, r.N, obj);
+  r.m = s.mats + kMatStride * obj;
+  r.phong = mk3(0.0f, 0.0f, 0.0f);
+  r.mask = 0;
+  for (int li = 0; li < s.n_lights; ++li) {
+    const float* l = s.lights + 6 * li;
+    f3 sd = norm3(sub3(mk3(l[0], l[1], l[2]), r.P));
+    f3 so = add3(r.P, scale3(kRayEps, sd));
+    cnt[kCntShadow]++;
+    AnyResult ar = any_hit<SH>(s, so, sd, col, stride, P.err);
+    cnt[kCntNodesA] += ar.nodes;
+    cnt[kCntTestsA] += ar.tests;
+    if (ar.hit) r.mask |= 1u << li;
+    else r.phong = add3(r.phong, phong_light(r.m, l, r.P, r.N, campos));
+  }
+  return r;
+}
+
+// A path of one secondary ray per hit, traced a ray at a time: begin, then step until it
+// returns true; colour with the reference's fold c_k = phong_k + w_k c_{k+1} (fold_colour).
+template <int SH>
+struct ChainPath {
+  f3 o, d;
+  int k;  // bounce of the ray
   f3 phong[kMaxBounces];
   float weight[kMaxBounces];
-  int nb = 0;
-  const f3 campos = mk3(P.cam[0], P.cam[1], P.cam[2]);
-  for (int k = 0; k <= P.trace_depth; ++k) {
+  int32_t hits[kMaxBounces];
+  uint32_t masks[kMaxBounces];
+
+  __device__ __forceinline__ void begin(const PlainParams& P, size_t path) {
+    k = 0;
+#pragma unroll
+    for (int i = 0; i < kMaxBounces; ++i) {
+      hits[i] = EOS_HIT_UNTRACED;
+      masks[i] = 0;
+    }
+  }
+  __device__ __forceinline__ bool step(const PlainParams& P, size_t path, f3& c, unsigned* cnt, uint32_t col,
+                                       uint32_t stride) {
+    const DevScene& s = P.s;
     cnt[k == 0 ? kCntPrimary : kCntSecondary]++;
     Hit h = closest_hit<SH>(s, o, d, col, stride, P.err);
     cnt[kCntNodesC] += h.nodes;
     cnt[kCntTestsC] += h.tests;
-    if (h.pos < 0) {
-      hits[k] = EOS_HIT_NONE;
-      break;
+    int nb = k;
+    hits[k] = h.pos < 0 ? EOS_HIT_NONE : h.id;
+    if (h.pos >= 0) {
+      cnt[kCntHits]++;
+      const ShadedHit r = shade_hit<SH>(P, o, d, h, cnt, col, stride);
+      masks[k] = r.mask;
+      phong[k] = r.phong;
+      nb = k + 1;
+      f3 ro, rd;
+      if (secondary_ray(r.m, s.ambient_index, d, r.P, r.N, ro, rd, weight[k]) && k < P.trace_depth) {
+        o = ro;
+        d = rd;
+        ++k;
+        return false;
+      }
     }
-    hits[k] = h.id;
-    cnt[kCntHits]++;
-    f3 Pp, N;
-    int obj;
-    hit_geometry(s, o, d, h, Pp, N, obj);
-    const float* m = s.mats + kMatStride * obj;
-    f3 acc = mk3(0.0f, 0.0f, 0.0f);
-    uint32_t mask = 0;
-    for (int li = 0; li < s.n_lights; ++li) {
-      const float* l = s.lights + 6 * li;
-      f3 sd = norm3(sub3(mk3(l[0], l[1], l[2]), Pp));
-      f3 so = add3(Pp, scale3(kRayEps, sd));
-      cnt[kCntShadow]++;
-      AnyResult ar = any_hit<SH>(s, so, sd, col, stride, P.err);
-      cnt[kCntNodesA] += ar.nodes;
-      cnt[kCntTestsA] += ar.tests;
-      if (ar.hit)
-        mask |= 1u << li;
-      else
-        acc = add3(acc, phong_light(m, l, Pp, N, campos));
+    c = mk3(0.0f, 0.0f, 0.0f);
+    for (int i = nb - 1; i >= 0; --i) c = fold_colour(phong[i], weight[i], c);
+    if (P.hit) P.hit[path] = hits[0];
+    if (P.paths) {
+      eos_path_record rec;
+#pragma unroll
+      for (int i = 0; i < kMaxBounces; ++i) {
+        rec.hit[i] = hits[i];
+        rec.shadow[i] = masks[i];
+      }
+      P.paths[path] = rec;
     }
-    masks[k] = mask;
-    phong[k] = acc;
-    nb = k + 1;
-    f3 ro, rd;
-    if (!secondary_ray(m, s.ambient_index, d, Pp, N, ro, rd, weight[k])) break;
-    o = ro;
-    d = rd;
+    return true;
   }
-  f3 c = mk3(0.0f, 0.0f, 0.0f);
-  for (int k = nb - 1; k >= 0; --k) c = fold_colour(phong[k], weight[k], c);
-  return c;
-}
+};
 
-// One shaded node of a ray tree waiting for its children (trace_tree).
+// One shaded node of a ray tree waiting for its children (TreePath).
 struct TreeFrame {
   f3 phong, cR;   // the node's Phong sum; its mirror child's colour once known
-  f3 to, td;      // its transparent child's ray
+  f3 to, td;      // its transparent child's ray; to: that child's colour once another lane has it
   float wR, K;    // reflectivity (0: no mirror ray), Fresnel weight of the transparent ray
   int node, depth;
   bool has_t;     // transparent ray present
-  bool in_t;      // the child being traced is the transparent one
+  bool in_t;      // the child being traced (or waited for) is the transparent one
 };
 
 // A path as a ray tree (materials both reflective and transparent trace both secondary
-// rays, src/RayTracer.cpp:339-407): a post-order walk with an explicit stack of shaded
-// nodes (at most one per bounce), mirror child first as the reference recurses; node
-// colours by tree_colour.  rec (nullable): the path's tree record, heap order.
+// rays, src/RayTracer.cpp:339-407), traced a ray at a time: a post-order walk with an
+// explicit stack of shaded nodes (at most one per bounce), mirror child first as the
+// reference recurses; node colours by tree_colour.  Tree records in heap order.
+//
+// What bounds a frame of ray trees is the serial walk of its deepest trees (31 nodes at trace
+// depth 4, each with its shadow rays), while most lanes' trees end after a ray or two.  So a
+// lane without a tree takes the transparent child of a waiting node from another lane of
+// its warp (share): the subtree nearest the root first, whose colour goes back to the
+// owner's frame, which sums it in its place, with the same operations.
 template <int SH>
-__device__ f3 trace_tree(const PlainParams& P, f3 o, f3 d, eos_tree_node* rec, int& root_hit, unsigned* cnt,
-                         uint32_t col, uint32_t stride) {
-  const DevScene& s = P.s;
-  const f3 campos = mk3(P.cam[0], P.cam[1], P.cam[2]);
-  const f3 zero = mk3(0.0f, 0.0f, 0.0f);
+struct TreePath {
+  f3 o, d;
+  int sp, node, depth;
+  uint32_t open;   // frames whose transparent child is still to be traced, by bit
+  uint32_t lent;   // frames whose transparent child another lane traces
+  int owner;       // lane and frame that this subtree's colour goes to, (lane | frame << 8); -1: a pixel
+  bool waiting;    // for the lent child of the top frame: nothing to trace
   TreeFrame st[kMaxBounces];
-  int sp = 0, node = 0, depth = 0;
-  for (;;) {
-    // trace the ray of (node, depth <= trace_depth) and shade its hit
-    f3 c = zero;
+
+  __device__ __forceinline__ void begin(const PlainParams& P, size_t path) {
+    sp = node = depth = 0;
+    open = lent = 0;
+    owner = -1;
+    waiting = false;
+    if (P.tree) {
+      const int nn = EOS_TREE_NODES(P.trace_depth);
+      eos_tree_node* rec = P.tree + path * nn;
+      for (int k = 0; k < nn; ++k) rec[k] = eos_tree_node{EOS_HIT_UNTRACED, 0u};
+    }
+  }
+  // The colour waited for is there: hand_up goes on.
+  __device__ __forceinline__ bool resumes() const { return waiting && !(lent >> (sp - 1) & 1u); }
+
+  __device__ __forceinline__ bool step(const PlainParams& P, size_t path, f3& c, unsigned* cnt, uint32_t col,
+                                       uint32_t stride) {
+    const DevScene& s = P.s;
+    const f3 zero = mk3(0.0f, 0.0f, 0.0f);
+    c = zero;
     cnt[depth == 0 ? kCntPrimary : kCntSecondary]++;
     Hit h = closest_hit<SH>(s, o, d, col, stride, P.err);
     cnt[kCntNodesC] += h.nodes;
     cnt[kCntTestsC] += h.tests;
-    if (node == 0) root_hit = h.pos < 0 ? EOS_HIT_NONE : h.id;
-    if (h.pos < 0) {
-      if (rec) rec[node].hit = EOS_HIT_NONE;
-    } else {
+    const int id = h.pos < 0 ? EOS_HIT_NONE : h.id;
+    if (node == 0 && P.hit) P.hit[path] = id;
+    eos_tree_node* rec = P.tree ? P.tree + path * EOS_TREE_NODES(P.trace_depth) + node : nullptr;
+    if (rec) rec->hit = id;
+    if (h.pos >= 0) {
       cnt[kCntHits]++;
-      f3 Pp, N;
-      int obj;
-      hit_geometry(s, o, d, h, Pp, N, obj);
-      const float* m = s.mats + kMatStride * obj;
+      const ShadedHit r = shade_hit<SH>(P, o, d, h, cnt, col, stride);
+      if (rec) rec->shadow = r.mask;
       TreeFrame F;
-      F.phong = zero;
-      uint32_t mask = 0;
-      for (int li = 0; li < s.n_lights; ++li) {
-        const float* l = s.lights + 6 * li;
-        f3 sd = norm3(sub3(mk3(l[0], l[1], l[2]), Pp));
-        f3 so = add3(Pp, scale3(kRayEps, sd));
-        cnt[kCntShadow]++;
-        AnyResult ar = any_hit<SH>(s, so, sd, col, stride, P.err);
-        cnt[kCntNodesA] += ar.nodes;
-        cnt[kCntTestsA] += ar.tests;
-        if (ar.hit) mask |= 1u << li;
-        else F.phong = add3(F.phong, phong_light(m, l, Pp, N, campos));
-      }
-      if (rec) {
-        rec[node].hit = h.id;
-        rec[node].shadow = mask;
-      }
+      F.phong = r.phong;
       f3 ro = zero, rd = zero;
-      const bool has_r = m[7] > 0.0f;
-      F.wR = has_r ? m[7] : 0.0f;
-      if (has_r) mirror_ray(d, Pp, N, ro, rd);
-      F.has_t = m[8] > 0.0f;
-      F.K = F.has_t ? transparent_ray(m, s.ambient_index, d, Pp, N, F.to, F.td) : 0.0f;
+      const bool has_r = r.m[7] > 0.0f;
+      F.wR = has_r ? r.m[7] : 0.0f;
+      if (has_r) mirror_ray(d, r.P, r.N, ro, rd);
+      F.has_t = r.m[8] > 0.0f;
+      F.K = F.has_t ? transparent_ray(r.m, s.ambient_index, d, r.P, r.N, F.to, F.td) : 0.0f;
       F.cR = zero;
       F.node = node;
       F.depth = depth;
       if (depth < P.trace_depth && (has_r || F.has_t)) {
         F.in_t = !has_r;
+        if (has_r && F.has_t) open |= 1u << sp;
         st[sp++] = F;
         if (has_r) {
           o = ro;
@@ -159,32 +210,113 @@ __device__ f3 trace_tree(const PlainParams& P, f3 o, f3 d, eos_tree_node* rec, i
           node = 2 * node + 2;
         }
         ++depth;
-        continue;
+        return false;
       }
       c = tree_colour(F.phong, F.wR, zero, F.has_t, F.K, zero);  // children beyond the trace depth
     }
-    // hand the colour up until a node still has its transparent child to trace
-    bool next = false;
+    return hand_up(c);
+  }
+  // Hands a finished child's colour up until a node still has its transparent child to
+  // trace or to wait for; true: c is the whole tree's.
+  __device__ __forceinline__ bool hand_up(f3& c) {
+    const f3 zero = mk3(0.0f, 0.0f, 0.0f);
+    if (waiting) {
+      const TreeFrame& F = st[--sp];
+      waiting = false;
+      c = tree_colour(F.phong, F.wR, F.cR, true, F.K, F.to);
+    }
     while (sp > 0) {
       TreeFrame& F = st[sp - 1];
+      const uint32_t bit = 1u << (sp - 1);
       if (!F.in_t) {
         F.cR = c;
         if (F.has_t) {
           F.in_t = true;
-          o = F.to;
-          d = F.td;
-          node = 2 * F.node + 2;
-          depth = F.depth + 1;
-          next = true;
-          break;
+          if (open & bit) {
+            open &= ~bit;
+            o = F.to;
+            d = F.td;
+            node = 2 * F.node + 2;
+            depth = F.depth + 1;
+            return false;
+          }
+          if (lent & bit) {
+            waiting = true;
+            return false;
+          }
+          c = tree_colour(F.phong, F.wR, F.cR, true, F.K, F.to);  // another lane traced it
+        } else {
+          c = tree_colour(F.phong, F.wR, F.cR, false, 0.0f, zero);
         }
-        c = tree_colour(F.phong, F.wR, F.cR, false, 0.0f, zero);
       } else {
         c = tree_colour(F.phong, F.wR, F.cR, true, F.K, c);
       }
       --sp;
     }
-    if (!next) return c;
+    return true;
+  }
+};
+
+// The `idle` lanes take open subtrees of the warp's other lanes, with the owner's pixel (x, ly,
+// smp).  Warp-uniform.
+template <int SH>
+__device__ __forceinline__ void share_trees(TreePath<SH>& t, uint32_t idle, bool& active, bool& fresh, int& x, int& ly,
+                                            int& smp) {
+  const int lane = threadIdx.x & 31;
+  uint32_t open = __ballot_sync(0xffffffffu, active && t.open != 0);
+  while (open && idle) {
+    const int from = __ffs(open) - 1, to = __ffs(idle) - 1;
+    open &= open - 1;
+    idle &= idle - 1;
+    f3 o = mk3(0, 0, 0), d = o;
+    int node = 0, depth = 0, frame = 0;
+    if (lane == from) {
+      frame = __ffs(t.open) - 1;
+      t.open &= t.open - 1;
+      t.lent |= 1u << frame;
+      const TreeFrame& F = t.st[frame];
+      o = F.to;
+      d = F.td;
+      node = 2 * F.node + 2;
+      depth = F.depth + 1;
+    }
+    o = mk3(__shfl_sync(~0u, o.x, from), __shfl_sync(~0u, o.y, from), __shfl_sync(~0u, o.z, from));
+    d = mk3(__shfl_sync(~0u, d.x, from), __shfl_sync(~0u, d.y, from), __shfl_sync(~0u, d.z, from));
+    node = __shfl_sync(~0u, node, from);
+    depth = __shfl_sync(~0u, depth, from);
+    frame = __shfl_sync(~0u, frame, from);
+    const int fx = __shfl_sync(~0u, x, from), fly = __shfl_sync(~0u, ly, from), fsmp = __shfl_sync(~0u, smp, from);
+    if (lane == to) {
+      t.o = o;
+      t.d = d;
+      t.node = node;
+      t.depth = depth;
+      t.sp = 0;
+      t.open = t.lent = 0;
+      t.owner = from | (frame << 8);
+      t.waiting = false;
+      x = fx;
+      ly = fly;
+      smp = fsmp;
+      active = true;
+      fresh = false;
+    }
+  }
+}
+
+// Colours of the subtrees that lanes of `done` have finished go to their owners.  Warp-uniform.
+template <int SH>
+__device__ __forceinline__ void return_trees(TreePath<SH>& t, uint32_t done, f3 c) {
+  const int lane = threadIdx.x & 31;
+  while (done) {
+    const int from = __ffs(done) - 1;
+    done &= done - 1;
+    const int owner = __shfl_sync(~0u, t.owner, from);
+    const f3 v = mk3(__shfl_sync(~0u, c.x, from), __shfl_sync(~0u, c.y, from), __shfl_sync(~0u, c.z, from));
+    if (lane == (owner & 255)) {
+      t.st[owner >> 8].to = v;
+      t.lent &= ~(1u << (owner >> 8));
+    }
   }
 }
 
@@ -196,63 +328,90 @@ __global__ void __maxnreg__(64) k_render_plain(PlainParams P) {
   extern __shared__ uint2 shstack[];
   const uint32_t col = shared_address(shstack + threadIdx.x), stride = 8 * blockDim.x;
   unsigned cnt[kNumCounts] = {0, 0, 0, 0, 0, 0, 0, 0};
-  // one warp = one 8x4 pixel tile (coherent primary rays)
-  const int g = blockIdx.x * blockDim.x + threadIdx.x;
+  const int lane = threadIdx.x & 31;
   const int tiles_x = (P.width + 7) >> 3;
-  const int tile = g >> 5, lane = g & 31;
-  const int x = (tile % tiles_x) * 8 + (lane & 7);
-  const int ly = (tile / tiles_x) * 4 + (lane >> 3);  // row within the rendered band
-  const int y = P.y0 + ly;
-  const int img_pix = y * P.width + x;  // pixel of the whole image: its sample hash
-  const int pix = ly * P.width + x;     // pixel of the outputs
-  if (x < P.width && ly < P.rows) {
-    f3 sum = mk3(0.0f, 0.0f, 0.0f);
-    for (int smp = 0; smp < P.spp; ++smp) {
-      float ox, oy;
-      sample_offset((uint32_t)img_pix, smp, P.spp, P.jitter_seed, P.pixel_offset, ox, oy, P.grid);
-      f3 d = primary_direction(P.cam, P.width, P.height, x, y, ox, oy);
-      f3 o = mk3(P.cam[0], P.cam[1], P.cam[2]);
-      size_t path = (size_t)pix * P.spp + smp;
-      if constexpr (TREE) {
-        const int nn = EOS_TREE_NODES(P.trace_depth);
-        eos_tree_node* rec = P.tree ? P.tree + path * nn : nullptr;
-        if (rec)
-          for (int k = 0; k < nn; ++k) rec[k] = eos_tree_node{EOS_HIT_UNTRACED, 0u};
-        int root_hit = EOS_HIT_NONE;
-        f3 c = trace_tree<SH>(P, o, d, rec, root_hit, cnt, col, stride);
-        sum = add3(sum, c);
-        if (P.hit) P.hit[path] = root_hit;
-      } else {
-        int32_t hits[kMaxBounces];
-        uint32_t masks[kMaxBounces];
-#pragma unroll
-        for (int k = 0; k < kMaxBounces; ++k) {
-          hits[k] = EOS_HIT_UNTRACED;
-          masks[k] = 0;
-        }
-        f3 c = trace_path<SH>(P, o, d, hits, masks, cnt, col, stride);
-        sum = add3(sum, c);
-        if (P.hit) P.hit[path] = hits[0];
-        if (P.paths) {
-          eos_path_record rec;
-#pragma unroll
-          for (int k = 0; k < kMaxBounces; ++k) {
-            rec.hit[k] = hits[k];
-            rec.shadow[k] = masks[k];
-          }
-          P.paths[path] = rec;
-        }
+  typename std::conditional<TREE, TreePath<SH>, ChainPath<SH>>::type path;
+  bool active = false, fresh = false;  // a pixel in hand; its next sample not begun
+  bool more = lane < P.lanes;          // may take another pixel
+  int x = 0, ly = 0, smp = 0;
+  f3 sum = mk3(0.0f, 0.0f, 0.0f);
+  for (;;) {
+    if constexpr (TREE) {
+      const uint32_t spare = __ballot_sync(0xffffffffu, lane < P.lanes && !active);
+      if (spare) share_trees(path, spare, active, fresh, x, ly, smp);
+    }
+    const uint32_t idle = __ballot_sync(0xffffffffu, more && !active);
+    const uint32_t busy = __ballot_sync(0xffffffffu, active);
+    // the next pixels once all lanes are done: taking them as single lanes end (or 8, 16, 24
+    // of them) mixes bounces in a warp and is no faster, 885 -> 906 us for a 1080p frame
+    if (idle && !busy) {
+      uint32_t base = 0;
+      if (lane == 0) base = atomicAdd(P.work, __popc(idle));
+      base = __shfl_sync(0xffffffffu, base, 0);
+      if (more && !active) {
+        const uint32_t g = base + __popc(idle & ((1u << lane) - 1u));
+        more = g < P.n_work;
+        // 32 consecutive pixels = one 8x4 tile (coherent primary rays)
+        const int tile = (int)(g >> 5), q = (int)(g & 31u);
+        x = (tile % tiles_x) * 8 + (q & 7);
+        ly = (tile / tiles_x) * 4 + (q >> 3);  // row within the rendered band
+        active = fresh = more && x < P.width && ly < P.rows;
+        smp = 0;
+        sum = mk3(0.0f, 0.0f, 0.0f);
       }
+    } else if (!busy) {
+      break;
     }
-    if (P.spp > 1 || P.grid > 0) sum = scale3(sample_weight(P.spp, P.grid), sum);
-    if (P.rgb) {
-      P.rgb[3 * (size_t)pix] = sum.x;
-      P.rgb[3 * (size_t)pix + 1] = sum.y;
-      P.rgb[3 * (size_t)pix + 2] = sum.z;
+    if (active && fresh) {
+      float ox, oy;  // the sample hash takes the pixel of the whole image
+      const int y = P.y0 + ly;
+      sample_offset((uint32_t)(y * P.width + x), smp, P.spp, P.jitter_seed, P.pixel_offset, ox, oy, P.grid);
+      path.d = primary_direction(P.cam, P.width, P.height, x, y, ox, oy);
+      path.o = mk3(P.cam[0], P.cam[1], P.cam[2]);
+      path.begin(P, ((size_t)ly * P.width + x) * P.spp + smp);
+      fresh = false;
     }
-    if (P.rgba8) {
-      uchar4 q = make_uchar4(quantize(sum.x), quantize(sum.y), quantize(sum.z), 255);
-      reinterpret_cast<uchar4*>(P.rgba8)[pix] = q;
+    // a ray of the path in hand (its index in the outputs); true when the path ends with colour c
+    auto trace = [&](f3& c) {
+      return path.step(P, ((size_t)ly * P.width + x) * P.spp + smp, c, cnt, col, stride);
+    };
+    auto end_sample = [&](f3 c) {
+      sum = add3(sum, c);
+      fresh = true;
+      if (++smp < P.spp) return;
+      active = false;
+      const size_t pix = (size_t)ly * P.width + x;  // pixel of the outputs
+      if (P.spp > 1 || P.grid > 0) sum = scale3(sample_weight(P.spp, P.grid), sum);
+      if (P.rgb) {
+        P.rgb[3 * pix] = sum.x;
+        P.rgb[3 * pix + 1] = sum.y;
+        P.rgb[3 * pix + 2] = sum.z;
+      }
+      if (P.rgba8)
+        reinterpret_cast<uchar4*>(P.rgba8)[pix] = make_uchar4(quantize(sum.x), quantize(sum.y), quantize(sum.z), 255);
+    };
+    if constexpr (!TREE) {
+      f3 c;
+      if (active && trace(c)) end_sample(c);
+      __syncwarp();
+    } else {
+      const bool traces = active && !path.waiting;
+      f3 c = mk3(0.0f, 0.0f, 0.0f);
+      bool ends = traces && trace(c);  // the tree, or the subtree in hand
+      // cannot happen: who waits has lent a subtree to a lane that traces or waits in turn
+      if (!__any_sync(0xffffffffu, traces) && __any_sync(0xffffffffu, active)) {
+        if (lane == 0) atomicOr(P.err, kErrTimeout);
+        break;
+      }
+      // subtree colours to their owners; owners that waited for one go on
+      uint32_t done = __ballot_sync(0xffffffffu, ends && path.owner >= 0);
+      while (done) {
+        return_trees(path, done, c);
+        if (done >> lane & 1u) active = ends = false;
+        if (active && !ends && path.resumes()) ends = path.hand_up(c);
+        done = __ballot_sync(0xffffffffu, ends && path.owner >= 0);
+      }
+      if (ends) end_sample(c);
     }
   }
 #pragma unroll
@@ -288,17 +447,42 @@ inline int pick_stack(int d) { return d <= 0 ? 16 : (d <= 8 ? 8 : (d <= 16 ? 16 
 
 namespace {
 
+// Lanes of a warp that trace.  A frame of few pixels is bound by the time of its slowest
+// warp, which walks the union of its lanes' nodes, while most of the chip idles: with fewer
+// lanes a warp the same pixels spread over more warps.  Chains: the fewest lanes that leave
+// every warp resident (32 warps of 64 registers per SM).  Measured, us at 32 / 16 / 8 / 4 lanes:
+// 64x64 of 200k triangles 243 / 219 / 207 / 166, 128x128 271 / 251 / 213 / 197, 256x256 284 /
+// 278 / 282, 512x512 405 / 448 / 569.  Ray trees have longer tails (a pixel's tree is walked by
+// a warp): 8 lanes up to four such fillings (400x300: 1,588 / 1,732 / 1,458), 16 up to eight
+// (961x541: 2,113 / 1,881 / 2,201; 1920x1080: 3,033 / 3,551).
+int lanes_of(uint32_t n_work, int num_sms, bool tree) {
+  const uint32_t full = 32u * (uint32_t)num_sms;  // warps that fill the chip
+  if (tree) return n_work / 8 <= 4 * full ? 8 : n_work / 16 <= 8 * full ? 16 : 32;
+  for (int lanes = 4; lanes < 32; lanes *= 2)
+    if (n_work / lanes <= full) return lanes;
+  return 32;
+}
+
+template <int SH, bool TREE>
+eos_status launch_plain(eos_ctx* ctx, const PlainParams& P, int block) {
+  const size_t smem = (size_t)SH * block * sizeof(uint2);
+  if (smem > 48 * 1024)  // opt in to more than the default 48 KB of dynamic shared memory
+    EOS_CUDA(cudaFuncSetAttribute(k_render_plain<SH, TREE>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
+  int resident = 0;
+  EOS_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&resident, k_render_plain<SH, TREE>, block, smem));
+  const long long per_block = (long long)P.lanes * (block / 32);
+  const long long blocks = ((long long)P.n_work + per_block - 1) / per_block;
+  const int grid = (int)std::max<long long>(1, std::min<long long>(blocks, (long long)ctx->num_sms * std::max(1, resident)));
+  k_render_plain<SH, TREE><<<grid, block, smem, ctx->stream>>>(P);
+  EOS_CUDA(cudaGetLastError());
+  return EOS_OK;
+}
+
 template <bool TREE>
-void launch_plain(const PlainParams& P, int sh, int grid, int block, size_t smem, cudaStream_t st) {
-  if (smem > 48 * 1024) {  // opt in to more than the default 48 KB of dynamic shared memory
-    if (sh == 8) cudaFuncSetAttribute(k_render_plain<8, TREE>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
-    else if (sh == 16)
-      cudaFuncSetAttribute(k_render_plain<16, TREE>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
-    else cudaFuncSetAttribute(k_render_plain<32, TREE>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
-  }
-  if (sh == 8) k_render_plain<8, TREE><<<grid, block, smem, st>>>(P);
-  else if (sh == 16) k_render_plain<16, TREE><<<grid, block, smem, st>>>(P);
-  else k_render_plain<32, TREE><<<grid, block, smem, st>>>(P);
+eos_status launch_plain(eos_ctx* ctx, const PlainParams& P, int sh, int block) {
+  if (sh == 8) return launch_plain<8, TREE>(ctx, P, block);
+  if (sh == 16) return launch_plain<16, TREE>(ctx, P, block);
+  return launch_plain<32, TREE>(ctx, P, block);
 }
 
 }  // namespace
@@ -331,14 +515,13 @@ eos_status render_plain(eos_ctx* ctx, const eos_scene* sc, const eos_camera& cam
   P.tree = tree ? (eos_tree_node*)paths : nullptr;
   P.err = ctx->d_err;
   P.counts = ctx->d_counts;
+  P.work = (uint32_t*)ctx->d_work;
+  P.n_work = (uint32_t)((long long)((cam.width + 7) / 8) * ((P.rows + 3) / 4) * 32);
+  P.lanes = lanes_of(P.n_work, ctx->num_sms, tree);
   const int block = clamp_block(p.block_size);
   const int sh = pick_stack(p.stack_depth);
-  const long long n_threads = (long long)((cam.width + 7) / 8) * ((P.rows + 3) / 4) * 32;
-  const int grid = (int)std::max<long long>(1, (n_threads + block - 1) / block);
-  const size_t smem = (size_t)sh * block * sizeof(uint2);
-  if (tree) launch_plain<true>(P, sh, grid, block, smem, ctx->stream);
-  else launch_plain<false>(P, sh, grid, block, smem, ctx->stream);
-  EOS_CUDA(cudaGetLastError());
+  const eos_status st = tree ? launch_plain<true>(ctx, P, sh, block) : launch_plain<false>(ctx, P, sh, block);
+  if (st != EOS_OK) return st;
   ctx->launches += 1;
   return EOS_OK;
 }
