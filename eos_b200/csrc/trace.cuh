@@ -572,14 +572,29 @@ __device__ __forceinline__ void to_object(const DevInstance* I, f3 o, f3 d, f3& 
            (c.x * d.x + c.y * d.y) + c.z * d.z);
 }
 
-// ANY: returns at the first hit (h.pos >= 0 then); otherwise the nearest hit.
-template <int SH, bool ANY>
-__device__ __noinline__ Hit traverse_instanced(const DevScene& s, f3 o, f3 d, uint32_t col, uint32_t stride,
-                                               int* err) {
+__device__ __forceinline__ bool prepare_ray(f3 o, f3 d, SlabRay& r) {
+  r = make_slab(o, d);
+  return true;
+}
+__device__ __forceinline__ bool prepare_ray(f3 o, f3 d, FmaSlabRay& r) {
+  const SlabRay e = make_slab(o, d);
+  r = make_fma_slab(e);
+  return fma_slab_ok(e);
+}
+
+// ANY: returns at the first hit (h.pos >= 0 then); otherwise the nearest hit.  *ok: false when
+// the ray, in world or some object space, needs the exact box test (Ray = FmaSlabRay only);
+// the result is then unusable.  The world-space ray is prepared again on the way out of an
+// instance rather than kept: its twelve registers would spill.
+template <int SH, bool ANY, class Ray>
+__device__ __forceinline__ Hit walk_instanced(const DevScene& s, f3 o, f3 d, uint32_t col, uint32_t stride, int* err,
+                                              bool* ok) {
+  constexpr float kCullR = RayCull<Ray>::k;
   Hit h;
   h.t = kInf; h.u = h.v = 0.0f; h.pos = -1; h.id = -1; h.nodes = 0; h.tests = 0;
-  const SlabRay rw = make_slab(o, d);
-  SlabRay r = rw;
+  Ray r;
+  *ok = prepare_ray(o, d, r);
+  if (!*ok) return h;
   f3 oo = o, od = d;
   const float4* nodes = s.nodes;
   const float4* tris = nullptr;
@@ -598,12 +613,12 @@ __device__ __noinline__ Hit traverse_instanced(const DevScene& s, f3 o, f3 d, ui
         return h;
       }
       if (ANY) follow_hits(st.top, stride, cur, ref, b.tn, b.tf);
-      else cur = follow_nearest(st, ref, b, h.t * kCull);
+      else cur = follow_nearest(st, ref, b, h.t * kCullR);
       continue;
     }
     if (cur == kDone) return h;
     if (cur == kExitMesh) {  // back to the instance tree
-      r = rw;
+      prepare_ray(o, d, r);
       nodes = s.nodes;
       in_mesh = false;
     } else if (cur == kRefill) {
@@ -611,7 +626,8 @@ __device__ __noinline__ Hit traverse_instanced(const DevScene& s, f3 o, f3 d, ui
     } else if (!in_mesh) {  // an instance: continue in its mesh, in object space
       const DevInstance* I = s.inst + leaf_first(cur);
       to_object(I, o, d, oo, od);
-      r = make_slab(oo, od);
+      *ok = prepare_ray(oo, od, r);
+      if (!*ok) return h;
       nodes = I->nodes;
       tris = I->tris;
       id_off = I->id_offset;
@@ -642,8 +658,33 @@ __device__ __noinline__ Hit traverse_instanced(const DevScene& s, f3 o, f3 d, ui
         }
       }
     }
-    cur = ANY ? st.pop() : st.pop_within(h.t * kCull);
+    cur = ANY ? st.pop() : st.pop_within(h.t * kCullR);
   }
+}
+
+template <int SH, bool ANY>
+__device__ __noinline__ Hit walk_instanced_exact(const DevScene& s, f3 o, f3 d, uint32_t col, uint32_t stride,
+                                                 int* err) {
+  bool ok;
+  return walk_instanced<SH, ANY, SlabRay>(s, o, d, col, stride, err, &ok);
+}
+
+// In the fma box test's form; the rare ray that needs the exact one starts again in that.
+// (Carrying both forms with a branch per visit cost 13 %; the exact form alone 10 % more than
+// this: 1080p view of 801 instances 12.1 -> 10.9 ms with the traversal inline.  Letting lanes
+// descend until all hold a leaf is slower, 10.1 -> 11.7: lanes change space at each instance.)
+template <int SH, bool ANY>
+__device__ __forceinline__ Hit traverse_instanced(const DevScene& s, f3 o, f3 d, uint32_t col, uint32_t stride,
+                                               int* err) {
+  bool ok;
+  const Hit h = walk_instanced<SH, ANY, FmaSlabRay>(s, o, d, col, stride, err, &ok);
+  return ok ? h : walk_instanced_exact<SH, ANY>(s, o, d, col, stride, err);
+}
+
+template <int SH, bool ANY>
+__device__ __noinline__ Hit traverse_instanced_call(const DevScene& s, f3 o, f3 d, uint32_t col, uint32_t stride,
+                                                    int* err) {
+  return traverse_instanced<SH, ANY>(s, o, d, col, stride, err);
 }
 
 // Instance holding global triangle id `gid` (instances in id order).
@@ -657,24 +698,34 @@ __device__ __forceinline__ const DevInstance* instance_of(const DevScene& s, int
   return s.inst + lo;
 }
 
-// CAP (inline traversals of flat scenes only): total stack entries, see TraversalStack.
-template <int SH, bool INLINE = false, int CAP = kStackMax>
-__device__ __forceinline__ Hit closest_hit(const DevScene& s, f3 o, f3 d, uint32_t col, uint32_t stride,
-                                            int* err) {
-  if (s.inst) return traverse_instanced<SH, false>(s, o, d, col, stride, err);
-  if (INLINE) return closest_hit_body<SH, CAP>(s, o, d, col, stride, err);
-  return closest_hit_call<SH>(s, o, d, col, stride, err);
+// How a kernel holds the traversals: kCalls both out of line (bounds the registers of a kernel
+// that makes several kinds of queries), kFlat the flat one inline and none for two-level
+// scenes, kTwoLevel the two-level one inline and the flat one out of line.  CAP (inline
+// traversals of flat scenes): total stack entries, see ColumnStack.
+enum TraversalForm { kCalls, kFlat, kTwoLevel };
+
+template <int SH, TraversalForm F = kCalls, int CAP = kStackMax>
+__device__ __forceinline__ Hit closest_hit(const DevScene& s, f3 o, f3 d, uint32_t col, uint32_t stride, int* err) {
+  if constexpr (F == kTwoLevel) {
+    if (s.inst) return traverse_instanced<SH, false>(s, o, d, col, stride, err);
+  } else if constexpr (F == kCalls) {
+    if (s.inst) return traverse_instanced_call<SH, false>(s, o, d, col, stride, err);
+  }
+  if constexpr (F == kFlat || CAP == SH) return closest_hit_body<SH, CAP>(s, o, d, col, stride, err);
+  else return closest_hit_call<SH>(s, o, d, col, stride, err);
 }
 
-template <int SH, bool INLINE = false, int CAP = kStackMax>
-__device__ __forceinline__ AnyResult any_hit(const DevScene& s, f3 o, f3 d, uint32_t col, uint32_t stride,
-                                            int* err) {
-  if (s.inst) {
-    const Hit h = traverse_instanced<SH, true>(s, o, d, col, stride, err);
-    return AnyResult{h.pos >= 0 ? 1 : 0, h.nodes, h.tests};
+template <int SH, TraversalForm F = kCalls, int CAP = kStackMax>
+__device__ __forceinline__ AnyResult any_hit(const DevScene& s, f3 o, f3 d, uint32_t col, uint32_t stride, int* err) {
+  if constexpr (F != kFlat) {
+    if (s.inst) {
+      const Hit h = F == kTwoLevel ? traverse_instanced<SH, true>(s, o, d, col, stride, err)
+                                   : traverse_instanced_call<SH, true>(s, o, d, col, stride, err);
+      return AnyResult{h.pos >= 0 ? 1 : 0, h.nodes, h.tests};
+    }
   }
-  if (INLINE) return any_hit_body<SH, CAP>(s, o, d, col, stride, err);
-  return any_hit_call<SH>(s, o, d, col, stride, err);
+  if constexpr (F == kFlat || CAP == SH) return any_hit_body<SH, CAP>(s, o, d, col, stride, err);
+  else return any_hit_call<SH>(s, o, d, col, stride, err);
 }
 
 // Traversal work counters, reduced per warp into the context's counter block:

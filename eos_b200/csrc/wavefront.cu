@@ -164,7 +164,11 @@ __device__ __forceinline__ int budget(int n, int work_limit, int* err) {
 // cost 2 and 0.5 % of a four-view 1080p batch of 1.06M triangles (5,107 us), 5 and 4 % of a
 // 30-job batch.  The shadow kernels are capped at 56, one more block of 128 threads per SM
 // than at 64 for 12 B less of spill stores: 5,107 -> 5,049 us; 48 (196 B of spills) 5,521, 72
-// 5,131.  CAP is the traversal stack's size (ColumnStack): kStackMax, or SH for the
+// 5,131.  INST: the pass holds a two-level scene, whose traversal is inline in these kernels
+// only (TraversalForm); it keeps both spaces' rays and is latency-bound, so it gains more from
+// registers than from warps: 1080p view of 801 instances 10.9 ms at 64 / 64, 10.3 at 80 / 64,
+// 10.0 at 80 / 96 (nearest hit / shadow), 10.3 at 114 / 96; out of line 12.9 at 64 / 64 and
+// 16.3 at 64 / 56.  CAP is the traversal stack's size (ColumnStack): kStackMax, or SH for the
 // small-stack test limit.
 // Appends the secondary rays of the lanes with `want` to R_k+1 (ballot / popc compaction,
 // one atomic per warp); node = the ray-tree node of the ray (0 outside tree mode).
@@ -190,8 +194,8 @@ __device__ __forceinline__ void emit_secondary(const WfArgs& A, int* ctr, bool w
   }
 }
 
-template <bool PRIMARY, int SH, int CAP = kStackMax, bool TREE = false>
-__global__ void __launch_bounds__(256, 4) k_wf_closest(WfArgs A) {
+template <bool PRIMARY, int SH, int CAP, bool TREE, bool INST>
+__global__ void __launch_bounds__(256, INST ? 3 : 4) k_wf_closest(WfArgs A) {
   extern __shared__ uint2 shstack[];
   const uint32_t col = shared_address(shstack + threadIdx.x), stride = 8 * blockDim.x;
   int* ctr = A.ctr + A.k * kCtr;
@@ -243,7 +247,7 @@ __global__ void __launch_bounds__(256, 4) k_wf_closest(WfArgs A) {
       const DevJob& J = A.jobs[jb];
       if (valid) {
         ++nrays;
-        Hit h = closest_hit<SH, true, CAP>(J.s, o, d, col, stride, A.err);
+        Hit h = closest_hit<SH, INST ? kTwoLevel : kFlat, CAP>(J.s, o, d, col, stride, A.err);
         nodes += h.nodes;
         tests += h.tests;
         hit = h.pos >= 0;
@@ -356,8 +360,8 @@ __global__ void __launch_bounds__(256, 4) k_wf_closest(WfArgs A) {
   warp_add_count(&A.counts[kCntTestsC], tests);
 }
 
-template <int SH, int CAP = kStackMax>
-__global__ void __maxnreg__(56) k_wf_any(WfArgs A) {
+template <int SH, int CAP, bool INST>
+__global__ void __maxnreg__(INST ? 96 : 56) k_wf_any(WfArgs A) {
   extern __shared__ int shrefs[];
   const uint32_t col = shared_address(shrefs + threadIdx.x), stride = 4 * blockDim.x;
   int* ctr = A.ctr + A.k * kCtr;
@@ -373,7 +377,7 @@ __global__ void __maxnreg__(56) k_wf_any(WfArgs A) {
       int key = __float_as_int(s.b.w);
       const DevJob& J = A.jobs[key >> 5];
       AnyResult ar =
-          any_hit<SH, true, CAP>(J.s, mk3(s.a.x, s.a.y, s.a.z), mk3(s.b.x, s.b.y, s.b.z), col, stride, A.err);
+          any_hit<SH, INST ? kTwoLevel : kFlat, CAP>(J.s, mk3(s.a.x, s.a.y, s.a.z), mk3(s.b.x, s.b.y, s.b.z), col, stride, A.err);
       nodes += ar.nodes;
       tests += ar.tests;
       if (ar.hit) atomicOr(&A.masks[hi], 1u << (key & 31));
@@ -571,6 +575,12 @@ struct StageTimer {
 // `queue_chunk` rays and finishes all before taking more.  small_stack selects the test
 // instantiation whose traversal stack is its SH shared-memory entries only (launch_config
 // pins SH = 8 then); tree the ray-tree mode.
+// Shared-memory entries of the shadow kernels' 4-byte stack columns for a stack depth of sh:
+// a little more than the nearest-hit kernels' 8-byte ones.  Deep trees spill less (4K view of
+// 4.5M triangles 65.1 -> 64.6 ms, 801 instances 16.3 -> 16.1; 24 and 32 entries are no
+// better), the others are unchanged.
+constexpr int any_entries(int sh) { return sh == 16 ? 20 : sh; }
+
 template <int SH>
 struct StageKernels {
   void (*closest_primary)(WfArgs);
@@ -579,17 +589,22 @@ struct StageKernels {
   void (*shade)(WfArgs);
   void (*init)(WfArgs);
   void (*resolve)(WfArgs);
-  static StageKernels get(bool small_stack, bool tree) {
+  static StageKernels get(bool small_stack, bool tree, bool inst) {
+    return inst ? pick<true>(small_stack, tree) : pick<false>(small_stack, tree);
+  }
+  template <bool INST>
+  static StageKernels pick(bool small_stack, bool tree) {
+    constexpr int SA = any_entries(SH);
     if (tree)
-      return {k_wf_closest<true, SH, kStackMax, true>, k_wf_closest<false, SH, kStackMax, true>, k_wf_any<SH>,
-              k_wf_shade<true>, k_wf_init<true>, k_wf_resolve<true>};
+      return {k_wf_closest<true, SH, kStackMax, true, INST>, k_wf_closest<false, SH, kStackMax, true, INST>,
+              k_wf_any<SA, kStackMax, INST>, k_wf_shade<true>, k_wf_init<true>, k_wf_resolve<true>};
     if constexpr (SH == 8) {
       if (small_stack)
-        return {k_wf_closest<true, 8, 8>, k_wf_closest<false, 8, 8>, k_wf_any<8, 8>,
+        return {k_wf_closest<true, 8, 8, false, INST>, k_wf_closest<false, 8, 8, false, INST>, k_wf_any<8, 8, INST>,
                 k_wf_shade<false>, k_wf_init<false>, k_wf_resolve<false>};
     }
-    return {k_wf_closest<true, SH>, k_wf_closest<false, SH>, k_wf_any<SH>,
-            k_wf_shade<false>, k_wf_init<false>, k_wf_resolve<false>};
+    return {k_wf_closest<true, SH, kStackMax, false, INST>, k_wf_closest<false, SH, kStackMax, false, INST>,
+            k_wf_any<SA, kStackMax, INST>, k_wf_shade<false>, k_wf_init<false>, k_wf_resolve<false>};
   }
 };
 
@@ -616,9 +631,9 @@ struct Overlap {
 template <int SH>
 eos_status launch_sequence(cudaStream_t st, int num_sms, const WfArgs& base, const Chunk* chunks, int n_chunks,
                            int depth, int block, int grid_closest, int grid_any, int* ctr, size_t smem, size_t smem_a,
-                           bool small_stack, bool tree, StageTimer tm, const Overlap& ov, uint32_t& launches) {
+                           bool small_stack, bool tree, bool inst, StageTimer tm, const Overlap& ov, uint32_t& launches) {
   const int grid_lin = num_sms * 8;
-  const StageKernels<SH> K = StageKernels<SH>::get(small_stack, tree);
+  const StageKernels<SH> K = StageKernels<SH>::get(small_stack, tree, inst);
   const bool split = ov.side != nullptr && !tm.on;  // stage timing times the stages one by one
   cudaStream_t st2 = split ? ov.side : st, st3 = split ? ov.shade : st;
   for (int ci = 0; ci < n_chunks; ++ci) {
@@ -717,12 +732,13 @@ struct LaunchConfig {
   int block, sh, qchunk, grid_c, grid_a;
   bool small_stack;  // test limit: 8-entry traversal stacks (chain mode)
   bool tree;         // ray-tree mode
+  bool inst;         // some job's scene is a two-level one
   size_t smem, smem_a;  // stack columns of the nearest-hit (ref, distance) and shadow (ref) kernels
 };
 
 template <int SH>
 void configure(LaunchConfig& c, int num_sms) {
-  const StageKernels<SH> K = StageKernels<SH>::get(c.small_stack, c.tree);
+  const StageKernels<SH> K = StageKernels<SH>::get(c.small_stack, c.tree, c.inst);
   if (c.smem > 48 * 1024) {  // opt in to more than the default 48 KB of dynamic shared memory
     cudaFuncSetAttribute(K.closest_primary, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)c.smem);
     cudaFuncSetAttribute(K.closest, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)c.smem);
@@ -735,16 +751,17 @@ void configure(LaunchConfig& c, int num_sms) {
   c.grid_a = num_sms * std::max(1, occ_a);
 }
 
-LaunchConfig launch_config(const eos_render_params& p, int num_sms, bool small_stack, bool tree) {
+LaunchConfig launch_config(const eos_render_params& p, int num_sms, bool small_stack, bool tree, bool inst) {
   LaunchConfig c;
   c.block = p.block_size > 0 ? std::min(512, std::max(32, (p.block_size / 32) * 32)) : 128;
   c.sh = p.stack_depth <= 0 ? 16 : (p.stack_depth <= 8 ? 8 : (p.stack_depth <= 16 ? 16 : 32));
   c.qchunk = p.queue_chunk > 0 ? std::max(32, (p.queue_chunk / 32) * 32) : 64;
   c.tree = tree;
+  c.inst = inst;
   c.small_stack = small_stack && !tree;
   if (c.small_stack) c.sh = 8;
   c.smem = (size_t)c.sh * c.block * sizeof(uint2);
-  c.smem_a = (size_t)c.sh * c.block * sizeof(int);
+  c.smem_a = (size_t)any_entries(c.sh) * c.block * sizeof(int);
   if (c.sh == 8) configure<8>(c, num_sms);
   else if (c.sh == 16) configure<16>(c, num_sms);
   else configure<32>(c, num_sms);
@@ -755,12 +772,12 @@ eos_status run_sequence(cudaStream_t st, int num_sms, const LaunchConfig& lc, co
                         int n_chunks, int depth, StageTimer tm, const Overlap& ov, uint32_t& launches) {
   if (lc.sh == 8)
     return launch_sequence<8>(st, num_sms, A, chunks, n_chunks, depth, lc.block, lc.grid_c, lc.grid_a, A.ctr, lc.smem,
-                              lc.smem_a, lc.small_stack, lc.tree, tm, ov, launches);
+                              lc.smem_a, lc.small_stack, lc.tree, lc.inst, tm, ov, launches);
   if (lc.sh == 16)
     return launch_sequence<16>(st, num_sms, A, chunks, n_chunks, depth, lc.block, lc.grid_c, lc.grid_a, A.ctr,
-                               lc.smem, lc.smem_a, false, lc.tree, tm, ov, launches);
+                               lc.smem, lc.smem_a, false, lc.tree, lc.inst, tm, ov, launches);
   return launch_sequence<32>(st, num_sms, A, chunks, n_chunks, depth, lc.block, lc.grid_c, lc.grid_a, A.ctr, lc.smem,
-                             lc.smem_a, false, lc.tree, tm, ov, launches);
+                             lc.smem_a, false, lc.tree, lc.inst, tm, ov, launches);
 }
 
 }  // namespace
@@ -773,11 +790,12 @@ eos_status render_wavefront(eos_ctx* ctx, const eos_job* jobs, uint32_t n_jobs, 
   int depth = 0, max_lights = 0;
   std::vector<Chunk> chunks;
   const bool tree_records = (p.flags & EOS_FLAG_TREE_RECORDS) != 0;
-  bool tree = tree_records;
+  bool tree = tree_records, inst = false;
   for (uint32_t j = 0; j < n_jobs; ++j) {
     depth = std::max(depth, jobs[j].trace_depth);
     max_lights = std::max(max_lights, (int)jobs[j].scene->dev.n_lights);
     tree = tree || jobs[j].scene->branching;
+    inst = inst || jobs[j].scene->instanced;
   }
   // Per path: rays per bounce (1, or up to 2^depth in tree mode) x (two ray queues, two
   // sets of hit record, mask and shadow queue: Overlap) + accumulators (one per bounce, or
@@ -843,13 +861,13 @@ eos_status render_wavefront(eos_ctx* ctx, const eos_job* jobs, uint32_t n_jobs, 
   eos_status es = EOS_OK;
   DevJob* d_jobs = (DevJob*)scratch(ctx, "wf.jobs", sizeof(DevJob) * n_jobs, &es);
   const eos_limits& lim = ctx->limits;
-  const LaunchConfig lc = launch_config(p, ctx->num_sms, lim.small_stack != 0, tree);
+  const LaunchConfig lc = launch_config(p, ctx->num_sms, lim.small_stack != 0, tree, inst);
   const int block = lc.block, sh = lc.sh, qchunk = lc.qchunk;
 
   WfArgs A[kLanes];
   Overlap ov[kLanes];
   std::vector<long long> key = {(long long)n_jobs, depth, max_lights, block, sh, qchunk, (long long)lc.small_stack,
-                                (long long)lc.tree, n_lanes, (long long)(size_t)d_jobs};
+                                (long long)lc.tree, (long long)lc.inst, n_lanes, (long long)(size_t)d_jobs};
   for (int l = 0; l < n_lanes; ++l) {
     int max_chunk = 0;
     for (const Chunk& c : lane_chunks[l]) max_chunk = std::max(max_chunk, c.n);
@@ -1106,7 +1124,8 @@ extern "C" eos_status eos_render_noalloc(const eos_scene* scene, const eos_camer
   // the scene context's tuning table, as eos_render applies it (the table is read here
   // only; it is changed by eos_ctx_set_tuning calls, which callers serialise with renders)
   const LaunchConfig lc =
-      launch_config(with_tuning(scene->ctx, *params, (uint32_t)scene->dev.n_tris), num_sms, false, false);
+      launch_config(with_tuning(scene->ctx, *params, (uint32_t)scene->dev.n_tris), num_sms, false, false,
+                    scene->instanced);
   A.qchunk = lc.qchunk;
   A.work_limit = 0x7fffffff;
   A.init_in_primary = 1;
