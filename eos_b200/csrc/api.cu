@@ -44,6 +44,7 @@ eos_ctx::~eos_ctx() {
   for (cudaEvent_t e : ring_ev)
     if (e) cudaEventDestroy(e);
   if (d_counts) cudaFree(d_counts);
+  if (call_host) cudaFreeHost(call_host);
   if (ev0) cudaEventDestroy(ev0);
   if (ev1) cudaEventDestroy(ev1);
   if (pool) cudaMemPoolDestroy(pool);
@@ -183,9 +184,9 @@ eos_status begin_call(eos_ctx* ctx) {
 
 // Waits for the call, reads the error word (and counters into stats).
 eos_status end_call(eos_ctx* ctx, eos_stats* stats) {
-  CallWords h;
-  EOS_CUDA(cudaMemcpyAsync(&h, ctx->d_counts, sizeof h, cudaMemcpyDeviceToHost, ctx->stream));
+  EOS_CUDA(cudaMemcpyAsync(ctx->call_host, ctx->d_counts, sizeof(CallWords), cudaMemcpyDeviceToHost, ctx->stream));
   EOS_CUDA(cudaStreamSynchronize(ctx->stream));
+  const CallWords& h = *static_cast<const CallWords*>(ctx->call_host);
   if (stats) {
     stats->primary_rays = h.c[0];
     stats->shadow_rays = h.c[1];
@@ -362,6 +363,7 @@ eos_status eos_ctx_create(int32_t device, eos_ctx** out) {
     }
     if (cudaEventCreate(&ctx->ev0) != cudaSuccess || cudaEventCreate(&ctx->ev1) != cudaSuccess) { st = EOS_ERR_CUDA; break; }
     if (cudaMalloc(&ctx->d_counts, sizeof(CallWords)) != cudaSuccess) { st = EOS_ERR_OOM; break; }
+    if (cudaHostAlloc(&ctx->call_host, sizeof(CallWords), cudaHostAllocDefault) != cudaSuccess) { st = EOS_ERR_OOM; break; }
     cudaMemset(ctx->d_counts, 0, sizeof(CallWords));
     ctx->d_err = &reinterpret_cast<CallWords*>(ctx->d_counts)->err;
     ctx->d_work = &reinterpret_cast<CallWords*>(ctx->d_counts)->work;

@@ -114,6 +114,7 @@ struct eos_ctx {
   unsigned long long* d_counts = nullptr;
   int* d_err = nullptr;
   int* d_work = nullptr;
+  void* call_host = nullptr;  // pinned copy of them: the end of every call reads it
   std::map<std::string, eos::DevBuffer> scratch;
   cudaMemPool_t pool = nullptr;  // scene arrays and small scratch (pool_alloc)
   std::vector<float> bw_cams;  // cameras of the adjoint call in progress

@@ -38,3 +38,18 @@ def test_plain_equals_wavefront_at_every_lane_count(ctx, both, size):
         orc = oracle.Oracle(sc)
         o = (orc.render_tree if both else orc.render)(cam, td, pixel_offset=0.5)
         assert np.abs(a["rgb"].cpu().numpy() - o["rgb"]).max() <= 1e-4
+
+
+@pytest.mark.parametrize("n", [1, 5, 18_949, 37_901, 75_803])
+def test_queries_at_every_lane_count(ctx, n):
+    """Ray counts on both sides of the rule's steps, a last warp that is partly filled."""
+    d = scenes.instanced_test_scene(5, n_instances=16)
+    flat = scenes.small_random_scene(64, n_spheres=8, level=2)
+    rng = np.random.default_rng(n)
+    rays = np.concatenate([rng.uniform(-4, 4, (n, 3)), rng.normal(size=(n, 3))], 1).astype(np.float32)
+    inst = api.InstancedScene(ctx, [api.DeviceScene(ctx, m) for m in d.meshes], d.instances, d.materials, d.lights)
+    for scene, orc in ((api.DeviceScene(ctx, flat), oracle.Oracle(flat)), (inst, oracle.OracleInstanced(d))):
+        ids, t = api.trace_closest(ctx, scene, rays)
+        oid, ot, _ = orc.closest(rays)
+        assert np.array_equal(ids, oid) and np.array_equal(t[ids >= 0], ot[oid >= 0])
+        assert np.array_equal(api.trace_any(ctx, scene, rays), orc.any(rays))
