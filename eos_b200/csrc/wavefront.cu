@@ -194,6 +194,26 @@ __device__ __forceinline__ void emit_secondary(const WfArgs& A, int* ctr, bool w
   }
 }
 
+// The output pixel of path gp (its first sample): FP32 RGB and / or RGBA8.
+__device__ __forceinline__ void write_pixel(const DevJob& J, long long gp, f3 c) {
+  int x, y, smp;
+  path_pixel(J, gp - J.path_off, x, y, smp);
+  const size_t pix = (size_t)y * J.w + x;
+  if (J.rgb) {
+    J.rgb[3 * pix] = c.x;
+    J.rgb[3 * pix + 1] = c.y;
+    J.rgb[3 * pix + 2] = c.z;
+  }
+  if (J.rgba8)
+    reinterpret_cast<uchar4*>(J.rgba8)[pix] = make_uchar4(quantize(c.x), quantize(c.y), quantize(c.z), 255);
+}
+
+// The path's pixel is its colour: the stage where the path ends writes it, nothing reads the
+// path's accumulators afterwards, and slots that no stage has written are never read.
+__device__ __forceinline__ bool one_sample(const WfArgs& A, const DevJob& J) {
+  return A.init_in_primary && J.spp == 1 && J.grid == 0;
+}
+
 template <bool PRIMARY, int SH, int CAP, bool TREE, bool INST>
 __global__ void __launch_bounds__(256, INST ? 3 : 4) k_wf_closest(WfArgs A) {
   extern __shared__ uint2 shstack[];
@@ -252,6 +272,7 @@ __global__ void __launch_bounds__(256, INST ? 3 : 4) k_wf_closest(WfArgs A) {
         tests += h.tests;
         hit = h.pos >= 0;
         nhits += hit;
+        bool ended = false;
         if constexpr (TREE) {
           if (J.tree) {
             int x, y, smp;
@@ -299,18 +320,24 @@ __global__ void __launch_bounds__(256, INST ? 3 : 4) k_wf_closest(WfArgs A) {
             refl = refl && A.k < J.trace_depth;
           }
           float4* row = A.acc + (size_t)path * (A.depth + 1);
-          if (whole) {
+          ended = PRIMARY && !hit && one_sample(A, J);
+          if (whole && !one_sample(A, J)) {
             row[0] = make_float4(0, 0, 0, w);
             for (int k = 1; k <= A.depth; ++k) row[k] = make_float4(0, 0, 0, 0);
           } else if (hit) {
             reinterpret_cast<float*>(row + A.k)[3] = w;
           }
         }
-        HitQ hq;
-        hq.a = make_float4(P.x, P.y, P.z, TREE ? __uint_as_float(tree_pack(path, node)) : __int_as_float(path));
-        hq.b = make_float4(N.x, N.y, N.z, __int_as_float(hit ? (TREE || refl ? obj : obj | kEndsBit) : -1));
-        A.hits[i] = hq;
-        A.masks[i] = 0u;
+        if (ended) {  // a primary ray that leaves the scene: its pixel here, and a padding mark
+          write_pixel(J, A.c0 + path, mk3(0.0f, 0.0f, 0.0f));
+          A.hits[i].a = make_float4(0, 0, 0, __int_as_float(-1));
+        } else {
+          HitQ hq;
+          hq.a = make_float4(P.x, P.y, P.z, TREE ? __uint_as_float(tree_pack(path, node)) : __int_as_float(path));
+          hq.b = make_float4(N.x, N.y, N.z, __int_as_float(hit ? (TREE || refl ? obj : obj | kEndsBit) : -1));
+          A.hits[i] = hq;
+          A.masks[i] = 0u;
+        }
       }
       // shadow rays, compacted light-major inside the warp's block of the queue so that a
       // warp of the any-hit kernel mostly traces rays towards one light
@@ -387,20 +414,6 @@ __global__ void __maxnreg__(INST ? 96 : 56) k_wf_any(WfArgs A) {
   warp_add_count(&A.counts[kCntTestsA], tests);
 }
 
-// The output pixel of path gp (its first sample): FP32 RGB and / or RGBA8.
-__device__ __forceinline__ void write_pixel(const DevJob& J, long long gp, f3 c) {
-  int x, y, smp;
-  path_pixel(J, gp - J.path_off, x, y, smp);
-  const size_t pix = (size_t)y * J.w + x;
-  if (J.rgb) {
-    J.rgb[3 * pix] = c.x;
-    J.rgb[3 * pix + 1] = c.y;
-    J.rgb[3 * pix + 2] = c.z;
-  }
-  if (J.rgba8)
-    reinterpret_cast<uchar4*>(J.rgba8)[pix] = make_uchar4(quantize(c.x), quantize(c.y), quantize(c.z), 255);
-}
-
 template <bool TREE = false>
 __global__ void k_wf_shade(WfArgs A) {
   int* ctr = A.ctr + A.k * kCtr;
@@ -425,17 +438,20 @@ __global__ void k_wf_shade(WfArgs A) {
       if (obj >= 0) obj &= ~kEndsBit;
     }
     const DevJob& J = A.jobs[find_job(A.jobs, A.n_jobs, A.c0 + path)];
+    const bool writes = !TREE && ends && one_sample(A, J);  // the path's pixel, here
+    f3 acc = mk3(0, 0, 0), colour = acc;
     if (obj >= 0) {
       f3 P = mk3(hq.a.x, hq.a.y, hq.a.z), N = mk3(hq.b.x, hq.b.y, hq.b.z);
       f3 cam = mk3(J.cam[0], J.cam[1], J.cam[2]);
       const float* m = J.s.mats + kMatStride * obj;
       uint32_t mask = A.masks[i];
-      f3 acc = mk3(0, 0, 0);
       for (int l = 0; l < J.s.n_lights; ++l)
         if (!(mask & (1u << l))) acc = add3(acc, phong_light(m, J.s.lights + 6 * l, P, N, cam));
       // .w: the bounce weight (tree mode: the weight of the edge into the node), set by the hit stage
       float4* e = TREE ? A.acc + (size_t)path * A.nn + node : A.acc + (size_t)path * (A.depth + 1) + A.k;
-      *e = make_float4(acc.x, acc.y, acc.z, e->w);
+      const float w = e->w;
+      if (writes) colour = fold_colour(acc, w, colour);
+      else *e = make_float4(acc.x, acc.y, acc.z, w);
       if (J.paths || (TREE && J.tree)) {
         int x, y, smp;
         path_pixel(J, A.c0 + path - J.path_off, x, y, smp);
@@ -445,17 +461,15 @@ __global__ void k_wf_shade(WfArgs A) {
       }
     }
     if constexpr (!TREE) {
-      // the path's colour is final: slots beyond this bounce hold zeros, which the fold of
-      // k_wf_resolve passes through unchanged (0 + 0 * 0 = +0), so folding from here gives
-      // its colour bit for bit
-      if (ends && A.init_in_primary && J.spp == 1 && J.grid == 0) {
+      // slots beyond this bounce would fold to zero (0 + 0 * 0 = +0), so folding from here
+      // gives k_wf_resolve's colour bit for bit
+      if (writes) {
         const float4* a = A.acc + (size_t)path * (A.depth + 1);
-        f3 c = mk3(0, 0, 0);
-        for (int k = A.k; k >= 0; --k) {
+        for (int k = A.k - 1; k >= 0; --k) {
           const float4 e = a[k];
-          c = fold_colour(mk3(e.x, e.y, e.z), e.w, c);
+          colour = fold_colour(mk3(e.x, e.y, e.z), e.w, colour);
         }
-        write_pixel(J, A.c0 + path, c);
+        write_pixel(J, A.c0 + path, colour);
       }
     }
   }
@@ -525,7 +539,7 @@ __global__ void k_wf_resolve(WfArgs A) {
   for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < A.n_chunk; i += gridDim.x * blockDim.x) {
     long long gp = A.c0 + i;
     const DevJob& J = A.jobs[find_job(A.jobs, A.n_jobs, gp)];
-    if (!TREE && A.init_in_primary && J.spp == 1 && J.grid == 0) continue;  // written by k_wf_shade
+    if (!TREE && one_sample(A, J)) continue;  // written where the path ended
     int x, y, smp;
     if (!path_pixel(J, gp - J.path_off, x, y, smp) || smp != 0) continue;
     f3 sum = mk3(0, 0, 0);
