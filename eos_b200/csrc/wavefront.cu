@@ -18,7 +18,8 @@
 // rays of uneven cost balance across the SMs.  Paths are processed in chunks of at most
 // kChunkPathsMax, fewer when the queues of a chunk would exceed kQueueBudget bytes: one
 // large chunk keeps the persistent kernels' tails short (8.3M paths in one chunk ran the
-// config-2 batch 25 % faster than four chunks of 2M).  Bounce k's shadow and shading stages
+// config-2 batch 25 % faster than four chunks of 2M; a 30-job batch of 18M paths takes 4,490 us
+// in chunks of 2^24, whose rest of 1.3M paths pays every stage's tail again, 4,257 in one).  Bounce k's shadow and shading stages
 // run beside bounce k+1's nearest-hit stage (Overlap), and a large chunk runs as kLanes
 // parts side by side (render_wavefront), so that stages fill each other's tails.  The whole
 // sequence for a batch is captured once as a CUDA graph and replayed; the job table is
@@ -34,7 +35,8 @@
 namespace eos {
 namespace {
 
-constexpr long long kChunkPathsMax = 1ll << 24;
+constexpr long long kChunkPathsMax = 1ll << 25;
+constexpr long long kTreeChunkPathsMax = 1ll << 24;  // a ray-tree hit record packs path and node
 constexpr long long kQueueBudget = 16ll << 30;  // bytes of queues and accumulators per chunk
 constexpr long long kLaneSplitMin = 1ll << 20;  // paths of a chunk from which it runs as several lanes
 constexpr int kLanes = 2;                       // lanes of such a chunk (<= eos_ctx::kWfLanes)
@@ -818,7 +820,8 @@ eos_status render_wavefront(eos_ctx* ctx, const eos_job* jobs, uint32_t n_jobs, 
   const int nn = EOS_TREE_NODES(depth);
   const long long per_path =
       width * (2ll * 32 + 2 * (32 + 4 + 32ll * std::max(1, max_lights))) + 16ll * (tree ? nn : depth + 1);
-  const long long chunk_paths = std::max(1ll << 16, std::min(kChunkPathsMax, kQueueBudget / per_path));
+  const long long chunk_paths =
+      std::max(1ll << 16, std::min(tree ? kTreeChunkPathsMax : kChunkPathsMax, kQueueBudget / per_path));
   for (uint32_t j = 0; j < n_jobs; ++j) {
     DevJob& d = dj[j];
     fill_job(jobs[j], total, tree_records, (p.flags & EOS_FLAG_AA_GRID) != 0, d);
