@@ -41,8 +41,6 @@ eos_ctx::~eos_ctx() {
   if (own_stream) cudaStreamSynchronize(own_stream);
   if (pinned) cudaFreeHost(pinned);
   if (ring_host) cudaFreeHost(ring_host);
-  for (cudaEvent_t e : ring_ev)
-    if (e) cudaEventDestroy(e);
   if (d_counts) cudaFree(d_counts);
   if (call_host) cudaFreeHost(call_host);
   if (ev0) cudaEventDestroy(ev0);

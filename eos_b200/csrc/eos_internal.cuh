@@ -121,10 +121,10 @@ struct eos_ctx {
   void* pinned = nullptr;
   size_t pinned_bytes = 0;
   // read-back ring of the builders' launches that run ahead of the host (made on first use,
-  // ring.cuh): mapped pinned slots, and one event per slot
+  // ring.cuh): mapped pinned slots, and the number of the next launch
   int* ring_host = nullptr;
   int* ring_dev = nullptr;
-  cudaEvent_t ring_ev[4] = {};
+  long long ring_next = 0;
   // autotuner table: min triangle count -> tuned parameters
   std::map<uint32_t, eos_tuning> tuning;
   // test limits of the wavefront kernels (eos_ctx_set_limits); zeros = none

@@ -455,21 +455,22 @@ __global__ void k_wide_init(int* __restrict__ state, int root, int* __restrict__
 // write sequence took three and a read-back of the size.
 __global__ void __launch_bounds__(kScanBlock) k_wide_level(BinaryTree T, int* __restrict__ state,
                                                            int* __restrict__ state_out, int* __restrict__ slot,
-                                                           int level, unsigned long long* __restrict__ words,
+                                                           int number, int level, unsigned long long* __restrict__ words,
                                                            const int* __restrict__ frontier,
                                                            int* __restrict__ frontier_out, int max_children,
                                                            float4* __restrict__ wnodes, int max_nodes, int* err) {
   __shared__ int s_tile;
   __shared__ unsigned long long s_before;
+  ring_wait();
   const int n_in = state[0], base = state[1], n = T.n;
   const int n_tiles = (n_in + kScanBlock - 1) / kScanBlock;
   const int next_base = base + n_in;
   if (blockIdx.x == 0 && threadIdx.x == 0) {
     state_out[3] = 0;
     if (n_in == 0) {  // past the last level
-      state_out[0] = slot[0] = 0;
-      state_out[1] = slot[1] = next_base;
-      slot[3] = level;
+      state_out[0] = 0;
+      state_out[1] = next_base;
+      ring_publish(slot, 0, next_base, 0, number);
     }
   }
   for (;;) {
@@ -489,9 +490,9 @@ __global__ void __launch_bounds__(kScanBlock) k_wide_level(BinaryTree T, int* __
       if (threadIdx.x == 0) {
         s_before = before;
         if (tile == n_tiles - 1 && before <= kTileValue) {
-          state_out[0] = slot[0] = (int)before + total;
-          state_out[1] = slot[1] = next_base;
-          slot[3] = level;
+          state_out[0] = (int)before + total;
+          state_out[1] = next_base;
+          ring_publish(slot, (int)before + total, next_base, 0, number);
         }
       }
     }
@@ -574,7 +575,7 @@ eos_status write_records(eos_ctx* ctx, const BinaryTree& T, int root, int width,
   unsigned long long* words = (unsigned long long*)scratch(ctx, "lbvh.wide.words", words_bytes, &es);
   int* state = (int*)scratch(ctx, "lbvh.wide.state", 32, &es);
   if (es != EOS_OK) return es;
-  RoundRing ring(ctx, 2);  // as many launches run past the last level
+  RoundRing ring(ctx);
   if ((es = ring.init()) != EOS_OK) return es;
   EOS_CUDA(cudaMemsetAsync(words, 0, words_bytes, st));
   k_wide_init<<<1, 1, 0, st>>>(state, root, frontier[0]);
@@ -589,10 +590,10 @@ eos_status write_records(eos_ctx* ctx, const BinaryTree& T, int root, int width,
     }
     const int k = (int)(ring.issued & 1);
     const int grid = (int)std::min<long long>(scan_blocks(most), ctx->num_sms * 4);
-    k_wide_level<<<grid, kScanBlock, 0, st>>>(T, state + 4 * k, state + 4 * (k ^ 1), ring.next_slot(),
-                                              (int)ring.issued, words, frontier[k], frontier[k ^ 1], width, out,
-                                              max_nodes, ctx->d_err);
-    if ((es = ring.launched()) != EOS_OK) return es;
+    es = ring.launch(k_wide_level, grid, kScanBlock, T, state + 4 * k, state + 4 * (k ^ 1), ring.next_slot(),
+                     ring.next_number(), (int)ring.issued, words, frontier[k], frontier[k ^ 1], width, out, max_nodes,
+                     ctx->d_err);
+    if (es != EOS_OK) return es;
     most = std::min<long long>(most * width, T.n);
   }
   *n_records = std::min(s[1] + s[0], max_nodes);

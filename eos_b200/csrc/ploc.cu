@@ -93,8 +93,8 @@ __device__ __forceinline__ int forced_partner(int i, int nc) { return (i & 1) ? 
 // the finished tree: builds of 20k and 1.06M triangles 1,240 -> 580 and 2,200 -> 1,210 us,
 // node records included.
 __global__ void __launch_bounds__(kRoundThreads) k_ploc_round(
-    PlocTree T, int* __restrict__ state, int* __restrict__ state_out, int* __restrict__ slot, int round, int force,
-    unsigned long long* __restrict__ words, const int* __restrict__ cid, const float4* __restrict__ lo,
+    PlocTree T, int* __restrict__ state, int* __restrict__ state_out, int* __restrict__ slot, int number, int round,
+    int force, unsigned long long* __restrict__ words, const int* __restrict__ cid, const float4* __restrict__ lo,
     const float4* __restrict__ hi, int* __restrict__ cid_out, float4* __restrict__ lo_out, float4* __restrict__ hi_out,
     int* __restrict__ err) {
   constexpr int kBoxes = 2 * kRoundThreads + 2 * kRadius;
@@ -103,6 +103,7 @@ __global__ void __launch_bounds__(kRoundThreads) k_ploc_round(
   __shared__ int s_tile;
   __shared__ unsigned long long s_before;
   const int t = threadIdx.x;
+  ring_wait();
   if (t == 0) s_tile = atomicAdd(&state[3], 1);
   const int nc = state[0], node_base = state[1];
   __syncthreads();
@@ -164,10 +165,10 @@ __global__ void __launch_bounds__(kRoundThreads) k_ploc_round(
     if (t == 0 && tile == n_tiles - 1 && before <= kTileValue) {
       const unsigned long long all = before + sum;
       const int kept = (int)(all & 0x1ffffffu), made = (int)(all >> 25);
-      state_out[0] = slot[0] = kept;
-      state_out[1] = slot[1] = node_base + made;
-      state_out[2] = slot[2] = made;
-      slot[3] = round;
+      state_out[0] = kept;
+      state_out[1] = node_base + made;
+      state_out[2] = made;
+      ring_publish(slot, kept, node_base + made, made, number);
     }
   }
   __syncthreads();
@@ -385,7 +386,7 @@ eos_status build_ploc(eos_ctx* ctx, int n, int max_leaf, int sah, float4* blo, f
   // Rounds run ahead of the host until at most kTail clusters are left (k_ploc_tail does the
   // rest): grids are sized by an upper bound of the cluster count
   // (the last one read back; it only falls), and the host reads each round's state
-  // kAhead rounds later instead of waiting after every round.  A round that merges nothing
+  // RoundRing::kAhead rounds later instead of waiting after every round.  A round that merges nothing
   // changes nothing, so the rounds queued behind one repeat it harmlessly; when the host
   // sees it, it waits for the queue and runs the forced round (as a synchronous loop
   // would right away), so the tree is the same.
@@ -397,12 +398,12 @@ eos_status build_ploc(eos_ctx* ctx, int n, int max_leaf, int sah, float4* blo, f
   auto enqueue = [&](int force) {
     const int r = (int)ring.issued;
     // the first round's clusters are the leaf boxes themselves
-    k_ploc_round<<<grid_of(nc_ub, kRoundTile), kRoundThreads, 0, st>>>(
-        T, state + 4 * cur, state + 4 * (cur ^ 1), ring.next_slot(), r, force, words, r ? cid[cur] : nullptr,
-        r ? clo[cur] : blo + (n - 1), r ? chi[cur] : bhi + (n - 1), cid[cur ^ 1], clo[cur ^ 1], chi[cur ^ 1],
-        ctx->d_err);
+    const eos_status st_l = ring.launch(
+        k_ploc_round, grid_of(nc_ub, kRoundTile), kRoundThreads, T, state + 4 * cur, state + 4 * (cur ^ 1),
+        ring.next_slot(), ring.next_number(), r, force, words, r ? cid[cur] : nullptr, r ? clo[cur] : blo + (n - 1),
+        r ? chi[cur] : bhi + (n - 1), cid[cur ^ 1], clo[cur ^ 1], chi[cur ^ 1], ctx->d_err);
     cur ^= 1;
-    return ring.launched();
+    return st_l;
   };
   for (;;) {
     if (nc_ub > kTail && ring.full()) {  // read the oldest round in flight

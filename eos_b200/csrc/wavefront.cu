@@ -769,7 +769,7 @@ void configure(LaunchConfig& c, int num_sms) {
 
 LaunchConfig launch_config(const eos_render_params& p, int num_sms, bool small_stack, bool tree, bool inst) {
   LaunchConfig c;
-  c.block = p.block_size > 0 ? std::min(512, std::max(32, (p.block_size / 32) * 32)) : 128;
+  c.block = p.block_size > 0 ? std::min(512, std::max(32, (p.block_size / 32) * 32)) : 64;
   c.sh = p.stack_depth <= 0 ? 16 : (p.stack_depth <= 8 ? 8 : (p.stack_depth <= 16 ? 16 : 32));
   c.qchunk = p.queue_chunk > 0 ? std::max(32, (p.queue_chunk / 32) * 32) : 64;
   c.tree = tree;
