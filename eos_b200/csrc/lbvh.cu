@@ -384,14 +384,19 @@ __device__ __forceinline__ void write_record(float4* nodes, int n, const float (
 __device__ __forceinline__ int wide_select_one(int n, const int2* __restrict__ child, const float4* __restrict__ blo,
                                                const float4* __restrict__ bhi, int node, int max_children, int* c,
                                                float4* lo, float4* hi) {
-  int2 ch = child[node];
-  c[0] = ch.x;
-  c[1] = ch.y;
+  // a child's own children are read along with its box, before it is known whether it is
+  // opened: one dependent read per opening instead of two
+  int2 sub[4];
+  auto take = [&](int i, int ci) {
+    c[i] = ci;
+    lo[i] = blo[ci];
+    hi[i] = bhi[ci];
+    sub[i] = ci < n - 1 ? child[ci] : make_int2(-1, -1);
+  };
+  const int2 ch = child[node];
+  take(0, ch.x);
+  take(1, ch.y);
   c[2] = c[3] = -1;
-  for (int i = 0; i < 2; ++i) {
-    lo[i] = blo[c[i]];
-    hi[i] = bhi[c[i]];
-  }
 #pragma unroll
   for (int k = 2; k < 4; ++k) {
     if (k >= max_children) break;
@@ -407,17 +412,14 @@ __device__ __forceinline__ int wide_select_one(int n, const int2* __restrict__ c
       }
     }
     if (best < 0) break;
+    int2 g = make_int2(0, 0);
 #pragma unroll
     for (int i = 0; i < k; ++i)
-      if (i == best) {
-        ch = child[c[i]];
-        c[i] = ch.x;
-        lo[i] = blo[ch.x];
-        hi[i] = bhi[ch.x];
-      }
-    c[k] = ch.y;
-    lo[k] = blo[ch.y];
-    hi[k] = bhi[ch.y];
+      if (i == best) g = sub[i];
+#pragma unroll
+    for (int i = 0; i < k; ++i)
+      if (i == best) take(i, g.x);
+    take(k, g.y);
   }
   int m = 0;
 #pragma unroll

@@ -27,10 +27,9 @@ namespace eos {
 namespace {
 
 constexpr int kRadius = 16;        // neighbours searched on each side
-// Clusters of one block's tile: two per thread over the tile and kRadius more on each side,
+// Clusters of one block's tile: one per thread over the tile and kRadius more on each side,
 // whose nearest neighbours decide which pairs at the tile's ends are mutual.
-constexpr int kRoundThreads = 256;
-constexpr int kRoundTile = 2 * kRoundThreads - 2 * kRadius;
+constexpr int round_tile(int threads) { return threads - 2 * kRadius; }
 constexpr int kTail = 1024;  // clusters at or below which one block runs the remaining rounds
 constexpr int kMaxWalk = 4 * kStackMax;  // bound of the walks to the root
 
@@ -84,22 +83,24 @@ __device__ __forceinline__ void make_node(const PlocTree& T, int k, int a, int b
 // of iterations.
 __device__ __forceinline__ int forced_partner(int i, int nc) { return (i & 1) ? i - 1 : (i + 1 < nc ? i + 1 : -1); }
 
-// One iteration.  Bound by latency and launches for most rounds (their cluster counts fall by
-// about a fifth each), by the neighbour search for the first: a thread searches for two
-// neighbouring clusters, so a box read from shared memory serves both (boxes of even and
-// odd index lie apart, which keeps the reads free of bank conflicts).  Places outside the
-// clusters hold an infinite box, whose merged area is never below the best.  Measured against
-// four launches an iteration (search, flags, scan of the block sums, merge) and a refit of
-// the finished tree: builds of 20k and 1.06M triangles 1,240 -> 580 and 2,200 -> 1,210 us,
-// node records included.
+// One iteration.  Bound by its serial chain and launches for most rounds (their cluster
+// counts fall by about a fifth each), by the neighbour search for the first: threads 2u and
+// 2u + 1 search for clusters 2u and 2u + 1 together, one over the boxes of even index, the other
+// over the odd ones, so a box read from shared memory serves both clusters and the search is
+// half as long (even and odd boxes lie apart, 64 bytes off in the banks: no conflicts).
+// Places outside the clusters hold an infinite box, whose merged area is never below the
+// best.  Measured against four launches an iteration (search, flags, scan of the block sums,
+// merge) and a refit of the finished tree: builds of 20k and 1.06M triangles 1,240 -> 580 and
+// 2,200 -> 1,210 us, node records included, with one thread searching for two clusters.
+template <int kRoundThreads>
 __global__ void __launch_bounds__(kRoundThreads) k_ploc_round(
     PlocTree T, int* __restrict__ state, int* __restrict__ state_out, int* __restrict__ slot, int number, int round,
     int force, unsigned long long* __restrict__ words, const int* __restrict__ cid, const float4* __restrict__ lo,
     const float4* __restrict__ hi, int* __restrict__ cid_out, float4* __restrict__ lo_out, float4* __restrict__ hi_out,
     int* __restrict__ err) {
-  constexpr int kBoxes = 2 * kRoundThreads + 2 * kRadius;
-  __shared__ float4 slo[2][kBoxes / 2], shi[2][kBoxes / 2];
-  __shared__ int sid[kBoxes], snn[2 * kRoundThreads];
+  constexpr int kBoxes = kRoundThreads + 2 * kRadius, kRoundTile = round_tile(kRoundThreads);
+  __shared__ float4 slo[2][kBoxes / 2 + 4], shi[2][kBoxes / 2 + 4];
+  __shared__ int sid[kBoxes], snn[kRoundThreads];
   __shared__ int s_tile;
   __shared__ unsigned long long s_before;
   const int t = threadIdx.x;
@@ -119,44 +120,42 @@ __global__ void __launch_bounds__(kRoundThreads) k_ploc_round(
     sid[e] = !in ? 0 : cid ? cid[g] : T.n - 1 + g;
   }
   __syncthreads();
-  const int i0 = base - kRadius + 2 * t;  // this thread's clusters: i0 and i0 + 1
-  constexpr int kMid = kRadius / 2;       // their boxes: slots t + kMid, even and odd
-  int p0 = -1, p1 = -1;                   // their partners
+  const int i = base - kRadius + t;  // this thread's cluster
+  const bool own = t >= kRadius && t < kRoundThreads - kRadius && i < nc;
+  int p = -1;  // its partner
   if (!force) {
-    const float4 al = slo[0][t + kMid], ah = shi[0][t + kMid], bl = slo[1][t + kMid], bh = shi[1][t + kMid];
+    constexpr int kMid = kRadius / 2;
+    const int u = t >> 1, h = t & 1;
+    const int i0 = base - kRadius + 2 * u;  // the pair's even cluster; box m is i0 - kRadius + 2 m + h
+    const float4 al = slo[0][u + kMid], ah = shi[0][u + kMid], bl = slo[1][u + kMid], bh = shi[1][u + kMid];
     float best0 = kInf, best1 = kInf;
-    int j0 = i0 == 0 ? 1 : i0 - 1, j1 = i0;
+    int m0 = 0, m1 = 0;
+    const int skip0 = h ? kRadius : kMid, skip1 = h ? kMid : 0;  // beyond kRadius, or the cluster itself
 #pragma unroll 1
     for (int m = 0; m <= kRadius; ++m) {
-      const int g = i0 - kRadius + 2 * m;  // even box, then its odd neighbour
-      const float4 el = slo[0][t + m], eh = shi[0][t + m], ol = slo[1][t + m], oh = shi[1][t + m];
-      const float e0 = merged_area(al, ah, el, eh), o0 = merged_area(al, ah, ol, oh);
-      const float e1 = merged_area(bl, bh, el, eh), o1 = merged_area(bl, bh, ol, oh);
-      if (m != kMid && e0 < best0) { best0 = e0; j0 = g; }
-      if (m != kRadius && o0 < best0) { best0 = o0; j0 = g + 1; }
-      if (m != 0 && e1 < best1) { best1 = e1; j1 = g; }
-      if (m != kMid && o1 < best1) { best1 = o1; j1 = g + 1; }
+      const float4 cl = slo[h][u + m], ch = shi[h][u + m];
+      const float a0 = merged_area(al, ah, cl, ch), a1 = merged_area(bl, bh, cl, ch);
+      if (m != skip0 && a0 < best0) { best0 = a0; m0 = m; }
+      if (m != skip1 && a1 < best1) { best1 = a1; m1 = m; }
     }
-    snn[2 * t] = j0;
-    snn[2 * t + 1] = j1;
+    // the least (area, index) of the two threads
+    int j0 = i0 - kRadius + 2 * m0 + h, j1 = i0 - kRadius + 2 * m1 + h;
+    const float o0 = __shfl_xor_sync(0xffffffffu, best0, 1), o1 = __shfl_xor_sync(0xffffffffu, best1, 1);
+    const int k0 = __shfl_xor_sync(0xffffffffu, j0, 1), k1 = __shfl_xor_sync(0xffffffffu, j1, 1);
+    if (o0 < best0 || (o0 == best0 && k0 < j0)) { best0 = o0; j0 = k0; }
+    if (o1 < best1 || (o1 == best1 && k1 < j1)) { best1 = o1; j1 = k1; }
+    int j = h ? j1 : j0;
+    if (!((h ? best1 : best0) < kInf)) j = i == 0 ? 1 : i - 1;
+    snn[t] = j;
     __syncthreads();
     // mutual?  (a neighbour of a cluster of the tile lies within the searched ones)
-    const int off = base - kRadius;
-    const bool own = t >= kRadius / 2 && t < kRoundThreads - kRadius / 2;
-    if (own && i0 < nc && j0 < nc && snn[j0 - off] == i0) p0 = j0;
-    if (own && i0 + 1 < nc && j1 < nc && snn[j1 - off] == i0 + 1) p1 = j1;
-  } else if (i0 >= 0) {
-    p0 = forced_partner(i0, nc);
-    p1 = forced_partner(i0 + 1, nc);
+    if (own && j < nc && snn[j - (base - kRadius)] == i) p = j;
+  } else if (own) {
+    p = forced_partner(i, nc);
   }
-  // kept clusters (low half) and made nodes (high half) of this thread's two
-  const bool own = t >= kRadius / 2 && t < kRoundThreads - kRadius / 2;
-  const bool v0 = own && i0 < nc, v1 = own && i0 + 1 < nc;
-  const int keep0 = v0 && (p0 < 0 || i0 < p0), keep1 = v1 && (p1 < 0 || i0 + 1 < p1);
-  const int make0 = keep0 && p0 >= 0, make1 = keep1 && p1 >= 0;
-  int total;
-  const int mine = (keep0 + keep1) | ((make0 + make1) << 16);
-  const int ex = block_exclusive_scan(mine, total);
+  const bool keep = own && (p < 0 || i < p), make = keep && p >= 0;
+  int total;  // kept clusters (low half) and made nodes (high half)
+  const int ex = block_exclusive_scan((int)keep | ((int)make << 16), total);
   if (t < 32) {
     const unsigned long long sum = (unsigned)(total & 0xffff) | ((unsigned long long)(total >> 16) << 25);
     const unsigned long long before = tiles_before(words, tile, sum, (unsigned)(round % 4095 + 1));
@@ -176,30 +175,25 @@ __global__ void __launch_bounds__(kRoundThreads) k_ploc_round(
     if (t == 0) atomicOr(err, kErrTimeout);
     return;
   }
-  int pos = (int)(s_before & 0x1ffffffu) + (ex & 0xffff);
-  int k = node_base + (int)(s_before >> 25) + (ex >> 16);
-#pragma unroll
-  for (int c = 0; c < 2; ++c) {
-    const int i = i0 + c, p = c ? p1 : p0;
-    if (!(c ? keep1 : keep0)) continue;
-    const int e = i - base + 2 * kRadius;
-    const float4 al = slo[e & 1][e >> 1], ah = shi[e & 1][e >> 1];
-    int id = sid[e], cnt = cluster_count(cid, ah);
-    float4 ol = al, oh = ah;
-    if (p >= 0) {
-      const int f = p - base + 2 * kRadius;
-      const float4 bl = slo[f & 1][f >> 1], bh = shi[f & 1][f >> 1];
-      const int cb = cluster_count(cid, bh);
-      if (k < T.n - 1)  // always: n leaves make n - 1 nodes
-        make_node(T, k, id, sid[f], cnt, cb, al, ah, bl, bh, ol, oh);
-      id = k++;
-      cnt += cb;
-    }
-    cid_out[pos] = id;
-    lo_out[pos] = ol;
-    hi_out[pos] = make_float4(oh.x, oh.y, oh.z, __int_as_float(cnt));
-    ++pos;
+  if (!keep) return;
+  const int pos = (int)(s_before & 0x1ffffffu) + (ex & 0xffff);
+  const int k = node_base + (int)(s_before >> 25) + (ex >> 16);
+  const int e = t + kRadius;
+  const float4 al = slo[e & 1][e >> 1], ah = shi[e & 1][e >> 1];
+  int id = sid[e], cnt = cluster_count(cid, ah);
+  float4 ol = al, oh = ah;
+  if (make) {
+    const int f = p - base + 2 * kRadius;
+    const float4 bl = slo[f & 1][f >> 1], bh = shi[f & 1][f >> 1];
+    const int cb = cluster_count(cid, bh);
+    if (k < T.n - 1)  // always: n leaves make n - 1 nodes
+      make_node(T, k, id, sid[f], cnt, cb, al, ah, bl, bh, ol, oh);
+    id = k;
+    cnt += cb;
   }
+  cid_out[pos] = id;
+  lo_out[pos] = ol;
+  hi_out[pos] = make_float4(oh.x, oh.y, oh.z, __int_as_float(cnt));
 }
 
 // The rounds left once at most kTail clusters remain, in one block with the clusters in
@@ -245,71 +239,81 @@ __global__ void __launch_bounds__(kTail) k_ploc_tail(PlocTree T, int* __restrict
       break;
     }
     if (!force) {
-      // 2^lg threads per cluster, each 32 / 2^lg of the neighbours; the least (area, index)
-      const int lg = nc > 512 ? 0 : nc > 256 ? 1 : nc > 128 ? 2 : nc > 64 ? 3 : nc > 32 ? 4 : 5;
-      const int c = i >> lg, g = i & ((1 << lg) - 1), per = (2 * kRadius) >> lg;
-      float best = kInf;
-      int bj = kTail;
-      if (c < nc) {
-        const float4 al = slo[c], ah = shi[c];
-        const int j0 = c - kRadius + g * per;
+      // 2^lg threads per cluster, each every 2^lg-th of its 32 neighbours (the threads of a warp
+      // read neighbouring boxes: no bank conflicts); the least (area, index)
+      const int lg = nc > 512 ? 0 : nc > 256 ? 1 : nc > 128 ? 2 : nc > 48 ? 3 : nc > 16 ? 4 : 5;
+      const int c = i >> lg, g = i & ((1 << lg) - 1);
+      if ((i & ~31) >> lg < nc) {  // warps without a cluster wait
+        float best = kInf;
+        int bj = kTail;
+        const float4 al = slo[c], ah = shi[c];  // c past nc in the last warp: an infinite box
 #pragma unroll 4
-        for (int w = 0; w < per; ++w) {
-          const int j = j0 + w + (g * per + w >= kRadius);  // all places but c
+        for (int w = g; w < 2 * kRadius; w += 1 << lg) {
+          const int j = c - kRadius + w + (w >= kRadius);  // all places but c
           const float a = merged_area(al, ah, slo[j], shi[j]);
           if (a < best) {
             best = a;
             bj = j;
           }
         }
+        for (int off = 1; off < (1 << lg); off <<= 1) {
+          const float o = __shfl_xor_sync(0xffffffffu, best, off);
+          const int oj = __shfl_xor_sync(0xffffffffu, bj, off);
+          if (o < best || (o == best && oj < bj)) {
+            best = o;
+            bj = oj;
+          }
+        }
+        if (c < nc && g == 0) snn[c] = best < kInf ? bj : (c == 0 ? 1 : c - 1);
       }
-      for (int off = 1; off < (1 << lg); off <<= 1) {
-        const float o = __shfl_xor_sync(0xffffffffu, best, off);
-        const int oj = __shfl_xor_sync(0xffffffffu, bj, off);
-        if (o < best || (o == best && oj < bj)) {
-          best = o;
-          bj = oj;
+    }
+    __syncthreads();
+    const bool works = warp * 32 < nc;  // warps with clusters: the others only wait
+    const int n_warps = (nc + 31) >> 5;
+    const uint32_t lt = (1u << lane) - 1u;
+    int partner = -1;
+    bool keep = false, make = false;
+    uint32_t kb = 0, mb = 0;
+    if (works) {
+      if (i < nc) {
+        if (force) {
+          partner = forced_partner(i, nc);
+        } else {
+          const int j = snn[i];
+          partner = j < nc && snn[j] == i ? j : -1;
         }
       }
-      if (c < nc && g == 0) snn[c] = best < kInf ? bj : (c == 0 ? 1 : c - 1);
+      keep = i < nc && (partner < 0 || i < partner);
+      make = keep && partner >= 0;
+      kb = __ballot_sync(0xffffffffu, keep);
+      mb = __ballot_sync(0xffffffffu, make);
+      if (lane == 0) wsum[warp] = __popc(kb) | (__popc(mb) << 16);
     }
     __syncthreads();
-    int partner = -1;
-    if (i < nc) {
-      if (force) {
-        partner = forced_partner(i, nc);
-      } else {
-        const int j = snn[i];
-        partner = j < nc && snn[j] == i ? j : -1;
+    unsigned total = 0;
+    for (int w = lane; w < n_warps; w += 32) total = wsum[w];
+    int pos = 0, id = 0, cnt = 0;
+    float4 ol = out_lo, oh = out_hi;
+    if (works) {
+      const unsigned before = __reduce_add_sync(0xffffffffu, lane < warp ? total : 0u);
+      pos = (int)(before & 0xffff) + __popc(kb & lt);
+      if (keep) {
+        id = scid[i];
+        cnt = scount[i];
+        ol = slo[i];
+        oh = shi[i];
+        if (make) {
+          const int k = node_base + (int)(before >> 16) + __popc(mb & lt);
+          const float4 al = ol, ah = oh;
+          const int cb = scount[partner];
+          if (k < T.n - 1)  // always: n leaves make n - 1 nodes
+            make_node(T, k, id, scid[partner], cnt, cb, al, ah, slo[partner], shi[partner], ol, oh);
+          id = k;
+          cnt += cb;
+        }
       }
     }
-    const bool keep = i < nc && (partner < 0 || i < partner);
-    const bool make = keep && partner >= 0;
-    const uint32_t kb = __ballot_sync(0xffffffffu, keep), mb = __ballot_sync(0xffffffffu, make);
-    if (lane == 0) wsum[warp] = __popc(kb) | (__popc(mb) << 16);
-    __syncthreads();
-    const unsigned w = wsum[lane];
-    const unsigned before = __reduce_add_sync(0xffffffffu, lane < warp ? w : 0u);
-    const unsigned total = __reduce_add_sync(0xffffffffu, w);
-    const uint32_t lt = (1u << lane) - 1u;
-    const int pos = (int)(before & 0xffff) + __popc(kb & lt);
-    int id = 0, cnt = 0;
-    float4 ol = make_float4(0.0f, 0.0f, 0.0f, 0.0f), oh = ol;
-    if (keep) {
-      id = scid[i];
-      cnt = scount[i];
-      ol = slo[i];
-      oh = shi[i];
-      if (make) {
-        const int k = node_base + (int)(before >> 16) + __popc(mb & lt);
-        const float4 al = ol, ah = oh;
-        const int cb = scount[partner];
-        if (k < T.n - 1)  // always: n leaves make n - 1 nodes
-          make_node(T, k, id, scid[partner], cnt, cb, al, ah, slo[partner], shi[partner], ol, oh);
-        id = k;
-        cnt += cb;
-      }
-    }
+    total = __reduce_add_sync(0xffffffffu, total);
     __syncthreads();  // every read of this round's clusters is done
     if (keep) {
       scid[pos] = id;
@@ -376,7 +380,10 @@ eos_status build_ploc(eos_ctx* ctx, int n, int max_leaf, int sah, float4* blo, f
   int* cid[2] = {(int*)scratch(ctx, "ploc.cid0", 4 * nn, &es), (int*)scratch(ctx, "ploc.cid1", 4 * nn, &es)};
   float4* clo[2] = {(float4*)scratch(ctx, "ploc.lo0", 16 * nn, &es), (float4*)scratch(ctx, "ploc.lo1", 16 * nn, &es)};
   float4* chi[2] = {(float4*)scratch(ctx, "ploc.hi0", 16 * nn, &es), (float4*)scratch(ctx, "ploc.hi1", 16 * nn, &es)};
-  const size_t words_bytes = 8 * (size_t)grid_of(n, kRoundTile);
+  // Blocks of 512 threads, and of 256 once those are fewer than the SMs: the search is then a
+  // shorter part of the round on more of them.
+  const int small_max = round_tile(256) * ctx->num_sms;
+  const size_t words_bytes = 8 * (size_t)std::max(grid_of(n, round_tile(512)), ctx->num_sms);
   unsigned long long* words = (unsigned long long*)scratch(ctx, "ploc.words", words_bytes, &es);
   int2* up = (int2*)scratch(ctx, "ploc.up", 8 * (2 * nn), &es);
   int* state = (int*)scratch(ctx, "ploc.state", 64, &es);  // two states, by round parity, and the depth
@@ -395,13 +402,20 @@ eos_status build_ploc(eos_ctx* ctx, int n, int max_leaf, int sah, float4* blo, f
   EOS_CUDA(cudaMemsetAsync(words, 0, words_bytes, st));
   k_ploc_state_init<<<1, 1, 0, st>>>(state, n, dmax);
   int nc_ub = n, cur = 0;
+  bool small = nc_ub <= small_max;
   auto enqueue = [&](int force) {
     const int r = (int)ring.issued;
+    if (!small && nc_ub <= small_max) {  // other tiles from here on
+      small = true;
+      EOS_CUDA(cudaMemsetAsync(words, 0, words_bytes, st));
+    }
+    const int threads = small ? 256 : 512;
     // the first round's clusters are the leaf boxes themselves
     const eos_status st_l = ring.launch(
-        k_ploc_round, grid_of(nc_ub, kRoundTile), kRoundThreads, T, state + 4 * cur, state + 4 * (cur ^ 1),
-        ring.next_slot(), ring.next_number(), r, force, words, r ? cid[cur] : nullptr, r ? clo[cur] : blo + (n - 1),
-        r ? chi[cur] : bhi + (n - 1), cid[cur ^ 1], clo[cur ^ 1], chi[cur ^ 1], ctx->d_err);
+        small ? k_ploc_round<256> : k_ploc_round<512>, grid_of(nc_ub, round_tile(threads)), threads, T,
+        state + 4 * cur, state + 4 * (cur ^ 1), ring.next_slot(), ring.next_number(), r, force, words,
+        r ? cid[cur] : nullptr, r ? clo[cur] : blo + (n - 1), r ? chi[cur] : bhi + (n - 1), cid[cur ^ 1],
+        clo[cur ^ 1], chi[cur ^ 1], ctx->d_err);
     cur ^= 1;
     return st_l;
   };
