@@ -42,7 +42,7 @@ struct ShadedHit {
   uint32_t mask;
 };
 
-template <int SH>
+template <int SH, TraversalForm F>
 __device__ __forceinline__ ShadedHit shade_hit(const PlainParams& P, f3 o, f3 d, const Hit& h, unsigned* cnt,
                                                uint32_t col, uint32_t stride) {
   const DevScene& s = P.s;
@@ -58,7 +58,7 @@ __device__ __forceinline__ ShadedHit shade_hit(const PlainParams& P, f3 o, f3 d,
     f3 sd = norm3(sub3(mk3(l[0], l[1], l[2]), r.P));
     f3 so = add3(r.P, scale3(kRayEps, sd));
     cnt[kCntShadow]++;
-    AnyResult ar = any_hit<SH>(s, so, sd, col, stride, P.err);
+    AnyResult ar = any_hit<SH, F>(s, so, sd, col, stride, P.err);
     cnt[kCntNodesA] += ar.nodes;
     cnt[kCntTestsA] += ar.tests;
     if (ar.hit) r.mask |= 1u << li;
@@ -69,7 +69,7 @@ __device__ __forceinline__ ShadedHit shade_hit(const PlainParams& P, f3 o, f3 d,
 
 // A path of one secondary ray per hit, traced a ray at a time: begin, then step until it
 // returns true; colour with the reference's fold c_k = phong_k + w_k c_{k+1} (fold_colour).
-template <int SH>
+template <int SH, TraversalForm F>
 struct ChainPath {
   f3 o, d;
   int k;  // bounce of the ray
@@ -90,14 +90,14 @@ struct ChainPath {
                                        uint32_t stride) {
     const DevScene& s = P.s;
     cnt[k == 0 ? kCntPrimary : kCntSecondary]++;
-    Hit h = closest_hit<SH>(s, o, d, col, stride, P.err);
+    Hit h = closest_hit<SH, F>(s, o, d, col, stride, P.err);
     cnt[kCntNodesC] += h.nodes;
     cnt[kCntTestsC] += h.tests;
     int nb = k;
     hits[k] = h.pos < 0 ? EOS_HIT_NONE : h.id;
     if (h.pos >= 0) {
       cnt[kCntHits]++;
-      const ShadedHit r = shade_hit<SH>(P, o, d, h, cnt, col, stride);
+      const ShadedHit r = shade_hit<SH, F>(P, o, d, h, cnt, col, stride);
       masks[k] = r.mask;
       phong[k] = r.phong;
       nb = k + 1;
@@ -145,7 +145,7 @@ struct TreeFrame {
 // lane without a tree takes the transparent child of a waiting node from another lane of
 // its warp (share): the subtree nearest the root first, whose colour goes back to the
 // owner's frame, which sums it in its place, with the same operations.
-template <int SH>
+template <int SH, TraversalForm F>
 struct TreePath {
   f3 o, d;
   int sp, node, depth;
@@ -175,7 +175,7 @@ struct TreePath {
     const f3 zero = mk3(0.0f, 0.0f, 0.0f);
     c = zero;
     cnt[depth == 0 ? kCntPrimary : kCntSecondary]++;
-    Hit h = closest_hit<SH>(s, o, d, col, stride, P.err);
+    Hit h = closest_hit<SH, F>(s, o, d, col, stride, P.err);
     cnt[kCntNodesC] += h.nodes;
     cnt[kCntTestsC] += h.tests;
     const int id = h.pos < 0 ? EOS_HIT_NONE : h.id;
@@ -184,7 +184,7 @@ struct TreePath {
     if (rec) rec->hit = id;
     if (h.pos >= 0) {
       cnt[kCntHits]++;
-      const ShadedHit r = shade_hit<SH>(P, o, d, h, cnt, col, stride);
+      const ShadedHit r = shade_hit<SH, F>(P, o, d, h, cnt, col, stride);
       if (rec) rec->shadow = r.mask;
       TreeFrame F;
       F.phong = r.phong;
@@ -260,8 +260,8 @@ struct TreePath {
 
 // The `idle` lanes take open subtrees of the warp's other lanes, with the owner's pixel (x, ly,
 // smp).  Warp-uniform.
-template <int SH>
-__device__ __forceinline__ void share_trees(TreePath<SH>& t, uint32_t idle, bool& active, bool& fresh, int& x, int& ly,
+template <class Path>
+__device__ __forceinline__ void share_trees(Path& t, uint32_t idle, bool& active, bool& fresh, int& x, int& ly,
                                             int& smp) {
   const int lane = threadIdx.x & 31;
   uint32_t open = __ballot_sync(0xffffffffu, active && t.open != 0);
@@ -306,8 +306,8 @@ __device__ __forceinline__ void share_trees(TreePath<SH>& t, uint32_t idle, bool
 }
 
 // Colours of the subtrees that lanes of `done` have finished go to their owners.  Warp-uniform.
-template <int SH>
-__device__ __forceinline__ void return_trees(TreePath<SH>& t, uint32_t done, f3 c) {
+template <class Path>
+__device__ __forceinline__ void return_trees(Path& t, uint32_t done, f3 c) {
   const int lane = threadIdx.x & 31;
   while (done) {
     const int from = __ffs(done) - 1;
@@ -321,17 +321,19 @@ __device__ __forceinline__ void return_trees(TreePath<SH>& t, uint32_t done, f3 
   }
 }
 
-// Registers capped at 64 (32 warps per SM with blocks of 128): the megakernel is latency-
-// bound and gains more from resident warps than it loses to spills (measured on config 2:
-// 112 registers 2,580 Mrays/s, 96 2,794, 80 2,913, 64 3,076, 56 2,987, 48 2,481).
-template <int SH, bool TREE = false>
-__global__ void __maxnreg__(64) k_render_plain(PlainParams P) {
+// The traversals are inline, for flat scenes without the two-level one (TraversalForm), and the
+// registers capped where resident warps and spills balance.  Measured, us for a 1080p frame of
+// 200k triangles and a 961x541 frame of ray trees: out of line at 64 registers 867 and 2,050;
+// inline at 56 854 and 1,917, 64 816 and 1,896, 72 807 and 1,769, 80 817 and 1,765, 88 842 and
+// 1,753.  1080p of 801 instances: out of line at 64 13.2 ms; inline at 64 12.1, 80 11.6, 96 12.0.
+template <int SH, bool TREE, TraversalForm F>
+__global__ void __maxnreg__(F == kTwoLevel ? 80 : TREE ? 88 : 72) k_render_plain(PlainParams P) {
   extern __shared__ uint2 shstack[];
   const uint32_t col = shared_address(shstack + threadIdx.x), stride = 8 * blockDim.x;
   unsigned cnt[kNumCounts] = {0, 0, 0, 0, 0, 0, 0, 0};
   const int lane = threadIdx.x & 31;
   const int tiles_x = (P.width + 7) >> 3;
-  typename std::conditional<TREE, TreePath<SH>, ChainPath<SH>>::type path;
+  typename std::conditional<TREE, TreePath<SH, F>, ChainPath<SH, F>>::type path;
   bool active = false, fresh = false;  // a pixel in hand; its next sample not begun
   bool more = lane < P.lanes;          // may take another pixel
   int x = 0, ly = 0, smp = 0;
@@ -466,39 +468,40 @@ namespace {
 // Lanes of a warp that trace.  A frame of few pixels is bound by the time of its slowest
 // warp, which walks the union of its lanes' nodes, while most of the chip idles: with fewer
 // lanes a warp the same pixels spread over more warps.  Chains: the fewest lanes that leave
-// every warp resident (32 warps of 64 registers per SM).  Measured, us at 32 / 16 / 8 / 4 lanes:
+// every warp resident (28 warps of 72 registers per SM).  Measured, us at 32 / 16 / 8 / 4 lanes:
 // 64x64 of 200k triangles 243 / 219 / 207 / 166, 128x128 271 / 251 / 213 / 197, 256x256 284 /
 // 278 / 282, 512x512 405 / 448 / 569.  Ray trees have longer tails (a pixel's tree is walked by
 // a warp): 8 lanes up to four such fillings (400x300: 1,588 / 1,732 / 1,458), 16 up to eight
 // (961x541: 2,113 / 1,881 / 2,201; 1920x1080: 3,033 / 3,551).
 int lanes_of(uint32_t n_work, int num_sms, bool tree) {
-  const uint32_t full = 32u * (uint32_t)num_sms;  // warps that fill the chip
+  const uint32_t full = 28u * (uint32_t)num_sms;  // warps that fill the chip
   if (tree) return n_work / 8 <= 4 * full ? 8 : n_work / 16 <= 8 * full ? 16 : 32;
   for (int lanes = 4; lanes < 32; lanes *= 2)
     if (n_work / lanes <= full) return lanes;
   return 32;
 }
 
-template <int SH, bool TREE>
+template <int SH, bool TREE, TraversalForm F>
 eos_status launch_plain(eos_ctx* ctx, const PlainParams& P, int block) {
+  auto* kernel = k_render_plain<SH, TREE, F>;
   const size_t smem = (size_t)SH * block * sizeof(uint2);
   if (smem > 48 * 1024)  // opt in to more than the default 48 KB of dynamic shared memory
-    EOS_CUDA(cudaFuncSetAttribute(k_render_plain<SH, TREE>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
+    EOS_CUDA(cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
   int resident = 0;
-  EOS_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&resident, k_render_plain<SH, TREE>, block, smem));
+  EOS_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&resident, kernel, block, smem));
   const long long per_block = (long long)P.lanes * (block / 32);
   const long long blocks = ((long long)P.n_work + per_block - 1) / per_block;
   const int grid = (int)std::max<long long>(1, std::min<long long>(blocks, (long long)ctx->num_sms * std::max(1, resident)));
-  k_render_plain<SH, TREE><<<grid, block, smem, ctx->stream>>>(P);
+  kernel<<<grid, block, smem, ctx->stream>>>(P);
   EOS_CUDA(cudaGetLastError());
   return EOS_OK;
 }
 
-template <bool TREE>
+template <bool TREE, TraversalForm F>
 eos_status launch_plain(eos_ctx* ctx, const PlainParams& P, int sh, int block) {
-  if (sh == 8) return launch_plain<8, TREE>(ctx, P, block);
-  if (sh == 16) return launch_plain<16, TREE>(ctx, P, block);
-  return launch_plain<32, TREE>(ctx, P, block);
+  if (sh == 8) return launch_plain<8, TREE, F>(ctx, P, block);
+  if (sh == 16) return launch_plain<16, TREE, F>(ctx, P, block);
+  return launch_plain<32, TREE, F>(ctx, P, block);
 }
 
 }  // namespace
@@ -536,7 +539,10 @@ eos_status render_plain(eos_ctx* ctx, const eos_scene* sc, const eos_camera& cam
   P.lanes = lanes_of(P.n_work, ctx->num_sms, tree);
   const int block = clamp_block(p.block_size);
   const int sh = pick_stack(p.stack_depth);
-  const eos_status st = tree ? launch_plain<true>(ctx, P, sh, block) : launch_plain<false>(ctx, P, sh, block);
+  const eos_status st = sc->instanced ? (tree ? launch_plain<true, kTwoLevel>(ctx, P, sh, block)
+                                              : launch_plain<false, kTwoLevel>(ctx, P, sh, block))
+                                      : (tree ? launch_plain<true, kFlat>(ctx, P, sh, block)
+                                              : launch_plain<false, kFlat>(ctx, P, sh, block));
   if (st != EOS_OK) return st;
   ctx->launches += 1;
   return EOS_OK;

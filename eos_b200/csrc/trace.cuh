@@ -542,8 +542,7 @@ __device__ __forceinline__ AnyResult any_hit_body(const DevScene& s, f3 o, f3 d,
   return any_traverse<SH, CAP>(s, o, d, r, col, stride, err);
 }
 
-// Out-of-line copies for the plain megakernel, which calls both traversals: keeping them
-// out of line bounds its register allocation.  The specialised wavefront kernels inline.
+// Out-of-line copies for kernels whose registers are set for two-level scenes.
 template <int SH>
 __device__ __noinline__ Hit closest_hit_call(const DevScene& s, f3 o, f3 d, uint32_t col, uint32_t stride, int* err) {
   return closest_hit_body<SH>(s, o, d, col, stride, err);
@@ -681,12 +680,6 @@ __device__ __forceinline__ Hit traverse_instanced(const DevScene& s, f3 o, f3 d,
   return ok ? h : walk_instanced_exact<SH, ANY>(s, o, d, col, stride, err);
 }
 
-template <int SH, bool ANY>
-__device__ __noinline__ Hit traverse_instanced_call(const DevScene& s, f3 o, f3 d, uint32_t col, uint32_t stride,
-                                                    int* err) {
-  return traverse_instanced<SH, ANY>(s, o, d, col, stride, err);
-}
-
 // Instance holding global triangle id `gid` (instances in id order).
 __device__ __forceinline__ const DevInstance* instance_of(const DevScene& s, int gid) {
   int lo = 0, hi = s.n_inst - 1;
@@ -698,32 +691,26 @@ __device__ __forceinline__ const DevInstance* instance_of(const DevScene& s, int
   return s.inst + lo;
 }
 
-// How a kernel holds the traversals: kCalls both out of line (bounds the registers of a kernel
-// that makes several kinds of queries), kFlat the flat one inline and none for two-level
-// scenes, kTwoLevel the two-level one inline and the flat one out of line.  CAP (inline
-// traversals of flat scenes): total stack entries, see ColumnStack.
-enum TraversalForm { kCalls, kFlat, kTwoLevel };
+// How a kernel holds the traversals: kFlat the flat one inline and none for two-level scenes,
+// kTwoLevel the two-level one inline and the flat one out of line (a pass may hold both kinds
+// of scenes).  CAP (inline traversals of flat scenes): total stack entries, see ColumnStack.
+enum TraversalForm { kFlat, kTwoLevel };
 
-template <int SH, TraversalForm F = kCalls, int CAP = kStackMax>
+template <int SH, TraversalForm F, int CAP = kStackMax>
 __device__ __forceinline__ Hit closest_hit(const DevScene& s, f3 o, f3 d, uint32_t col, uint32_t stride, int* err) {
-  if constexpr (F == kTwoLevel) {
+  if constexpr (F == kTwoLevel)
     if (s.inst) return traverse_instanced<SH, false>(s, o, d, col, stride, err);
-  } else if constexpr (F == kCalls) {
-    if (s.inst) return traverse_instanced_call<SH, false>(s, o, d, col, stride, err);
-  }
   if constexpr (F == kFlat || CAP == SH) return closest_hit_body<SH, CAP>(s, o, d, col, stride, err);
   else return closest_hit_call<SH>(s, o, d, col, stride, err);
 }
 
-template <int SH, TraversalForm F = kCalls, int CAP = kStackMax>
+template <int SH, TraversalForm F, int CAP = kStackMax>
 __device__ __forceinline__ AnyResult any_hit(const DevScene& s, f3 o, f3 d, uint32_t col, uint32_t stride, int* err) {
-  if constexpr (F != kFlat) {
+  if constexpr (F == kTwoLevel)
     if (s.inst) {
-      const Hit h = F == kTwoLevel ? traverse_instanced<SH, true>(s, o, d, col, stride, err)
-                                   : traverse_instanced_call<SH, true>(s, o, d, col, stride, err);
+      const Hit h = traverse_instanced<SH, true>(s, o, d, col, stride, err);
       return AnyResult{h.pos >= 0 ? 1 : 0, h.nodes, h.tests};
     }
-  }
   if constexpr (F == kFlat || CAP == SH) return any_hit_body<SH, CAP>(s, o, d, col, stride, err);
   else return any_hit_call<SH>(s, o, d, col, stride, err);
 }
