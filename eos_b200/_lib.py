@@ -124,6 +124,7 @@ SIGNATURES = [
     ("eos_ctx_set_tuning", c_int32, [c_void_p, c_uint32, POINTER(Tuning)]),
     ("eos_ctx_clear_tuning", c_int32, [c_void_p]),
     ("eos_ctx_set_limits", c_int32, [c_void_p, POINTER(Limits)]),
+    ("eos_ctx_set_build_polls", c_int32, [c_void_p, c_int32]),
     ("eos_scene_create", c_int32, [c_void_p, c_void_p, c_void_p, c_uint32, c_void_p, c_void_p, c_uint32,
                                    c_void_p, c_uint32, c_void_p, c_uint32, POINTER(BuildParams), POINTER(c_void_p)]),
     ("eos_scene_destroy", c_int32, [c_void_p]),

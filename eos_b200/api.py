@@ -108,6 +108,10 @@ class Context:
         lim = L.Limits(int(queue_entries), int(work_budget), 1 if small_stack else 0)
         L.check(self.lib.eos_ctx_set_limits(self.h, byref(lim)), "eos_ctx_set_limits")
 
+    def set_build_polls(self, polls: int = -1):
+        """Test limit of the scene builders (eos_ctx_set_build_polls); no argument clears it."""
+        L.check(self.lib.eos_ctx_set_build_polls(self.h, int(polls)), "eos_ctx_set_build_polls")
+
 
 def materials_array(mats):
     """Material rows in the C layout (eos_material, 10 floats): numpy rows of 8 or 10, or a

@@ -425,6 +425,12 @@ eos_status eos_ctx_set_limits(eos_ctx* ctx, const eos_limits* lim) {
   return EOS_OK;
 }
 
+eos_status eos_ctx_set_build_polls(eos_ctx* ctx, int32_t polls) {
+  if (!ctx) return EOS_ERR_INVALID_ARG;
+  ctx->build_polls = polls < 0 ? eos_ctx::kBuildPolls : std::min<int>(polls, eos_ctx::kBuildPolls);
+  return EOS_OK;
+}
+
 eos_status eos_scene_create(eos_ctx* ctx, const float* verts, const float* normals, uint32_t n_verts,
                             const uint32_t* tris, const uint32_t* tri_obj, uint32_t n_tris,
                             const eos_material* materials, uint32_t n_materials, const eos_light* lights,

@@ -125,6 +125,10 @@ struct eos_ctx {
   int* ring_host = nullptr;
   int* ring_dev = nullptr;
   long long ring_next = 0;
+  // polls of a missing word before a look-back of the builders gives up (scan.cuh): a
+  // fraction of a second; a test limit sets fewer (eos_ctx_set_build_polls)
+  static constexpr int kBuildPolls = 1 << 18;
+  int build_polls = kBuildPolls;
   // autotuner table: min triangle count -> tuned parameters
   std::map<uint32_t, eos_tuning> tuning;
   // test limits of the wavefront kernels (eos_ctx_set_limits); zeros = none

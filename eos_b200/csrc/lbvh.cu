@@ -442,9 +442,7 @@ struct BinaryTree {
 
 // Level state: [0] nodes of the level, [1] their first record, [3] tickets taken.
 __global__ void k_wide_init(int* __restrict__ state, int root, int* __restrict__ frontier) {
-  state[0] = 1;
-  state[1] = 0;
-  state[3] = 0;
+  for (int k = 0; k < 8; ++k) state[k] = k == 0;  // the other state: no nodes until a level writes it
   frontier[0] = root;
 }
 
@@ -457,7 +455,8 @@ __global__ void k_wide_init(int* __restrict__ state, int root, int* __restrict__
 // write sequence took three and a read-back of the size.
 __global__ void __launch_bounds__(kScanBlock) k_wide_level(BinaryTree T, int* __restrict__ state,
                                                            int* __restrict__ state_out, int* __restrict__ slot,
-                                                           int number, int level, unsigned long long* __restrict__ words,
+                                                           int number, int level, int polls,
+                                                           unsigned long long* __restrict__ words,
                                                            const int* __restrict__ frontier,
                                                            int* __restrict__ frontier_out, int max_children,
                                                            float4* __restrict__ wnodes, int max_nodes, int* err) {
@@ -469,14 +468,14 @@ __global__ void __launch_bounds__(kScanBlock) k_wide_level(BinaryTree T, int* __
   const int next_base = base + n_in;
   if (blockIdx.x == 0 && threadIdx.x == 0) {
     state_out[3] = 0;
-    if (n_in == 0) {  // past the last level
+    if (n_in == 0 && !(*(volatile int*)err & kErrTimeout)) {  // past the last level
       state_out[0] = 0;
       state_out[1] = next_base;
       ring_publish(slot, 0, next_base, 0, number);
     }
   }
   for (;;) {
-    if (threadIdx.x == 0) s_tile = atomicAdd(&state[3], 1);
+    if (threadIdx.x == 0) s_tile = take_tile(&state[3], err);
     __syncthreads();
     const int tile = s_tile;
     if (tile >= n_tiles) return;
@@ -488,7 +487,8 @@ __global__ void __launch_bounds__(kScanBlock) k_wide_level(BinaryTree T, int* __
     int total;
     const int ex = block_exclusive_scan(m, total);
     if (threadIdx.x < 32) {
-      const unsigned long long before = tiles_before(words, tile, (unsigned long long)total, (unsigned)(level % 4095 + 1));
+      const unsigned long long before = tiles_before(words, tile, (unsigned long long)total,
+                                                     (unsigned)(level % 4095 + 1), polls);
       if (threadIdx.x == 0) {
         s_before = before;
         if (tile == n_tiles - 1 && before <= kTileValue) {
@@ -593,7 +593,7 @@ eos_status write_records(eos_ctx* ctx, const BinaryTree& T, int root, int width,
     const int k = (int)(ring.issued & 1);
     const int grid = (int)std::min<long long>(scan_blocks(most), ctx->num_sms * 4);
     es = ring.launch(k_wide_level, grid, kScanBlock, T, state + 4 * k, state + 4 * (k ^ 1), ring.next_slot(),
-                     ring.next_number(), (int)ring.issued, words, frontier[k], frontier[k ^ 1], width, out, max_nodes,
+                     ring.next_number(), (int)ring.issued, ctx->build_polls, words, frontier[k], frontier[k ^ 1], width, out, max_nodes,
                      ctx->d_err);
     if (es != EOS_OK) return es;
     most = std::min<long long>(most * width, T.n);

@@ -47,7 +47,7 @@ __global__ void k_ploc_state_init(int* __restrict__ state, int n, int* __restric
   state[0] = n;
   state[1] = 0;
   state[2] = 1;
-  state[3] = 0;
+  for (int k = 3; k < 8; ++k) state[k] = 0;  // the other state: no clusters until a round writes it
   *depth_max = 0;
 }
 
@@ -95,9 +95,9 @@ __device__ __forceinline__ int forced_partner(int i, int nc) { return (i & 1) ? 
 template <int kRoundThreads>
 __global__ void __launch_bounds__(kRoundThreads) k_ploc_round(
     PlocTree T, int* __restrict__ state, int* __restrict__ state_out, int* __restrict__ slot, int number, int round,
-    int force, unsigned long long* __restrict__ words, const int* __restrict__ cid, const float4* __restrict__ lo,
+    int force, int polls, unsigned long long* __restrict__ words, const int* __restrict__ cid, const float4* __restrict__ lo,
     const float4* __restrict__ hi, int* __restrict__ cid_out, float4* __restrict__ lo_out, float4* __restrict__ hi_out,
-    int* __restrict__ err) {
+    int* err) {
   constexpr int kBoxes = kRoundThreads + 2 * kRadius, kRoundTile = round_tile(kRoundThreads);
   __shared__ float4 slo[2][kBoxes / 2 + 4], shi[2][kBoxes / 2 + 4];
   __shared__ int sid[kBoxes], snn[kRoundThreads];
@@ -105,7 +105,7 @@ __global__ void __launch_bounds__(kRoundThreads) k_ploc_round(
   __shared__ unsigned long long s_before;
   const int t = threadIdx.x;
   ring_wait();
-  if (t == 0) s_tile = atomicAdd(&state[3], 1);
+  if (t == 0) s_tile = take_tile(&state[3], err);
   const int nc = state[0], node_base = state[1];
   __syncthreads();
   const int tile = s_tile;
@@ -158,7 +158,7 @@ __global__ void __launch_bounds__(kRoundThreads) k_ploc_round(
   const int ex = block_exclusive_scan((int)keep | ((int)make << 16), total);
   if (t < 32) {
     const unsigned long long sum = (unsigned)(total & 0xffff) | ((unsigned long long)(total >> 16) << 25);
-    const unsigned long long before = tiles_before(words, tile, sum, (unsigned)(round % 4095 + 1));
+    const unsigned long long before = tiles_before(words, tile, sum, (unsigned)(round % 4095 + 1), polls);
     if (t == 0) s_before = before;
     if (t == 0 && tile == 0) state_out[3] = 0;
     if (t == 0 && tile == n_tiles - 1 && before <= kTileValue) {
@@ -212,6 +212,7 @@ __global__ void __launch_bounds__(kTail) k_ploc_tail(PlocTree T, int* __restrict
   float4 *const slo = slo_ + kRadius, *const shi = shi_ + kRadius;
   const float4 out_lo = make_float4(-kInf, -kInf, -kInf, 0.0f), out_hi = make_float4(kInf, kInf, kInf, 0.0f);
   const int i = threadIdx.x, lane = i & 31, warp = i >> 5;
+  if (*err & kErrTimeout) return;  // a round gave up: its clusters are not complete
   int nc = state[0], node_base = state[1];
   int force = state[2] == 0 && nc > 1;  // the last round merged nothing: the forced round is next
   if (nc > kTail) {  // the host launches this only at or below kTail
@@ -339,14 +340,17 @@ __global__ void __launch_bounds__(kTail) k_ploc_tail(PlocTree T, int* __restrict
 
 // Depth-first position of the first triangle of every leaf (perm[p], by Morton position) and
 // of every collapsed subtree (first[v]): the sum of the left siblings' counts on the way to
-// the root.  An unfinished or too deep tree is reported as deeper than kMaxWalk.
+// the root.  A too deep tree is reported as deeper than kMaxWalk, an unfinished one (a round
+// gave up) as kUnfinished.
+constexpr int kUnfinished = kMaxWalk + 2;
 __global__ void k_ploc_positions(PlocTree T, const int* __restrict__ state, int* __restrict__ first,
-                                 uint32_t* __restrict__ perm, int* __restrict__ depth_max) {
+                                 uint32_t* __restrict__ perm, int* __restrict__ depth_max,
+                                 const int* __restrict__ err) {
   const int v = blockIdx.x * blockDim.x + threadIdx.x;
   const int n = T.n;
   int steps = 0;
-  if (state[1] != n - 1) {
-    steps = kMaxWalk + 1;
+  if (state[1] != n - 1 || (*err & kErrTimeout)) {
+    steps = kUnfinished;
   } else if (v >= n - 1 ? v < 2 * n - 1 : T.bhi[v].w != 0.0f) {
     int pos = 0, node = v;
     while (node != n - 2 && steps <= kMaxWalk) {
@@ -371,7 +375,7 @@ inline int grid_of(long long n, int block) { return (int)std::max<long long>(1, 
 // decision of every interior node, perm[p] = the record position of Morton position p and
 // first[v] = that of a collapsed subtree's first triangle.  *depth = the deepest node's
 // depth; above 4 * kStackMax first and perm are not complete and the caller must use another
-// builder.
+// builder.  EOS_ERR_TIMEOUT when a round gave up: nothing may be read then.
 eos_status build_ploc(eos_ctx* ctx, int n, int max_leaf, int sah, float4* blo, float4* bhi, int2* child, int* count,
                       int* first, uint32_t* perm, int* depth) {
   cudaStream_t st = ctx->stream;
@@ -413,7 +417,7 @@ eos_status build_ploc(eos_ctx* ctx, int n, int max_leaf, int sah, float4* blo, f
     // the first round's clusters are the leaf boxes themselves
     const eos_status st_l = ring.launch(
         small ? k_ploc_round<256> : k_ploc_round<512>, grid_of(nc_ub, round_tile(threads)), threads, T,
-        state + 4 * cur, state + 4 * (cur ^ 1), ring.next_slot(), ring.next_number(), r, force, words,
+        state + 4 * cur, state + 4 * (cur ^ 1), ring.next_slot(), ring.next_number(), r, force, ctx->build_polls, words,
         r ? cid[cur] : nullptr, r ? clo[cur] : blo + (n - 1), r ? chi[cur] : bhi + (n - 1), cid[cur ^ 1],
         clo[cur ^ 1], chi[cur ^ 1], ctx->d_err);
     cur ^= 1;
@@ -443,10 +447,11 @@ eos_status build_ploc(eos_ctx* ctx, int n, int max_leaf, int sah, float4* blo, f
     if (ring.issued > 4ll * n + 8) return EOS_ERR_TIMEOUT;  // cannot happen: every round or its forced repeat merges
     if ((es = enqueue(0)) != EOS_OK) return es;
   }
-  k_ploc_positions<<<grid_of(2 * (long long)n - 1, 256), 256, 0, st>>>(T, state + 4 * cur, first, perm, dmax);
+  k_ploc_positions<<<grid_of(2 * (long long)n - 1, 256), 256, 0, st>>>(T, state + 4 * cur, first, perm, dmax,
+                                                                       ctx->d_err);
   EOS_CUDA(cudaMemcpyAsync(depth, dmax, 4, cudaMemcpyDeviceToHost, st));
   EOS_CUDA(cudaStreamSynchronize(st));
-  return EOS_OK;
+  return *depth == kUnfinished ? EOS_ERR_TIMEOUT : EOS_OK;
 }
 
 }  // namespace eos

@@ -4,15 +4,19 @@
 // sums (Merrill & Garland, "Single-pass Parallel Prefix Scan with Decoupled Look-back",
 // 2016).  Tickets are taken in order by running blocks, so the tiles waited for always run.
 #pragma once
-#include <cuda_runtime.h>
-#include <stdint.h>
+#include "eos_internal.cuh"
 
 namespace eos {
 
 constexpr int kScanBlock = 256;
-// Polls of a look-back before it gives up (a fraction of a second); its caller then raises
-// the timeout bit of the error word and leaves the launch without writing.
-constexpr int kMaxPolls = 1 << 18;
+constexpr int kNoTile = 0x7fffffff;
+
+// This block's next tile; kNoTile once a look-back of the call has given up (raised the timeout
+// bit), so that no later launch reads what the tile that gave up left unwritten.  One thread.
+__device__ __forceinline__ int take_tile(int* tickets, const int* err) {
+  const int tile = atomicAdd(tickets, 1);
+  return *(const volatile int*)err & kErrTimeout ? kNoTile : tile;
+}
 
 template <class T>
 __device__ __forceinline__ T warp_inclusive_scan(T v) {
@@ -46,7 +50,7 @@ __device__ __forceinline__ T block_exclusive_scan(T v, T& total) {
 }
 
 // Published sum of a tile: flag in the top two bits (1 = the tile's own sum, 2 = the sum of
-// all tiles up to it), the launch's epoch in the next twelve, the value in the low 50.  A
+// all tiles up to it, 3 = it gave up, as does who meets it), the launch's epoch in the next twelve, the value in the low 50.  A
 // word of an earlier launch carries another epoch, so the array is cleared once per build,
 // not per launch.  Epochs repeat after 4,095 launches: a build of more (PLOC rounds of a
 // degenerate scene) must write every word it reads in each of them, which it does because
@@ -57,9 +61,11 @@ __device__ __forceinline__ unsigned long long tile_word(unsigned flag, unsigned 
 }
 
 // Sum of the tiles before `tile`, whose own sum is `sum`; called by all lanes of one warp
-// with the same arguments.  kTileValue + 1 when a tile did not publish in time.
+// with the same arguments.  kTileValue + 1 when a tile did not publish within `polls` polls
+// of its word (eos_ctx::build_polls); the caller then raises the timeout bit and leaves the
+// launch without writing.
 __device__ __forceinline__ unsigned long long tiles_before(volatile unsigned long long* words, int tile,
-                                                           unsigned long long sum, unsigned epoch) {
+                                                           unsigned long long sum, unsigned epoch, int polls) {
   const int lane = threadIdx.x & 31;
   if (lane == 0) words[tile] = tile_word(tile == 0 ? 2u : 1u, epoch, sum);
   unsigned long long before = 0;
@@ -67,14 +73,17 @@ __device__ __forceinline__ unsigned long long tiles_before(volatile unsigned lon
     const int i = at - lane;
     unsigned long long w = tile_word(2u, epoch, 0);  // before the first tile
     unsigned missing = 1;
-    for (int poll = 0; missing && poll < kMaxPolls; ++poll) {
+    for (int poll = 0; missing && poll < polls; ++poll) {
       if (i >= 0) w = words[i];
       const bool there = (w >> 62) != 0 && ((w >> 50) & 0xfffu) == (epoch & 0xfffu);
       missing = __ballot_sync(0xffffffffu, !there);
     }
-    if (missing) return kTileValue + 1;
-    const unsigned whole = __ballot_sync(0xffffffffu, (w >> 62) == 2u);
+    const unsigned whole = missing ? 0 : __ballot_sync(0xffffffffu, (w >> 62) == 2u);
     const int last = whole ? __ffs(whole) - 1 : 31;  // nearest tile that holds a full prefix
+    if (missing || __any_sync(0xffffffffu, lane <= last && (w >> 62) == 3u)) {
+      if (lane == 0) words[tile] = tile_word(3u, epoch, 0);
+      return kTileValue + 1;
+    }
     unsigned long long v = lane <= last ? (w & kTileValue) : 0;
     for (int off = 16; off > 0; off >>= 1) v += __shfl_xor_sync(0xffffffffu, v, off);
     before += v;

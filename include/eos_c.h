@@ -290,6 +290,10 @@ typedef struct eos_limits {
   int32_t small_stack;
 } eos_limits;
 eos_status eos_ctx_set_limits(eos_ctx* ctx, const eos_limits* limits);
+/* Test limit of the scene builders, as above: polls a block spends on the sum of an earlier
+ * one before it gives up; a build in which one does returns EOS_ERR_TIMEOUT and makes no
+ * scene, and the context stays usable.  polls < 0: the default (a fraction of a second). */
+eos_status eos_ctx_set_build_polls(eos_ctx* ctx, int32_t polls);
 
 /* ---------------------------------------------------------------------------- scenes */
 /* verts / normals [n_verts*3], tris [n_tris*3] vertex indices, tri_obj [n_tris] material
