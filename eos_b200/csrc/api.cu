@@ -4,6 +4,7 @@
 #include <algorithm>
 #include <cstdio>
 #include <cstring>
+#include <mutex>
 #include <type_traits>
 #include <vector>
 
@@ -11,7 +12,20 @@
 
 using namespace eos;
 
+namespace {
+
+// The process's contexts: pool_free waits for their asynchronous batches.  The lock also
+// covers the making of a context's copy stream.
+std::mutex g_contexts_mutex;
+std::vector<eos_ctx*> g_contexts;
+
+}  // namespace
+
 eos_ctx::~eos_ctx() {
+  {
+    std::lock_guard<std::mutex> lock(g_contexts_mutex);
+    g_contexts.erase(std::remove(g_contexts.begin(), g_contexts.end(), this), g_contexts.end());
+  }
   if (copy_stream) cudaStreamSynchronize(copy_stream);
   for (AsyncSlot& a : async) {
     if (a.rendered) cudaEventDestroy(a.rendered);
@@ -56,7 +70,11 @@ void* scratch(eos_ctx* ctx, const char* name, size_t bytes, eos_status* st) {
   if (b.bytes >= bytes && b.ptr) return b.ptr;
   if (b.ptr) {
     if (b.pooled) {
-      pool_free(ctx, &b.ptr, 1);
+      const eos_status freed = pool_free(ctx, &b.ptr, 1);
+      if (freed != EOS_OK) {
+        if (st) *st = freed;
+        return nullptr;
+      }
     } else {
       cudaStreamSynchronize(ctx->stream);
       cudaFree(b.ptr);
@@ -95,11 +113,17 @@ cudaError_t pool_alloc(eos_ctx* ctx, void** p, size_t bytes) {
   return e;
 }
 
-void pool_free(eos_ctx* ctx, void* const* p, int n) {
-  cudaDeviceSynchronize();
+eos_status pool_free(eos_ctx* ctx, void* const* p, int n) {
+  EOS_CUDA(cudaStreamSynchronize(ctx->stream));
+  {
+    std::lock_guard<std::mutex> lock(g_contexts_mutex);
+    for (const eos_ctx* c : g_contexts)
+      if (c->device == ctx->device && c->copy_stream) EOS_CUDA(cudaStreamSynchronize(c->copy_stream));
+  }
   for (int k = 0; k < n; ++k)
-    if (p[k]) cudaFreeAsync(p[k], ctx->own_stream);
-  cudaStreamSynchronize(ctx->own_stream);
+    if (p[k]) EOS_CUDA(cudaFreeAsync(p[k], ctx->own_stream));
+  EOS_CUDA(cudaStreamSynchronize(ctx->own_stream));
+  return EOS_OK;
 }
 
 namespace {
@@ -234,7 +258,10 @@ eos_status set_device(eos_ctx* ctx) {
 // Copy stream, events and pinned read-back of asynchronous batches (made on first use).
 eos_status async_setup(eos_ctx* ctx) {
   if (ctx->copy_stream) return EOS_OK;
-  EOS_CUDA(cudaStreamCreateWithFlags(&ctx->copy_stream, cudaStreamNonBlocking));
+  {
+    std::lock_guard<std::mutex> lock(g_contexts_mutex);
+    EOS_CUDA(cudaStreamCreateWithFlags(&ctx->copy_stream, cudaStreamNonBlocking));
+  }
   for (eos_ctx::AsyncSlot& a : ctx->async) {
     EOS_CUDA(cudaEventCreateWithFlags(&a.rendered, cudaEventDisableTiming));
     EOS_CUDA(cudaEventCreateWithFlags(&a.copied, cudaEventDisableTiming));
@@ -370,6 +397,10 @@ eos_status eos_ctx_create(int32_t device, eos_ctx** out) {
     cudaGetLastError();
     delete ctx;
     return st;
+  }
+  {
+    std::lock_guard<std::mutex> lock(g_contexts_mutex);
+    g_contexts.push_back(ctx);
   }
   *out = ctx;
   return EOS_OK;
@@ -507,9 +538,9 @@ eos_status eos_scene_destroy(eos_scene* sc) {
   }
   void* bufs[] = {sc->d_nodes, sc->d_tris, sc->d_shade, sc->d_pos_of_id, sc->d_mats, sc->d_lights, sc->d_codes,
                   sc->d_order, sc->d_inst};
-  if (sc->ctx) pool_free(sc->ctx, bufs, (int)(sizeof bufs / sizeof bufs[0]));
+  const eos_status st = sc->ctx ? pool_free(sc->ctx, bufs, (int)(sizeof bufs / sizeof bufs[0])) : EOS_OK;
   delete sc;
-  return EOS_OK;
+  return st;
 }
 
 eos_status eos_scene_set_materials(eos_scene* sc, const eos_material* m, uint32_t n) {

@@ -218,15 +218,19 @@ void* scratch(eos_ctx* ctx, const char* name, size_t bytes, eos_status* st);
 // the device at once and all of it with the context, or when an allocation of the context
 // fails.  Allocations and frees are ordered on the context's own stream; the calls that
 // allocate fill the arrays on the context's stream, after the allocation, and wait for it
-// before they return, so a finished scene may be used on any stream.  A free waits for the
-// whole device first, as cudaFree does.  Scratch from kPoolScratch bytes on stays with
+// before they return, so a finished scene may be used on any stream.  A free first waits for
+// the context's stream and for the asynchronous batches of every context on the device, which
+// may render this one's scenes (a batch's copy stream follows its render; all other calls wait
+// for their work themselves).  It does not wait for the device, which is invalid while some
+// thread captures a stream, as a batch's first call does.  Where a wait fails nothing is given
+// back.  Scratch from kPoolScratch bytes on stays with
 // cudaMalloc: a new context's first call that needs 3.6 GB of queues (four 1080p views) takes
 // 12 ms with it and 28 ms from the pool, while one that needs buffers below the line takes
 // 2.1 ms from the pool and 3.6 without (a 512 x 512 view with four samples).
 constexpr unsigned long long kPoolKeep = 1ull << 30;
 constexpr size_t kPoolScratch = 64u << 20;
 cudaError_t pool_alloc(eos_ctx* ctx, void** p, size_t bytes);
-void pool_free(eos_ctx* ctx, void* const* p, int n);
+eos_status pool_free(eos_ctx* ctx, void* const* p, int n);
 // Pointer classification (cudaPointerGetAttributes): true for device/managed memory.
 bool is_device_ptr(const void* p);
 
