@@ -65,22 +65,36 @@ eos_ctx::~eos_ctx() {
 
 namespace eos {
 
+namespace {
+
+eos_status free_buffer(eos_ctx* ctx, DevBuffer& b) {
+  if (!b.ptr) return EOS_OK;
+  if (b.pooled) {
+    EOS_TRY(pool_free(ctx, &b.ptr, 1));
+  } else {
+    cudaStreamSynchronize(ctx->stream);
+    cudaFree(b.ptr);
+  }
+  b.ptr = nullptr;
+  b.bytes = 0;
+  return EOS_OK;
+}
+
+}  // namespace
+
+eos_status release_scratch(eos_ctx* ctx, const char* prefix) {
+  for (auto& kv : ctx->scratch)
+    if (kv.first.compare(0, std::strlen(prefix), prefix) == 0) EOS_TRY(free_buffer(ctx, kv.second));
+  return EOS_OK;
+}
+
 void* scratch(eos_ctx* ctx, const char* name, size_t bytes, eos_status* st) {
   DevBuffer& b = ctx->scratch[name];
   if (b.bytes >= bytes && b.ptr) return b.ptr;
-  if (b.ptr) {
-    if (b.pooled) {
-      const eos_status freed = pool_free(ctx, &b.ptr, 1);
-      if (freed != EOS_OK) {
-        if (st) *st = freed;
-        return nullptr;
-      }
-    } else {
-      cudaStreamSynchronize(ctx->stream);
-      cudaFree(b.ptr);
-    }
-    b.ptr = nullptr;
-    b.bytes = 0;
+  const eos_status freed = free_buffer(ctx, b);
+  if (freed != EOS_OK) {
+    if (st) *st = freed;
+    return nullptr;
   }
   const size_t want = std::max<size_t>(bytes, 256);
   b.pooled = want < kPoolScratch;

@@ -161,6 +161,7 @@ struct eos_ctx {
   WfLane wf_lane[kWfLanes];
   cudaEvent_t ev_fork = nullptr;
   cudaEvent_t ev_join[kWfLanes] = {};
+  bool low_memory = false;  // a large chunk's queues did not fit the device (render_wavefront)
   int async_next = 0;
   long long async_seq = 0;
   unsigned long long* async_host = nullptr;  // pinned [2][kCounters + 1] (counters, error word)
@@ -211,6 +212,8 @@ namespace eos {
 
 // Scratch buffers owned by the context, grown on demand and reused across calls.
 void* scratch(eos_ctx* ctx, const char* name, size_t bytes, eos_status* st);
+// Gives back the scratch buffers whose names begin with `prefix`.
+eos_status release_scratch(eos_ctx* ctx, const char* prefix);
 // Scene arrays and scratch buffers below kPoolScratch come from a memory pool of the context,
 // because cudaMalloc and cudaFree of the 250 MB of a 1M-triangle scene cost more than its
 // build (create + destroy 26 ms of which 3.8 ms build, and up to 0.7 s on a busy host).  What
@@ -294,6 +297,12 @@ namespace eos {
 // Records a failing CUDA call for eos_last_error_detail (per host thread).
 void note_cuda_error(cudaError_t e, const char* file, int line);
 }  // namespace eos
+
+#define EOS_TRY(x)                  \
+  do {                              \
+    eos_status s_ = (x);            \
+    if (s_ != EOS_OK) return s_;    \
+  } while (0)
 
 #define EOS_CUDA(call)                                   \
   do {                                                   \

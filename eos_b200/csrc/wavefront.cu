@@ -36,6 +36,7 @@ namespace eos {
 namespace {
 
 constexpr long long kChunkPathsMax = 1ll << 25;
+constexpr long long kChunkPathsLow = 1ll << 24;  // where the device has no memory for those
 constexpr long long kTreeChunkPathsMax = 1ll << 24;  // a ray-tree hit record packs path and node
 constexpr long long kQueueBudget = 16ll << 30;  // bytes of queues and accumulators per chunk
 constexpr long long kLaneSplitMin = 1ll << 20;  // paths of a chunk from which it runs as several lanes
@@ -596,12 +597,6 @@ struct StageTimer {
   }
 };
 
-#define EOS_TRY(x)                  \
-  do {                              \
-    eos_status s_ = (x);            \
-    if (s_ != EOS_OK) return s_;    \
-  } while (0)
-
 // The kernels of one configuration: a warp of the nearest-hit / shadow kernels takes
 // `queue_chunk` rays and finishes all before taking more.  small_stack selects the test
 // instantiation whose traversal stack is its SH shared-memory entries only (launch_config
@@ -811,10 +806,10 @@ eos_status run_sequence(cudaStream_t st, int num_sms, const LaunchConfig& lc, co
                              lc.smem_a, false, lc.tree, lc.inst, tm, ov, launches);
 }
 
-}  // namespace
-
-eos_status render_wavefront(eos_ctx* ctx, const eos_job* jobs, uint32_t n_jobs, const eos_render_params& p,
-                            bool use_graph) {
+// A pass in chunks of at most chunk_max paths; EOS_ERR_OOM comes before anything is queued.
+// *biggest_out: paths of its largest chunk.
+eos_status render_chunks(eos_ctx* ctx, const eos_job* jobs, uint32_t n_jobs, const eos_render_params& p,
+                         bool use_graph, long long chunk_max, long long* biggest_out) {
   // host job table + chunk plan
   std::vector<DevJob> dj(n_jobs);
   long long total = 0;
@@ -836,7 +831,7 @@ eos_status render_wavefront(eos_ctx* ctx, const eos_job* jobs, uint32_t n_jobs, 
   const long long per_path =
       width * (2ll * 32 + 2 * (32 + 4 + 32ll * std::max(1, max_lights))) + 16ll * (tree ? nn : depth + 1);
   const long long chunk_paths =
-      std::max(1ll << 16, std::min(tree ? kTreeChunkPathsMax : kChunkPathsMax, kQueueBudget / per_path));
+      std::max(1ll << 16, std::min(tree ? std::min(chunk_max, kTreeChunkPathsMax) : chunk_max, kQueueBudget / per_path));
   for (uint32_t j = 0; j < n_jobs; ++j) {
     DevJob& d = dj[j];
     fill_job(jobs[j], total, tree_records, (p.flags & EOS_FLAG_AA_GRID) != 0, d);
@@ -861,6 +856,7 @@ eos_status render_wavefront(eos_ctx* ctx, const eos_job* jobs, uint32_t n_jobs, 
   const bool timing = (p.flags & EOS_FLAG_STAGE_TIMING) != 0;
   long long biggest = 0;
   for (const Chunk& c : merged) biggest = std::max<long long>(biggest, c.n);
+  *biggest_out = biggest;
   std::vector<Chunk> lane_chunks[kLanes];
   if (timing || depth == 0 || !use_graph || biggest < kLaneSplitMin) {
     lane_chunks[0] = merged;
@@ -1019,6 +1015,20 @@ eos_status render_wavefront(eos_ctx* ctx, const eos_job* jobs, uint32_t n_jobs, 
   if (ctx->graphs.size() >= 8) ctx->graphs.erase(ctx->graphs.begin());
   ctx->graphs.push_back(std::move(bg));
   return EOS_OK;
+}
+
+}  // namespace
+
+eos_status render_wavefront(eos_ctx* ctx, const eos_job* jobs, uint32_t n_jobs, const eos_render_params& p,
+                            bool use_graph) {
+  long long biggest = 0;
+  const eos_status st =
+      render_chunks(ctx, jobs, n_jobs, p, use_graph, ctx->low_memory ? kChunkPathsLow : kChunkPathsMax, &biggest);
+  if (st != EOS_ERR_OOM || biggest <= kChunkPathsLow) return st;
+  cudaGetLastError();
+  ctx->low_memory = true;  // the context's later passes do not try again: buffers and graphs stay
+  EOS_TRY(release_scratch(ctx, "wf."));  // a part of the large chunk's buffers
+  return render_chunks(ctx, jobs, n_jobs, p, use_graph, kChunkPathsLow, &biggest);
 }
 
 }  // namespace eos
