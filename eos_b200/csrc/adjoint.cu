@@ -165,7 +165,7 @@ __device__ __forceinline__ void hit_adjoint(const BwArgs& A, bool alive, f3 P, f
       const float* lp = s.lights + 6 * l;
       const float C[3] = {__ldg(lp + 3), __ldg(lp + 4), __ldg(lp + 5)};
       f3 u = sub3(mk3(__ldg(lp), __ldg(lp + 1), __ldg(lp + 2)), P);
-      const float iul = 1.0f / sqrtf(dot3(u, u));
+      const float ul = sqrtf(dot3(u, u)), iul = 1.0f / ul;
       f3 L = scale3(iul, u);
       float ndl = dot3(N, L);
       f3 wv = sub3(scale3(2.0f * ndl, N), L);
@@ -184,13 +184,15 @@ __device__ __forceinline__ void hit_adjoint(const BwArgs& A, bool alive, f3 P, f
         b += gT[c] * C[c] * ks[c];
       }
       f3 gp = mk3(0, 0, 0);
-      if (ndl > 0.0f) gp = add3(gp, scale3(a * iul, sub3(N, scale3(ndl, L))));
+      if (ndl > 0.0f) gp = add3(gp, scale3(a / ul, sub3(N, scale3(ndl, L))));
       if (vr > 0.0f) {
         gm[6] += b * fs * logf(vr) * shin;
         f3 q = scale3(iwl, sub3(V, scale3(vr, R)));
         f3 q2 = sub3(scale3(2.0f * dot3(N, q), N), q);
         f3 gs = scale3(iul, sub3(q2, scale3(dot3(L, q2), L)));
-        gp = add3(gp, scale3(b * shin * (fs / vr), gs));  // s (V.R)^(s-1)
+        // s (V.R)^(s-1): by a second power where (V.R)^s has lost bits or all of them
+        const float p1 = fs >= 0x1p-126f ? fs / vr : powf(vr, shin - 1.0f);
+        gp = add3(gp, scale3(b * (shin * p1), gs));
       }
       gl[3] = gp.x;
       gl[4] = gp.y;
