@@ -59,7 +59,7 @@ def build(force: bool = False, verbose_ptxas: bool = False) -> str:
     with cf.ThreadPoolExecutor(max_workers=min(8, max(1, len(jobs)))) as ex:
         results = list(ex.map(lambda c: subprocess.run(c, capture_output=True, text=True), jobs))
     for c, r in zip(jobs, results):
-        if verbose_ptxas or r.returncode != 0:
+        if verbose_ptxas or r.returncode != 0 or "warning" in r.stderr:
             sys.stderr.write(r.stdout + r.stderr)
         if r.returncode != 0:
             raise RuntimeError(f"nvcc failed: {' '.join(c)}")

@@ -186,34 +186,34 @@ struct TreePath {
       cnt[kCntHits]++;
       const ShadedHit r = shade_hit<SH, F>(P, o, d, h, cnt, col, stride);
       if (rec) rec->shadow = r.mask;
-      TreeFrame F;
-      F.phong = r.phong;
+      TreeFrame f;
+      f.phong = r.phong;
       f3 ro = zero, rd = zero;
       const bool has_r = r.m[7] > 0.0f;
-      F.wR = has_r ? r.m[7] : 0.0f;
+      f.wR = has_r ? r.m[7] : 0.0f;
       if (has_r) mirror_ray(d, r.P, r.N, ro, rd);
-      F.has_t = r.m[8] > 0.0f;
-      F.K = F.has_t ? transparent_ray(r.m, s.ambient_index, d, r.P, r.N, F.to, F.td) : 0.0f;
-      F.cR = zero;
-      F.node = node;
-      F.depth = depth;
-      if (depth < P.trace_depth && (has_r || F.has_t)) {
-        F.in_t = !has_r;
-        if (has_r && F.has_t) open |= 1u << sp;
-        st[sp++] = F;
+      f.has_t = r.m[8] > 0.0f;
+      f.K = f.has_t ? transparent_ray(r.m, s.ambient_index, d, r.P, r.N, f.to, f.td) : 0.0f;
+      f.cR = zero;
+      f.node = node;
+      f.depth = depth;
+      if (depth < P.trace_depth && (has_r || f.has_t)) {
+        f.in_t = !has_r;
+        if (has_r && f.has_t) open |= 1u << sp;
+        st[sp++] = f;
         if (has_r) {
           o = ro;
           d = rd;
           node = 2 * node + 1;
         } else {
-          o = F.to;
-          d = F.td;
+          o = f.to;
+          d = f.td;
           node = 2 * node + 2;
         }
         ++depth;
         return false;
       }
-      c = tree_colour(F.phong, F.wR, zero, F.has_t, F.K, zero);  // children beyond the trace depth
+      c = tree_colour(f.phong, f.wR, zero, f.has_t, f.K, zero);  // children beyond the trace depth
     }
     return hand_up(c);
   }
@@ -222,35 +222,35 @@ struct TreePath {
   __device__ __forceinline__ bool hand_up(f3& c) {
     const f3 zero = mk3(0.0f, 0.0f, 0.0f);
     if (waiting) {
-      const TreeFrame& F = st[--sp];
+      const TreeFrame& f = st[--sp];
       waiting = false;
-      c = tree_colour(F.phong, F.wR, F.cR, true, F.K, F.to);
+      c = tree_colour(f.phong, f.wR, f.cR, true, f.K, f.to);
     }
     while (sp > 0) {
-      TreeFrame& F = st[sp - 1];
+      TreeFrame& f = st[sp - 1];
       const uint32_t bit = 1u << (sp - 1);
-      if (!F.in_t) {
-        F.cR = c;
-        if (F.has_t) {
-          F.in_t = true;
+      if (!f.in_t) {
+        f.cR = c;
+        if (f.has_t) {
+          f.in_t = true;
           if (open & bit) {
             open &= ~bit;
-            o = F.to;
-            d = F.td;
-            node = 2 * F.node + 2;
-            depth = F.depth + 1;
+            o = f.to;
+            d = f.td;
+            node = 2 * f.node + 2;
+            depth = f.depth + 1;
             return false;
           }
           if (lent & bit) {
             waiting = true;
             return false;
           }
-          c = tree_colour(F.phong, F.wR, F.cR, true, F.K, F.to);  // another lane traced it
+          c = tree_colour(f.phong, f.wR, f.cR, true, f.K, f.to);  // another lane traced it
         } else {
-          c = tree_colour(F.phong, F.wR, F.cR, false, 0.0f, zero);
+          c = tree_colour(f.phong, f.wR, f.cR, false, 0.0f, zero);
         }
       } else {
-        c = tree_colour(F.phong, F.wR, F.cR, true, F.K, c);
+        c = tree_colour(f.phong, f.wR, f.cR, true, f.K, c);
       }
       --sp;
     }
@@ -275,11 +275,11 @@ __device__ __forceinline__ void share_trees(Path& t, uint32_t idle, bool& active
       frame = __ffs(t.open) - 1;
       t.open &= t.open - 1;
       t.lent |= 1u << frame;
-      const TreeFrame& F = t.st[frame];
-      o = F.to;
-      d = F.td;
-      node = 2 * F.node + 2;
-      depth = F.depth + 1;
+      const TreeFrame& f = t.st[frame];
+      o = f.to;
+      d = f.td;
+      node = 2 * f.node + 2;
+      depth = f.depth + 1;
     }
     o = mk3(__shfl_sync(~0u, o.x, from), __shfl_sync(~0u, o.y, from), __shfl_sync(~0u, o.z, from));
     d = mk3(__shfl_sync(~0u, d.x, from), __shfl_sync(~0u, d.y, from), __shfl_sync(~0u, d.z, from));
