@@ -264,6 +264,7 @@ template <class Path>
 __device__ __forceinline__ void share_trees(Path& t, uint32_t idle, bool& active, bool& fresh, int& x, int& ly,
                                             int& smp) {
   const int lane = threadIdx.x & 31;
+  __syncwarp();  // the owner's clearing of its tree record comes before the taker's writes to it
   uint32_t open = __ballot_sync(0xffffffffu, active && t.open != 0);
   while (open && idle) {
     const int from = __ffs(open) - 1, to = __ffs(idle) - 1;
