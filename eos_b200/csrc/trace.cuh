@@ -147,7 +147,6 @@ struct AnyResult {
 //   leaf          0x80000000 | (count - 1) << 25 | first   (count <= 32, first < 2^25)
 //   kDone (-1)    end of traversal (never stored in a node; bit 30 distinguishes it)
 constexpr int kDone = -1;
-__device__ __forceinline__ bool is_leaf_ref(int r) { return ((uint32_t)r & 0xC0000000u) == 0x80000000u; }
 __device__ __forceinline__ int leaf_first(int r) { return r & 0x01ffffff; }
 __device__ __forceinline__ int leaf_count(int r) { return ((r >> 25) & 31) + 1; }
 
