@@ -552,12 +552,13 @@ __global__ void k_wf_resolve(WfArgs A) {
     f3 sum = mk3(0, 0, 0);
     int x, y, smp;
     if (spp <= 32 && (spp & (spp - 1)) == 0) {
-      const f3 c = path_colour<TREE>(A, i);
+      const bool pixel = path_pixel(J, gp - J.path_off, x, y, smp);  // else padding: no stage wrote its slots
+      const f3 c = pixel ? path_colour<TREE>(A, i) : mk3(0, 0, 0);
       const int first = (threadIdx.x & 31) & ~(spp - 1);
       for (int s = 0; s < spp; ++s)
         sum = add3(sum, mk3(__shfl_sync(0xffffffffu, c.x, first + s), __shfl_sync(0xffffffffu, c.y, first + s),
                             __shfl_sync(0xffffffffu, c.z, first + s)));
-      if (!path_pixel(J, gp - J.path_off, x, y, smp) || smp != 0) continue;
+      if (!pixel || smp != 0) continue;
     } else {
       if (!path_pixel(J, gp - J.path_off, x, y, smp) || smp != 0) continue;
       for (int s = 0; s < spp; ++s) sum = add3(sum, path_colour<TREE>(A, i + s));
