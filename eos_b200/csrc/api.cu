@@ -54,7 +54,6 @@ eos_ctx::~eos_ctx() {
     }
   if (own_stream) cudaStreamSynchronize(own_stream);
   if (pinned) cudaFreeHost(pinned);
-  if (ring_host) cudaFreeHost(ring_host);
   if (d_counts) cudaFree(d_counts);
   if (call_host) cudaFreeHost(call_host);
   if (ev0) cudaEventDestroy(ev0);
@@ -170,6 +169,27 @@ struct CallWords {
   int err, work;
 };
 
+}  // namespace
+
+eos_status eos::host_words(eos_ctx* ctx) {
+  if (ctx->call_host) return EOS_OK;
+  constexpr size_t kRingAt = (sizeof(CallWords) + 15) / 16 * 16;
+  char *host = nullptr, *dev = nullptr;
+  if (cudaHostAlloc(&host, kRingAt + 16 * eos_ctx::kRingSlots, cudaHostAllocMapped) != cudaSuccess ||
+      cudaHostGetDevicePointer(&dev, host, 0) != cudaSuccess) {
+    cudaGetLastError();
+    if (host) cudaFreeHost(host);
+    return EOS_ERR_OOM;
+  }
+  ctx->call_host = host;
+  ctx->ring_host = reinterpret_cast<int*>(host + kRingAt);
+  ctx->ring_dev = reinterpret_cast<int*>(dev + kRingAt);
+  for (int k = 0; k < 4 * eos_ctx::kRingSlots; ++k) ctx->ring_host[k] = -1;
+  return EOS_OK;
+}
+
+namespace {
+
 // Device view of a caller buffer: device pointers pass through, host buffers are copied
 // into a named scratch buffer on the context stream.
 const void* stage_in(eos_ctx* ctx, const char* name, const void* p, size_t bytes, eos_status* st) {
@@ -212,6 +232,7 @@ eos_status copy_out(eos_ctx* ctx, const OutBuf& o) {
 
 // Clears the error word and counters before a call.
 eos_status begin_call(eos_ctx* ctx) {
+  EOS_TRY(host_words(ctx));
   ctx->launches = 0;
   ctx->stage_ms[0] = ctx->stage_ms[1] = ctx->stage_ms[2] = 0.0f;
   EOS_CUDA(cudaMemsetAsync(ctx->d_counts, 0, sizeof(CallWords), ctx->stream));
@@ -402,7 +423,6 @@ eos_status eos_ctx_create(int32_t device, eos_ctx** out) {
     }
     if (cudaEventCreate(&ctx->ev0) != cudaSuccess || cudaEventCreate(&ctx->ev1) != cudaSuccess) { st = EOS_ERR_CUDA; break; }
     if (cudaMalloc(&ctx->d_counts, sizeof(CallWords)) != cudaSuccess) { st = EOS_ERR_OOM; break; }
-    if (cudaHostAlloc(&ctx->call_host, sizeof(CallWords), cudaHostAllocDefault) != cudaSuccess) { st = EOS_ERR_OOM; break; }
     cudaMemset(ctx->d_counts, 0, sizeof(CallWords));
     ctx->d_err = &reinterpret_cast<CallWords*>(ctx->d_counts)->err;
     ctx->d_work = &reinterpret_cast<CallWords*>(ctx->d_counts)->work;

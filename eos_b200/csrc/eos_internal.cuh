@@ -114,17 +114,20 @@ struct eos_ctx {
   unsigned long long* d_counts = nullptr;
   int* d_err = nullptr;
   int* d_work = nullptr;
-  void* call_host = nullptr;  // pinned copy of them: the end of every call reads it
+  // one block of mapped pinned memory, made by the context's first call (host_words; pinning
+  // takes 2 ms and more): a copy of those words, which the end of every call reads, and the
+  // read-back ring of the builders' launches that run ahead of the host (ring.cuh), slots of
+  // four ints; ring_next: the number of the next launch
+  static constexpr int kRingSlots = 2;
+  void* call_host = nullptr;
+  int* ring_host = nullptr;
+  int* ring_dev = nullptr;
+  long long ring_next = 0;
   std::map<std::string, eos::DevBuffer> scratch;
   cudaMemPool_t pool = nullptr;  // scene arrays and small scratch (pool_alloc)
   std::vector<float> bw_cams;  // cameras of the adjoint call in progress
   void* pinned = nullptr;
   size_t pinned_bytes = 0;
-  // read-back ring of the builders' launches that run ahead of the host (made on first use,
-  // ring.cuh): mapped pinned slots, and the number of the next launch
-  int* ring_host = nullptr;
-  int* ring_dev = nullptr;
-  long long ring_next = 0;
   // polls of a missing word before a look-back of the builders gives up (scan.cuh): a
   // fraction of a second; a test limit sets fewer (eos_ctx_set_build_polls)
   static constexpr int kBuildPolls = 1 << 18;
@@ -234,6 +237,8 @@ constexpr unsigned long long kPoolKeep = 1ull << 30;
 constexpr size_t kPoolScratch = 64u << 20;
 cudaError_t pool_alloc(eos_ctx* ctx, void** p, size_t bytes);
 eos_status pool_free(eos_ctx* ctx, void* const* p, int n);
+// Makes the context's pinned block where there is none yet.
+eos_status host_words(eos_ctx* ctx);
 // Pointer classification (cudaPointerGetAttributes): true for device/managed memory.
 bool is_device_ptr(const void* p);
 

@@ -29,21 +29,12 @@ __device__ __forceinline__ void ring_publish(int* slot, int a, int b, int c, int
 struct RoundRing {
   // Two launches in flight keep the device busy; more run on past the last round or level
   // (builds of 20k and 1.06M triangles 530 and 1,118 us with four, 516 and 1,087 with two).
-  static constexpr int kAhead = 2;
+  static constexpr int kAhead = eos_ctx::kRingSlots;
   eos_ctx* ctx;
   long long issued = 0, done = 0;
   explicit RoundRing(eos_ctx* c) : ctx(c) {}
   eos_status init() {
-    if (!ctx->ring_host) {
-      if (cudaHostAlloc(&ctx->ring_host, 16 * kAhead, cudaHostAllocMapped) != cudaSuccess ||
-          cudaHostGetDevicePointer(&ctx->ring_dev, ctx->ring_host, 0) != cudaSuccess) {
-        cudaGetLastError();
-        if (ctx->ring_host) cudaFreeHost(ctx->ring_host);
-        ctx->ring_host = ctx->ring_dev = nullptr;
-        return EOS_ERR_OOM;
-      }
-      for (int k = 0; k < 4 * kAhead; ++k) ctx->ring_host[k] = -1;
-    }
+    EOS_TRY(host_words(ctx));
     // launch numbers go on from sequence to sequence: a late write of an earlier sequence's
     // launch past its end is never taken for one of this
     base = ctx->ring_next;
