@@ -346,8 +346,8 @@ __global__ void __maxnreg__(F == kTwoLevel ? 80 : TREE ? 88 : 72) k_render_plain
     }
     const uint32_t idle = __ballot_sync(0xffffffffu, more && !active);
     const uint32_t busy = __ballot_sync(0xffffffffu, active);
-    // the next pixels once all lanes are done: taking them as single lanes end (or 8, 16, 24
-    // of them) mixes bounces in a warp and is no faster, 885 -> 906 us for a 1080p frame
+    // the next pixels once all lanes are done: taking them as single lanes end, or 16 of them,
+    // mixes bounces in a warp, 813 -> 841 and 830 us for a 1080p frame of 200k triangles
     if (idle && !busy) {
       uint32_t base = 0;
       if (lane == 0) base = atomicAdd(P.work, __popc(idle));
@@ -469,11 +469,17 @@ namespace {
 // Lanes of a warp that trace.  A frame of few pixels is bound by the time of its slowest
 // warp, which walks the union of its lanes' nodes, while most of the chip idles: with fewer
 // lanes a warp the same pixels spread over more warps.  Chains: the fewest lanes that leave
-// every warp resident (28 warps of 72 registers per SM).  Measured, us at 32 / 16 / 8 / 4 lanes:
-// 64x64 of 200k triangles 243 / 219 / 207 / 166, 128x128 271 / 251 / 213 / 197, 256x256 284 /
-// 278 / 282, 512x512 405 / 448 / 569.  Ray trees have longer tails (a pixel's tree is walked by
-// a warp): 8 lanes up to four such fillings (400x300: 1,588 / 1,732 / 1,458), 16 up to eight
-// (961x541: 2,113 / 1,881 / 2,201; 1920x1080: 3,033 / 3,551).
+// every warp resident in the kernel for flat scenes (28 warps of 72 registers per SM; the
+// two-level one holds 25, the queries 32 and 21, and their steps are taken at the same
+// place).  Measured, us at 32 / 16 / 8 / 4 lanes: 64x64 of 200k triangles 207 / 188 / 181 / 147,
+// 128x128 238 / 226 / 189 / 174, 256x256 247 / 244 / 249 / 287, 512x512 355 / 396 / 518 / 763;
+// 801 instances 64x64 1,294 / 969 / 777 / 629, 256x256 2,045 / 1,797 / 1,636 / 1,870, 512x512
+// 2,893 / 3,391; nearest hits of 1,000 rays 61 / 61 / 59 / 58, 33,000 71 / 70 / 71 / 83, 300,000
+// 157 / 194.  Ray trees have longer tails (a pixel's tree is walked by a warp): 8 lanes up to
+// four such fillings, 16 up to eight.  At 32 / 16 / 8 lanes: 400x300 1,449 / 1,565 / 1,300,
+// 640x360 1,644 / 1,429 / 1,287, 800x450 1,651 / 1,545 / 1,626, 961x541 1,886 / 1,721 / 1,998,
+// 1200x675 2,210 / 2,143 / 2,361, 1440x810 2,394 / 2,483; between the steps the rule is up to
+// 10 % from the best count.
 int lanes_of(uint32_t n_work, int num_sms, bool tree) {
   const uint32_t full = 28u * (uint32_t)num_sms;  // warps that fill the chip
   if (tree) return n_work / 8 <= 4 * full ? 8 : n_work / 16 <= 8 * full ? 16 : 32;

@@ -163,11 +163,11 @@ __device__ __forceinline__ int budget(int n, int work_limit, int* err) {
   return work_limit;
 }
 
-// The nearest-hit kernels are capped at 64 registers (blocks up to 256, 4 per SM): 56 and 72
-// cost 2 and 0.5 % of a four-view 1080p batch of 1.06M triangles (5,107 us), 5 and 4 % of a
-// 30-job batch.  The shadow kernels are capped at 56, one more block of 128 threads per SM
-// than at 64 for 12 B less of spill stores: 5,107 -> 5,049 us; 48 (196 B of spills) 5,521, 72
-// 5,131.  INST: the pass holds a two-level scene, whose traversal is inline in these kernels
+// The nearest-hit kernels are capped at 64 registers (blocks up to 256, 4 per SM), the shadow
+// kernels at 56 (36 warps per SM in blocks of 64, 32 at 64 registers).  Measured, us in blocks
+// of 64, four 1080p views of 1.06M triangles / a batch of 30 jobs: nearest hit at 56 5,036 /
+// 4,332, 64 4,970 / 4,203, 72 4,967 / 4,237; shadow at 48 5,428 / 4,469, 56 4,970 / 4,203, 64
+// 4,957 / 4,195 (in blocks of 128 1 % slower than 56), 72 5,025 / 4,235.  INST: the pass holds a two-level scene, whose traversal is inline in these kernels
 // only (TraversalForm); it keeps both spaces' rays and is latency-bound, so it gains more from
 // registers than from warps: 1080p view of 801 instances 10.9 ms at 64 / 64, 10.3 at 80 / 64,
 // 10.0 at 80 / 96 (nearest hit / shadow), 10.3 at 114 / 96; out of line 12.9 at 64 / 64 and
@@ -598,16 +598,16 @@ struct StageTimer {
   }
 };
 
-// The kernels of one configuration: a warp of the nearest-hit / shadow kernels takes
-// `queue_chunk` rays and finishes all before taking more.  small_stack selects the test
-// instantiation whose traversal stack is its SH shared-memory entries only (launch_config
-// pins SH = 8 then); tree the ray-tree mode.
 // Shared-memory entries of the shadow kernels' 4-byte stack columns for a stack depth of sh:
 // a little more than the nearest-hit kernels' 8-byte ones.  Deep trees spill less (4K view of
 // 4.5M triangles 65.1 -> 64.6 ms, 801 instances 16.3 -> 16.1; 24 and 32 entries are no
 // better), the others are unchanged.
 constexpr int any_entries(int sh) { return sh == 16 ? 20 : sh; }
 
+// The kernels of one configuration: a warp of the nearest-hit / shadow kernels takes
+// `queue_chunk` rays and finishes all before taking more.  small_stack selects the test
+// instantiation whose traversal stack is its SH shared-memory entries only (launch_config
+// pins SH = 8 then); tree the ray-tree mode.
 template <int SH>
 struct StageKernels {
   void (*closest_primary)(WfArgs);
