@@ -807,10 +807,10 @@ eos_status run_sequence(cudaStream_t st, int num_sms, const LaunchConfig& lc, co
                              lc.smem_a, false, lc.tree, lc.inst, tm, ov, launches);
 }
 
-// A pass in chunks of at most chunk_max paths; EOS_ERR_OOM comes before anything is queued.
-// *biggest_out: paths of its largest chunk.
+// A pass in chunks of at most chunk_max paths.  *too_large: its buffers did not fit the device
+// and those of chunks of kChunkPathsLow would be smaller; nothing is queued then.
 eos_status render_chunks(eos_ctx* ctx, const eos_job* jobs, uint32_t n_jobs, const eos_render_params& p,
-                         bool use_graph, long long chunk_max, long long* biggest_out) {
+                         bool use_graph, long long chunk_max, bool* too_large) {
   // host job table + chunk plan
   std::vector<DevJob> dj(n_jobs);
   long long total = 0;
@@ -857,7 +857,6 @@ eos_status render_chunks(eos_ctx* ctx, const eos_job* jobs, uint32_t n_jobs, con
   const bool timing = (p.flags & EOS_FLAG_STAGE_TIMING) != 0;
   long long biggest = 0;
   for (const Chunk& c : merged) biggest = std::max<long long>(biggest, c.n);
-  *biggest_out = biggest;
   std::vector<Chunk> lane_chunks[kLanes];
   if (timing || depth == 0 || !use_graph || biggest < kLaneSplitMin) {
     lane_chunks[0] = merged;
@@ -949,7 +948,10 @@ eos_status render_chunks(eos_ctx* ctx, const eos_job* jobs, uint32_t n_jobs, con
       ov[l].ev_any = ln.ev_any;
       ov[l].ev_shaded = ln.ev_shaded;
     }
-    if (es != EOS_OK) return es;
+    if (es != EOS_OK) {
+      *too_large = es == EOS_ERR_OOM && biggest > kChunkPathsLow;
+      return es;
+    }
     for (long long v : {(long long)a.cap_r, (long long)a.cap_s, (long long)a.work_limit, (long long)a.init_in_primary,
                         (long long)a.resolve, (long long)(size_t)a.rout, (long long)(size_t)a.rin,
                         (long long)(size_t)a.hits, (long long)(size_t)a.masks, (long long)(size_t)a.sq,
@@ -1022,14 +1024,13 @@ eos_status render_chunks(eos_ctx* ctx, const eos_job* jobs, uint32_t n_jobs, con
 
 eos_status render_wavefront(eos_ctx* ctx, const eos_job* jobs, uint32_t n_jobs, const eos_render_params& p,
                             bool use_graph) {
-  long long biggest = 0;
+  bool too_large = false;
   const eos_status st =
-      render_chunks(ctx, jobs, n_jobs, p, use_graph, ctx->low_memory ? kChunkPathsLow : kChunkPathsMax, &biggest);
-  if (st != EOS_ERR_OOM || biggest <= kChunkPathsLow) return st;
-  cudaGetLastError();
+      render_chunks(ctx, jobs, n_jobs, p, use_graph, ctx->low_memory ? kChunkPathsLow : kChunkPathsMax, &too_large);
+  if (!too_large) return st;
   ctx->low_memory = true;  // the context's later passes do not try again: buffers and graphs stay
   EOS_TRY(release_scratch(ctx, "wf."));  // a part of the large chunk's buffers
-  return render_chunks(ctx, jobs, n_jobs, p, use_graph, kChunkPathsLow, &biggest);
+  return render_chunks(ctx, jobs, n_jobs, p, use_graph, kChunkPathsLow, &too_large);
 }
 
 }  // namespace eos
